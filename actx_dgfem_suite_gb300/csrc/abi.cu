@@ -241,6 +241,14 @@ struct dg_plan {
   dg::LaunchShape tcb_shape[2];
   int tcb_grid[2] = {0, 0};
   int64_t tcb_ntiles[2] = {0, 0};
+  // symmetry-adapted kernel (dg_sym.cuh): the face-shared path's main kernel
+  // for operators that have the tetrahedron's symmetry
+  bool sym = false;
+  void* d_sym_ops = nullptr;
+  uint32_t sym_ops_bytes = 0;
+  dg::LaunchShape sym_shape;
+  int sym_grid = 0;
+  int64_t sym_ntiles = 0;
   // face-shared path and adjoint (wave, FP64): the mesh's face_partner
   const int32_t* face_partner = nullptr;
   void* d_adj_ops = nullptr;
@@ -388,6 +396,11 @@ int main_grid(const dg_plan* p) {
     if ((p->variant - kFirstShapeVariant) & 1)
       return (int)(p->tcb_ntiles[k] < 0x7fffffff ? p->tcb_ntiles[k] : 0x7fffffff);
     return p->tcb_grid[k];
+  }
+  if (p->sym) {
+    if (p->variant & 2)
+      return (int)(p->sym_ntiles < 0x7fffffff ? p->sym_ntiles : 0x7fffffff);
+    return p->sym_grid;
   }
   if (p->variant & 2) return (int)(p->ntiles < 0x7fffffff ? p->ntiles : 0x7fffffff);
   return (p->variant & 1) && p->precision == DG_FP32_MIXED ? p->grid_mtc : p->grid;
@@ -648,6 +661,25 @@ cudaError_t tc_launch_of(int eq, int order, int mode, const dg::RhsArgs& a, int 
   }
 }
 
+cudaError_t sym_shape_of(int eq, int order, bool stage, dg::LaunchShape* out) {
+  switch (eq) {
+    case DG_WAVE: return dg::sym_shape_wave(order, stage, out);
+    case DG_EULER: return dg::sym_shape_euler(order, stage, out);
+    case DG_MAXWELL: return dg::sym_shape_maxwell(order, stage, out);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t sym_launch_of(int eq, int order, bool stage, const dg::RhsArgs& a, int grid,
+                          cudaStream_t s) {
+  switch (eq) {
+    case DG_WAVE: return dg::sym_launch_wave(order, stage, a, grid, s);
+    case DG_EULER: return dg::sym_launch_euler(order, stage, a, grid, s);
+    case DG_MAXWELL: return dg::sym_launch_maxwell(order, stage, a, grid, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 // launch mode of tcgen05 form k (0 digits, 1 3xTF32, 2 3xTF32 at the other
 // CTA size), RHS; | 1 for the RK stage
 int tcm_mode(int k) { return k == 0 ? 0 : (k == 1 ? 2 : 6); }
@@ -892,6 +924,37 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     if (code != DG_OK) {
       dg_plan_destroy(p);
       return code;
+    }
+  }
+
+  if (split && !tc) {
+    const bool strong = equation == DG_MAXWELL;
+    std::vector<unsigned char> sops(
+        dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong, nullptr, 0));
+    const int bytes = dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong,
+                                       sops.data(), (int)sops.size());
+    if (bytes > 0) {  // the operators have the symmetry
+      dg::LaunchShape s0, s1;
+      err = sym_shape_of(equation, N, false, &s0);
+      if (err == cudaSuccess) err = sym_shape_of(equation, N, true, &s1);
+      if (err == cudaSuccess) err = cudaMalloc(&p->d_sym_ops, bytes);
+      if (err == cudaSuccess)
+        err = cudaMemcpy(p->d_sym_ops, sops.data(), bytes, cudaMemcpyHostToDevice);
+      if (err != cudaSuccess) {
+        dg_plan_destroy(p);
+        return cuda_fail(err, "symmetry-adapted kernel configuration");
+      }
+      if (s1.blocks_per_sm < s0.blocks_per_sm) s0.blocks_per_sm = s1.blocks_per_sm;
+      if (bytes != s0.ops_bytes || s0.blocks_per_sm < 1) {
+        dg_plan_destroy(p);
+        return fail(DG_ERR_CUDA, "symmetry-adapted kernel: layout mismatch or does not fit");
+      }
+      p->sym = true;
+      p->sym_ops_bytes = static_cast<uint32_t>(bytes);
+      p->sym_shape = s0;
+      p->sym_ntiles = (p->nel + s0.elems_per_tile - 1) / s0.elems_per_tile;
+      const int64_t sfull = (int64_t)nsm * s0.blocks_per_sm;
+      p->sym_grid = (int)(p->sym_ntiles < sfull ? p->sym_ntiles : sfull);
     }
   }
 
@@ -1199,6 +1262,31 @@ int autotune_impl(dg_plan* p, const double* q, double* rhs, const double* ref,
   return code;
 }
 
+// The main kernel (volume and LIFT, with the fluxes where they are fused)
+// under the plan's precision, path and variant: RHS or RK stage.
+cudaError_t launch_main(const dg_plan* p, dg::RhsArgs a, bool stage, cudaStream_t s) {
+  const int prec = p->precision == DG_FP32_MIXED ? 1 : 0;
+  if (p->tc) {
+    a.ops = p->d_tc_ops;
+    a.ops_bytes = p->tc_ops_bytes;
+    return tc_launch_of(p->equation, p->order, stage ? 1 : 0, a, p->tc_grid, s);
+  }
+  if (is_tcm_variant(p->variant)) {
+    const int k = p->variant - 4;
+    a.ops = p->d_tcm_ops[k];
+    a.ops_bytes = p->tcm_ops_bytes[k];
+    return tcm_launch_of(p->equation, p->order, tcm_mode(k) | (stage ? 1 : 0), a,
+                         p->tcm_grid[k], s);
+  }
+  if (p->sym) {
+    a.ops = p->d_sym_ops;
+    a.ops_bytes = p->sym_ops_bytes;
+    return sym_launch_of(p->equation, p->order, stage, a, main_grid(p), s);
+  }
+  const int base = (stage ? dg::MODE_STAGE : dg::MODE_RHS) | (p->split ? dg::MODE_SPLIT : 0);
+  return launch_of(p->equation, p->order, prec, main_mode(p, base), a, main_grid(p), s);
+}
+
 dg::VjpArgs vjp_args(const dg_plan* p, const double* q, const double* x, double* y) {
   dg::VjpArgs a;
   std::memset(&a, 0, sizeof(a));
@@ -1426,21 +1514,7 @@ int dg_rhs(dg_plan* p, const double* q, double* rhs, void* stream) {
                                                 p->params[0], p->pres_grid, s);
     if (err != cudaSuccess) return cuda_fail(err, "pressure kernel launch");
   }
-  cudaError_t err;
-  if (p->tc) {
-    a.ops = p->d_tc_ops;
-    a.ops_bytes = p->tc_ops_bytes;
-    err = tc_launch_of(p->equation, p->order, 0, a, p->tc_grid, s);
-  } else if (is_tcm_variant(p->variant)) {
-    const int k = p->variant - 4;
-    a.ops = p->d_tcm_ops[k];
-    a.ops_bytes = p->tcm_ops_bytes[k];
-    err = tcm_launch_of(p->equation, p->order, tcm_mode(k), a, p->tcm_grid[k], s);
-  } else {
-    err = launch_of(p->equation, p->order, p->precision == DG_FP32_MIXED ? 1 : 0,
-                    main_mode(p, p->split ? dg::MODE_SPLIT : dg::MODE_RHS), a,
-                    main_grid(p), s);
-  }
+  cudaError_t err = launch_main(p, a, false, s);
   if (err != cudaSuccess) return cuda_fail(err, "rhs launch");
   return DG_OK;
 }
@@ -1483,21 +1557,7 @@ int dg_rk_stage(dg_plan* p, const double* q_in, double* q_out, double* res,
                                                 p->params[0], p->pres_grid, s);
     if (err != cudaSuccess) return cuda_fail(err, "pressure kernel launch");
   }
-  cudaError_t err;
-  if (p->tc) {
-    a.ops = p->d_tc_ops;
-    a.ops_bytes = p->tc_ops_bytes;
-    err = tc_launch_of(p->equation, p->order, 1, a, p->tc_grid, s);
-  } else if (is_tcm_variant(p->variant)) {
-    const int k = p->variant - 4;
-    a.ops = p->d_tcm_ops[k];
-    a.ops_bytes = p->tcm_ops_bytes[k];
-    err = tcm_launch_of(p->equation, p->order, tcm_mode(k) | 1, a, p->tcm_grid[k], s);
-  } else {
-    err = launch_of(p->equation, p->order, p->precision == DG_FP32_MIXED ? 1 : 0,
-                    main_mode(p, dg::MODE_STAGE | (p->split ? dg::MODE_SPLIT : 0)), a,
-                    main_grid(p), s);
-  }
+  cudaError_t err = launch_main(p, a, true, s);
   if (err != cudaSuccess) return cuda_fail(err, "rk stage launch");
   return DG_OK;
 }
@@ -1612,7 +1672,7 @@ int dg_plan_destroy(dg_plan* p) {
   for (void* b : {(void*)p->d_owned, (void*)p->d_flux, (void*)p->d_aux,
                   (void*)p->d_tc_ops, p->d_tcm_ops[0], p->d_tcm_ops[1],
                   p->d_tcm_ops[2] != p->d_tcm_ops[1] ? p->d_tcm_ops[2] : nullptr,
-                  (void*)p->d_pres})
+                  (void*)p->d_pres, p->d_sym_ops})
     if (b && cudaFree(b) != cudaSuccess) code = DG_ERR_CUDA;
   delete p;
   if (code != DG_OK) return fail(code, "cudaFree failed");
@@ -1714,11 +1774,14 @@ int dg_plan_info(const dg_plan* p, int64_t* nelements, int32_t* order,
   if (block)
     *block = p->tc ? p->tc_shape.threads
                    : (m4 ? p->tcm_shape[k].threads
-                         : (mb ? p->tcb_shape[kb].threads : dg::kBlock));
+                         : (mb ? p->tcb_shape[kb].threads
+                               : (p->sym ? p->sym_shape.threads : dg::kBlock)));
   if (smem_bytes)
     *smem_bytes = p->tc ? p->tc_shape.smem_bytes
                         : (m4 ? p->tcm_shape[k].smem_bytes
-                              : (mb ? p->tcb_shape[kb].smem_bytes : p->shape.smem_bytes));
+                              : (mb ? p->tcb_shape[kb].smem_bytes
+                                    : (p->sym ? p->sym_shape.smem_bytes
+                                                   : p->shape.smem_bytes)));
   return DG_OK;
 }
 

@@ -14,8 +14,9 @@
 //       the flux once and writes the lifted-flux input of BOTH glued face
 //       points; the neighbour's value follows from how each flux transforms
 //       when the two sides swap (n -> -n, jumps change sign);
-//   (c) dg_rhs_kernel with MODE_SPLIT: volume term + LIFT of the stored face
-//       values, in the same persistent tile loop as the fused kernel.
+//   (c) the volume term and the LIFT of the stored face values:
+//       dg_rhs_sym_kernel (dg_sym.cuh) for operators with the tetrahedron's
+//       symmetry, dg_rhs_kernel with MODE_SPLIT for any others.
 //
 // Face values live in HBM as (nfields, Nel, 4 Nfp) doubles, face point
 // (e, f, j) at e * 4 Nfp + f Nfp + j -- the fused kernel's shared-memory

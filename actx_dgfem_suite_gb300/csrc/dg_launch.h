@@ -57,6 +57,8 @@ inline OpsOffsets ops_offsets(int np, int nfp, int rs) {
 // tcm_shape_* / tcm_launch_*: the mixed-precision kernel with its
 // contractions on tcgen05 (mode bit 0: RK stage; bit 1: 3xTF32 products,
 // else exact digit-pair products; bit 2, with bit 1: the other CTA size).
+// sym_shape_* / sym_launch_*: the face-shared volume/LIFT kernel in the
+// symmetry-adapted basis (dg_sym.cuh), for operators that pack_sym_ops accepts.
 #define DG_DECLARE_EQ(name)                                                   \
   cudaError_t shape_##name(int order, int precision, int mode,               \
                            LaunchShape* out);                                \
@@ -70,6 +72,9 @@ inline OpsOffsets ops_offsets(int np, int nfp, int rs) {
                                int grid, cudaStream_t s);                    \
   cudaError_t tcm_shape_##name(int order, int mode, LaunchShape* out);       \
   cudaError_t tcm_launch_##name(int order, int mode, const RhsArgs& a,       \
+                                int grid, cudaStream_t s);                   \
+  cudaError_t sym_shape_##name(int order, bool stage, LaunchShape* out);     \
+  cudaError_t sym_launch_##name(int order, bool stage, const RhsArgs& a,     \
                                 int grid, cudaStream_t s);
 DG_DECLARE_EQ(wave)
 DG_DECLARE_EQ(euler)
@@ -94,6 +99,13 @@ int pack_tc_ops(int eq, int order, const double* diff, const double* lift,
 int pack_tcm_ops(int order, const double* diff, const double* lift,
                  const int32_t* face_nodes, unsigned char* out, int out_bytes,
                  bool tf32);
+
+// Operator block of the symmetry-adapted kernels (sym::Ops in dg_sym.cuh);
+// `strong`: diff holds strong derivatives.  Returns the block size (out ==
+// NULL: size only), or -1 when the operators do not have the tetrahedron's
+// four-group symmetry to rounding (or out_bytes is short).
+int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
+                 bool strong, unsigned char* out, int out_bytes);
 
 // Triangle meshes (rhs_2d.cu): shape query and launch of dg_rhs2d_kernel
 // for mode MODE_RHS or MODE_STAGE (FP64), and the operator block

@@ -1,0 +1,493 @@
+// FP64 volume/LIFT kernel in the symmetry-adapted basis of the tetrahedron
+// (sm_103a), the main kernel of the face-shared path (dg_face.cuh).
+//
+// What bounds it: the FP64 pipe.  GB300 issues two FP64 multiply-adds per SM
+// and clock (measured 1.25 TFLOP/s), so the dense products of dg_rhs_kernel
+// held that pipe at 94-97 % for orders 2-4 and the only way down is fewer
+// FP64 operations.  The reference tetrahedron gives them: its node set and
+// operators are invariant under permutations of its vertices, and the
+// four-group V = {id, g1 = (01)(23), g2 = (02)(13), g3 = (03)(12)} is enough
+// to split every operator into blocks.  With one butterfly (sum and difference
+// transform) per orbit of nodes a field splits into four parts, A (even under
+// every g) and B1, B2, B3 (B_k even under g_k, odd under the other two).
+// Along the directions that join the midpoints of opposite edges,
+// d_k = v0 + v_k - (the other two), every g maps d_k to plus or minus itself,
+// so the derivative along d_k takes part sigma to the single part
+// rho = sigma xor k (parts numbered 0 for A and k for B_k), and LIFT takes each
+// part of the face values (V permutes the faces without fixed points: Nfp
+// orbits of four points) to the same part of the nodes.  The dense Np x Np
+// derivatives and the Np x 4 Nfp LIFT become four blocks each: a quarter of
+// the multiply-adds for two additions per node or face point and field.
+//
+//   multiply-adds per field   derivative (one direction)      LIFT
+//   order 1 / 2 / 3 / 4       16 / 100 / 400 / 1225 dense     48 / 240 / 800 / 2100
+//                              1 /  24 / 100 /  304 here      12 /  60 / 200 /  525
+//
+// The direction metric follows from the element's dr/dx:
+// sum_r g_r D_r = sum_k h_k D'_k with h_1 = g_2 + g_3 (cyclic) and
+// D'_k = -1/2 D_{d_k}; the host folds all constants and the butterflies'
+// normalisation into the blocks, and takes this path only for operators whose
+// blocks outside the pattern vanish to rounding (pack_sym_ops, sym_ops.cu);
+// others keep dg_rhs_kernel.
+//
+// Measured (GB300, CUDA events, whole RHS with its face kernel, dense kernel
+// before -> now): Maxwell P4 584,016 tets 38.9 -> 14.3 ms, Euler P4 118,098 tets
+// 7.08 -> 3.57 ms, wave P3 215,622 tets 2.69 -> 1.27 ms, Euler P2 LSRK step
+// 413,526 tets 16.7 -> 11.6 ms, wave P1 5.14 M tets 5.77 -> 4.56 ms.  The kernel
+// runs at 72-88 % of the FP64 pipe's rate by operation count.
+//
+// Work split: a tile of E elements with one lane per element and one warp per
+// part rho, so that every operator entry is the same for a whole warp and is
+// read once, by a broadcast, for all fields of the thread; accumulators stay
+// in registers.  Data sits in shared memory as [array][slot][element] with an
+// odd element pitch (no bank conflicts along elements or slots).  Per tile:
+// state -> slots; transform; volume blocks; face values (transformed on the
+// way in, over the state's shared memory); LIFT blocks; inverse transform;
+// store or Runge-Kutta stage.
+#pragma once
+
+#include "dg_rhs.cuh"
+
+namespace dg {
+namespace sym {
+
+// Orbits of the node set under V: NO4 orbits of four nodes, NPR pairs (edge
+// midpoints) per direction, NSG fixed points (the centroid); DA and DB nodes
+// in parts A and B_k.
+template <int N>
+struct Basis {
+  static constexpr int NP = Shape<N>::NP, NFP = Shape<N>::NFP, NFPT = 4 * NFP;
+  static constexpr int NPR = N % 2 == 0 ? 1 : 0, NSG = N == 4 ? 1 : 0;
+  static constexpr int NO4 = (NP - 6 * NPR - NSG) / 4;
+  static constexpr int DB = NO4 + NPR, DA = NO4 + 3 * NPR + NSG;
+  static_assert(DA + 3 * DB == NP, "the parts cover the node set");
+};
+
+// Operator block: doubles in rows of one input each, padded to 16 bytes.
+// Volume blocks of part 0, then 1, 2, 3, each for k = 1, 2, 3 (inputs of part
+// rho xor k); LIFT blocks the same way (NFP inputs).  Then two int32 tables:
+// node -> slot, and the face point of every face slot (part r of orbit o at
+// r NFP + o).
+template <int N>
+struct Ops {
+  using B = Basis<N>;
+  static constexpr int PA = (B::DA + 1) & ~1, PB = (B::DB + 1) & ~1;
+  static constexpr int VOL0 = 3 * B::DB * PA;               // entries of part 0
+  static constexpr int VOLB = (B::DA + 2 * B::DB) * PB;     // of each part B_k
+  static constexpr int LIFT = VOL0 + 3 * VOLB;
+  static constexpr int LIFTB = LIFT + B::NFP * PA;
+  static constexpr int ENTRIES = LIFTB + 3 * B::NFP * PB;
+  static constexpr int NODE_SLOT = ENTRIES * 8;             // bytes from here
+  static constexpr int FACE_POINT = NODE_SLOT + pad16(B::NP * 4);
+  static constexpr int SIZE = FACE_POINT + pad16(B::NFPT * 4);
+};
+
+// Tile shape.  Maxwell's E and H equations have the same form, so the two
+// halves of a warp take one each: 16 elements per tile, and the order-4 tile
+// (49 KB) fits four times on an SM.  Wave and Euler keep all fields in a
+// thread and 32 elements per tile.  Face values and result reuse the state's
+// arrays.
+template <int N, int EQ>
+struct Tile {
+  using B = Basis<N>;
+  static constexpr int NF = EqInfo<EQ>::NF;
+  static constexpr int NX = EQ == DG_EULER ? 12 : NF;       // euler: flux components
+  static constexpr int GROUPS = EQ == DG_MAXWELL ? 2 : 1;
+  static constexpr int NA = NF / GROUPS;                    // fields of a thread
+  static constexpr int E = 32 / GROUPS, PE = E + 1;
+  static constexpr int BLOCK = 128;
+  static constexpr int X = Ops<N>::SIZE;
+  static constexpr int X_BYTES = pad16(NX * B::NP * PE * 8);
+  static constexpr int F_BYTES = pad16(NF * B::NFPT * PE * 8);
+  static constexpr int H = X + (X_BYTES > F_BYTES ? X_BYTES : F_BYTES);
+  static constexpr int SMEM = H + pad16(9 * PE * 8);
+};
+
+// (x0, x1, x2, x3) at (n, g1 n, g2 n, g3 n) <-> parts A, B1, B2, B3 (its own
+// inverse up to the factor 4 that the operator blocks hold)
+__device__ __forceinline__ void butterfly(double& a, double& b, double& c, double& d) {
+  const double s = a + b, t = a - b, u = c + d, v = c - d;
+  a = s + u;
+  b = s - u;
+  c = t + v;
+  d = t - v;
+}
+
+// Barrier of the whole CTA for warps that arrive from different branches (the
+// parts' code differs where their sizes do); the branch is uniform per warp.
+template <int BLOCK>
+__device__ __forceinline__ void cta_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(BLOCK) : "memory");
+}
+
+// One row of operator entries, the same for the whole warp.
+template <int P>
+__device__ __forceinline__ void load_row(const double* p, double (&r)[P]) {
+#pragma unroll
+  for (int k = 0; k < P; k += 2) {
+    const double2 v = *reinterpret_cast<const double2*>(p + k);
+    r[k] = v.x;
+    r[k + 1] = v.y;
+  }
+}
+
+// Volume term of part rho (D outputs, row pitch P).  x: the thread's element
+// in shared memory; h: metric of the three directions (pitch PE per entry);
+// f0: first input field (Maxwell); sgn: Maxwell's curl sign, wave's -c.
+template <int N, int EQ, int D, int P>
+__device__ __forceinline__ void volume(const double* __restrict__ x,
+                                       const double* __restrict__ h,
+                                       const double* __restrict__ row, int rho, int f0,
+                                       double sgn, double (&acc)[Tile<N, EQ>::NA][D]) {
+  using B = Basis<N>;
+  constexpr int PE = Tile<N, EQ>::PE, FS = B::NP * PE;  // array stride
+  constexpr bool STRONG = EQ == DG_MAXWELL;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int sig = rho ^ (k + 1);
+    const int din = sig == 0 ? B::DA : B::DB;
+    const double* xs = x + (sig == 0 ? 0 : B::DA + (sig - 1) * B::DB) * PE;
+    // order 1: strong derivatives reach part A only, weak ones leave it only
+    if (N == 1 && (STRONG ? rho != 0 : sig != 0)) {
+      row += din * P;
+      continue;
+    }
+    const double h0 = sgn * h[(k * 3 + 0) * PE], h1 = sgn * h[(k * 3 + 1) * PE],
+                 h2 = sgn * h[(k * 3 + 2) * PE];
+    if constexpr (EQ == DG_WAVE) {
+      double g[D];
+#pragma unroll
+      for (int i = 0; i < D; ++i) g[i] = 0.0;
+#pragma unroll 1
+      for (int j = 0; j < din; ++j, row += P, xs += PE) {
+        const double u = xs[0];
+        const double w = fma(h0, xs[FS], fma(h1, xs[2 * FS], h2 * xs[3 * FS]));
+        double t[P];
+        load_row<P>(row, t);
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          acc[0][i] = fma(t[i], w, acc[0][i]);
+          g[i] = fma(t[i], u, g[i]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        acc[1][i] = fma(h0, g[i], acc[1][i]);
+        acc[2][i] = fma(h1, g[i], acc[2][i]);
+        acc[3][i] = fma(h2, g[i], acc[3][i]);
+      }
+    } else if constexpr (EQ == DG_EULER) {
+      // arrays 0-2: m; 3-5: (E + p) u; 6-11: m u + p (xx, xy, xz, yy, yz, zz)
+      constexpr int S[5][3] = {{0, 1, 2}, {3, 4, 5}, {6, 7, 8}, {7, 9, 10}, {8, 10, 11}};
+#pragma unroll 1
+      for (int j = 0; j < din; ++j, row += P, xs += PE) {
+        double v[12], t[P];
+#pragma unroll
+        for (int m = 0; m < 12; ++m) v[m] = xs[m * FS];
+        load_row<P>(row, t);
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+          const double w = fma(h0, v[S[f][0]], fma(h1, v[S[f][1]], h2 * v[S[f][2]]));
+#pragma unroll
+          for (int i = 0; i < D; ++i) acc[f][i] = fma(t[i], w, acc[f][i]);
+        }
+      }
+    } else {
+      const double* xf = xs + f0 * FS;
+#pragma unroll 1
+      for (int j = 0; j < din; ++j, row += P, xf += PE) {
+        const double v0 = xf[0], v1 = xf[FS], v2 = xf[2 * FS];
+        double t[P];
+        load_row<P>(row, t);
+        const double w0 = fma(h1, v2, -h2 * v1);
+        const double w1 = fma(h2, v0, -h0 * v2);
+        const double w2 = fma(h0, v1, -h1 * v0);
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+          acc[0][i] = fma(t[i], w0, acc[0][i]);
+          acc[1][i] = fma(t[i], w1, acc[1][i]);
+          acc[2][i] = fma(t[i], w2, acc[2][i]);
+        }
+      }
+    }
+  }
+}
+
+// LIFT of part rho: f is the thread's element at its part's first face slot
+// (and first output field).
+template <int N, int EQ, int D, int P>
+__device__ __forceinline__ void lift(const double* __restrict__ f,
+                                     const double* __restrict__ row,
+                                     double (&acc)[Tile<N, EQ>::NA][D]) {
+  using B = Basis<N>;
+  constexpr int PE = Tile<N, EQ>::PE, FS = B::NFPT * PE, NA = Tile<N, EQ>::NA;
+#pragma unroll 1
+  for (int o = 0; o < B::NFP; ++o, row += P, f += PE) {
+    double v[NA], t[P];
+#pragma unroll
+    for (int m = 0; m < NA; ++m) v[m] = f[m * FS];
+    load_row<P>(row, t);
+#pragma unroll
+    for (int m = 0; m < NA; ++m)
+#pragma unroll
+      for (int i = 0; i < D; ++i) acc[m][i] = fma(t[i], v[m], acc[m][i]);
+  }
+}
+
+// In-place (inverse) transform of `narrays` node arrays of a tile.
+template <int N, int PE, int E, int BLOCK>
+__device__ __forceinline__ void transform(double* x, int narrays) {
+  using B = Basis<N>;
+  constexpr int NO = B::NO4 + 3 * B::NPR;
+  const int le = threadIdx.x % E;
+  for (int job = threadIdx.x / E; job < narrays * NO; job += BLOCK / E) {
+    const int f = job / NO, o = job - f * NO;
+    double* p = x + f * (B::NP * PE) + le;
+    if (o < B::NO4) {
+      double* b = p + (B::DA + o) * PE;
+      butterfly(p[o * PE], b[0], b[B::DB * PE], b[2 * B::DB * PE]);
+    } else {  // the pair of direction o - NO4 + 1
+      double& u = p[o * PE];
+      double& v = p[(B::DA + (o - B::NO4) * B::DB + B::NO4) * PE];
+      const double s = u + v, d = u - v;
+      u = s;
+      v = d;
+    }
+  }
+}
+
+// Euler: node state (arrays 0-4), pressure (5) and 1/rho (6) to the twelve
+// flux components, transformed, in place.
+template <int N, int PE, int E, int BLOCK>
+__device__ __forceinline__ void euler_inputs(double* x) {
+  using B = Basis<N>;
+  constexpr int NO = B::NO4 + 3 * B::NPR + B::NSG, FS = B::NP * PE;
+  const int le = threadIdx.x % E;
+  for (int o = threadIdx.x / E; o < NO; o += BLOCK / E) {
+    const int pair = o - B::NO4;                 // 0-2: pairs, 3: the centroid
+    const int cnt = NO == B::NO4 || pair < 0 ? 4 : (pair < 3 ? 2 : 1);
+    double* p[4];
+    p[0] = x + o * PE + le;
+    p[1] = x + (pair < 0 ? B::DA + o : B::DA + pair * B::DB + B::NO4) * PE + le;
+    p[2] = x + (B::DA + B::DB + o) * PE + le;
+    p[3] = x + (B::DA + 2 * B::DB + o) * PE + le;
+    double m[4][3], u[4][3], pr[4], ep[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      if (n >= cnt) break;
+      const double rinv = p[n][6 * FS];
+      pr[n] = p[n][5 * FS];
+      ep[n] = p[n][FS] + pr[n];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        m[n][c] = p[n][(2 + c) * FS];
+        u[n][c] = m[n][c] * rinv;
+      }
+    }
+    auto put = [&](int arr, auto val) {
+      if (cnt == 4) {
+        double v0 = val(0), v1 = val(1), v2 = val(2), v3 = val(3);
+        butterfly(v0, v1, v2, v3);
+        p[0][arr * FS] = v0;
+        p[1][arr * FS] = v1;
+        p[2][arr * FS] = v2;
+        p[3][arr * FS] = v3;
+      } else if (cnt == 2) {
+        const double v0 = val(0), v1 = val(1);
+        p[0][arr * FS] = v0 + v1;
+        p[1][arr * FS] = v0 - v1;
+      } else {
+        p[0][arr * FS] = val(0);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < 3; ++c) put(c, [&](int n) { return m[n][c]; });
+#pragma unroll
+    for (int c = 0; c < 3; ++c) put(3 + c, [&](int n) { return ep[n] * u[n][c]; });
+    int arr = 6;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int d = c; d < 3; ++d, ++arr)
+        put(arr, [&](int n) {
+          return c == d ? fma(m[n][c], u[n][d], pr[n]) : m[n][c] * u[n][d];
+        });
+  }
+}
+
+template <int N, int EQ, bool STAGE>
+__global__ void __launch_bounds__(Tile<N, EQ>::BLOCK) dg_rhs_sym_kernel(const RhsArgs a) {
+  using T = Tile<N, EQ>;
+  using O = Ops<N>;
+  using B = Basis<N>;
+  constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT, NF = T::NF, NA = T::NA;
+  constexpr int E = T::E, PE = T::PE, BLOCK = T::BLOCK;
+  constexpr int XS = NP * PE, FS = NFPT * PE;  // array strides
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint64_t bar;
+  __shared__ int ops_ok;
+  const double* ops = reinterpret_cast<const double*>(smem);
+  const int* node_slot = reinterpret_cast<const int*>(smem + O::NODE_SLOT);
+  const int* face_point = reinterpret_cast<const int*>(smem + O::FACE_POINT);
+  double* sX = reinterpret_cast<double*>(smem + T::X);
+  double* sH = reinterpret_cast<double*>(smem + T::H);
+
+  const int t = threadIdx.x;
+  if (t == 0) {
+    mbar_init(&bar, 1);
+    mbar_arrive_expect_tx(&bar, a.ops_bytes);
+    bulk_g2s(smem, a.ops, a.ops_bytes, &bar);
+    const bool ok = mbar_wait_bounded(&bar, 0);
+    if (!ok) {
+      raise_status(a.status, DG_ERR_TIMEOUT);
+      mbar_wait_bounded(&bar, 0);  // give the copy one more bounded chance
+    }
+    ops_ok = ok ? 1 : 0;
+  }
+  __syncthreads();
+  if (!ops_ok) return;
+
+  const int lane = t & 31;
+  const int le = lane % E;              // element of the tile
+  const int grp = lane / E;             // Maxwell: 0 the E fields, 1 the H fields
+  const int64_t nel = a.nel;
+  const int64_t nelnp = nel * NP;
+  const int64_t ntiles = (nel + E - 1) / E;
+
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int64_t e0 = tile * E;
+    const int ecount = (nel - e0) < (int64_t)E ? (int)(nel - e0) : E;
+
+    // {{{ state and metric -> shared memory, then the volume term's inputs
+    {
+      const double* qk = a.q + e0 * NP;
+      for (int rem = t; rem < E * NP; rem += BLOCK) {
+        const int el = rem / NP;
+        double* x = sX + node_slot[rem - el * NP] * PE + el;
+        const bool in = rem < ecount * NP;
+        double v[NF];
+#pragma unroll
+        for (int k = 0; k < NF; ++k) v[k] = in ? __ldg(qk + k * nelnp + rem) : 0.0;
+        if constexpr (EQ == DG_EULER) {
+          const double* ax = a.aux + e0 * NP + rem;
+          x[5 * XS] = in ? __ldg(ax) : 0.0;
+          x[6 * XS] = in ? __ldg(ax + nelnp) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < NF; ++k) x[k * XS] = v[k];
+      }
+      const double* mt = a.metric + e0 * 9;
+      for (int idx = t; idx < 9 * E; idx += BLOCK) {
+        const int el = idx / 9, kx = idx - el * 9, k = kx / 3, x = kx - k * 3;
+        double v = 0.0;
+        if (el < ecount)
+          v = __ldg(mt + el * 9 + (k == 0 ? 3 : 0) + x) + __ldg(mt + el * 9 + (k == 2 ? 3 : 6) + x);
+        sH[kx * PE + el] = v;
+      }
+    }
+    __syncthreads();
+    if constexpr (EQ == DG_EULER) euler_inputs<N, PE, E, BLOCK>(sX);
+    else transform<N, PE, E, BLOCK>(sX, NF);
+    __syncthreads();
+    // }}}
+
+    // {{{ volume and LIFT blocks, one part per warp.  The parts differ in size
+    // at orders 2 and 4, so they rotate over the warps (and with them over
+    // the SM's four quadrants) from tile to tile.
+    const int rho = ((t >> 5) + (int)tile) & 3;
+    const int f_in = EQ == DG_MAXWELL ? 3 - 3 * grp : 0;
+    const int f_out = EQ == DG_MAXWELL ? 3 * grp : 0;
+    const double sgn = EQ == DG_MAXWELL ? (grp == 0 ? 1.0 : -1.0)
+                                        : (EQ == DG_WAVE ? -a.p0 : 1.0);
+
+    // the tile's face values, transformed on the way in
+    auto load_faces = [&]() {
+      const int64_t nfpt_all = nel * NFPT;
+      const double* fk = a.flux_in + e0 * NFPT;
+      for (int idx = t; idx < E * NFP; idx += BLOCK) {
+        const int el = idx / NFP, o = idx - el * NFP;
+        // the orbit's four points, one per face
+        const int p0 = face_point[o], p1 = face_point[NFP + o],
+                  p2 = face_point[2 * NFP + o], p3 = face_point[3 * NFP + o];
+        const double* fe = fk + el * NFPT;
+        const bool in = el < ecount;
+        double v[NF][4];
+#pragma unroll
+        for (int k = 0; k < NF; ++k, fe += nfpt_all) {
+          v[k][0] = in ? __ldg(fe + p0) : 0.0;
+          v[k][1] = in ? __ldg(fe + p1) : 0.0;
+          v[k][2] = in ? __ldg(fe + p2) : 0.0;
+          v[k][3] = in ? __ldg(fe + p3) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+          butterfly(v[k][0], v[k][1], v[k][2], v[k][3]);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) sX[k * FS + (r * NFP + o) * PE + el] = v[k][r];
+        }
+      }
+    };
+
+    auto part = [&](auto dtag, auto ptag, int slot0, const double* vops, const double* lops) {
+      constexpr int D = decltype(dtag)::value, P = decltype(ptag)::value;
+      double acc[NA][D];
+#pragma unroll
+      for (int m = 0; m < NA; ++m)
+#pragma unroll
+        for (int i = 0; i < D; ++i) acc[m][i] = 0.0;
+      volume<N, EQ, D, P>(sX + le, sH + le, vops, rho, f_in, sgn, acc);
+      cta_sync<BLOCK>();  // the state's slots are free
+      load_faces();
+      cta_sync<BLOCK>();
+      lift<N, EQ, D, P>(sX + f_out * FS + rho * NFP * PE + le, lops, acc);
+      cta_sync<BLOCK>();  // every warp has read its inputs
+      [[maybe_unused]] const double post = grp == 0 ? a.k[4] : a.k[5];  // 1/eps, 1/mu
+#pragma unroll
+      for (int m = 0; m < NA; ++m)
+#pragma unroll
+        for (int i = 0; i < D; ++i)
+          sX[(f_out + m) * XS + (slot0 + i) * PE + le] =
+              EQ == DG_MAXWELL ? acc[m][i] * post : acc[m][i];
+    };
+    using IA = std::integral_constant<int, B::DA>;
+    using IB = std::integral_constant<int, B::DB>;
+    using PA = std::integral_constant<int, O::PA>;
+    using PB = std::integral_constant<int, O::PB>;
+    if (B::DA != B::DB && rho == 0)
+      part(IA{}, PA{}, 0, ops, ops + O::LIFT);
+    else
+      part(IB{}, PB{}, rho == 0 ? 0 : B::DA + (rho - 1) * B::DB,
+           ops + (rho == 0 ? 0 : O::VOL0 + (rho - 1) * O::VOLB),
+           ops + (rho == 0 ? O::LIFT : O::LIFTB + (rho - 1) * (NFP * O::PB)));
+    __syncthreads();
+    // }}}
+
+    // {{{ back to nodes, then store or fold into the RK stage
+    transform<N, PE, E, BLOCK>(sX, NF);
+    __syncthreads();
+    for (int rem = t; rem < ecount * NP; rem += BLOCK) {
+      const int el = rem / NP;
+      const double* y = sX + node_slot[rem - el * NP] * PE + el;
+      int64_t gidx = e0 * NP + rem;
+#pragma unroll
+      for (int k = 0; k < NF; ++k, gidx += nelnp) {
+        double val = y[k * XS];
+        if constexpr (STAGE)
+          if (a.rhs_unscaled) a.rhs_unscaled[gidx] = val;
+        if (a.elem_scale) val *= __ldg(a.elem_scale + e0 + el);
+        if constexpr (!STAGE) {
+          a.rhs[gidx] = val;
+        } else {
+          const double r = (a.rk_a != 0.0 ? a.rk_a * a.res[gidx] : 0.0) + a.rk_dt * val;
+          a.res[gidx] = r;
+          a.q_out[gidx] = __ldg(a.q + gidx) + a.rk_b * r;
+        }
+      }
+    }
+    __syncthreads();
+    // }}}
+  }
+}
+
+}  // namespace sym
+}  // namespace dg

@@ -1,0 +1,239 @@
+// Operator blocks of the symmetry-adapted kernels (layout: sym::Ops in
+// dg_sym.cuh), derived on the host from the caller's derivative matrices and
+// LIFT.
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "dg_launch.h"
+#include "dg_sym.cuh"
+
+namespace dg {
+namespace {
+
+// vertex permutations id, (01)(23), (02)(13), (03)(12)
+constexpr int kGroup[4][4] = {{0, 1, 2, 3}, {1, 0, 3, 2}, {2, 3, 0, 1}, {3, 2, 1, 0}};
+// value of part r's functions under group element g
+constexpr int kChar[4][4] = {{1, 1, 1, 1}, {1, 1, -1, -1}, {1, -1, 1, -1}, {1, -1, -1, 1}};
+// Operators whose entries outside the block pattern exceed this fraction of
+// the largest entry are not symmetric and keep the general kernels.  FP64
+// operators assembled in FP64 stay below 4e-15 at orders 1-4.
+constexpr double kAsymmetry = 5e-14;
+
+struct Vec {  // one symmetric combination of nodes or face points
+  int n = 0;
+  int idx[4];
+  int sign[4];
+};
+
+Vec combo(const int* orbit, int n, int part) {
+  Vec v;
+  v.n = n;
+  for (int k = 0; k < n; ++k) {
+    v.idx[k] = orbit[k];
+    v.sign[k] = n == 4 ? kChar[part][k] : (k == 0 || part == 0 ? 1 : -1);
+  }
+  return v;
+}
+
+template <int N>
+int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool strong,
+         unsigned char* out, int out_bytes) {
+  using B = sym::Basis<N>;
+  using O = sym::Ops<N>;
+  constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT;
+  if (!out) return O::SIZE;
+  if (out_bytes < O::SIZE) return -1;
+
+  // {{{ action of the group on nodes (barycentric multi-indices, first index
+  // fastest) and on face points
+  int alpha[NP][4], perm[4][NP];
+  {
+    int n = 0;
+    for (int k = 0; k <= N; ++k)
+      for (int j = 0; j <= N - k; ++j)
+        for (int i = 0; i <= N - k - j; ++i, ++n) {
+          alpha[n][0] = N - i - j - k;
+          alpha[n][1] = i;
+          alpha[n][2] = j;
+          alpha[n][3] = k;
+        }
+  }
+  for (int g = 0; g < 4; ++g)
+    for (int n = 0; n < NP; ++n)
+      for (int m = 0; m < NP; ++m) {
+        bool same = true;
+        for (int v = 0; v < 4; ++v) same = same && alpha[m][v] == alpha[n][kGroup[g][v]];
+        if (same) perm[g][n] = m;
+      }
+  int fperm[4][NFPT];
+  for (int g = 0; g < 4; ++g)
+    for (int f = 0; f < 4; ++f) {
+      int target = -1;
+      for (int f2 = 0; f2 < 4 && target < 0; ++f2) {
+        bool all = true;
+        for (int j = 0; j < NFP; ++j) {
+          bool found = false;
+          for (int j2 = 0; j2 < NFP; ++j2)
+            found = found || face_nodes[f2 * NFP + j2] == perm[g][face_nodes[f * NFP + j]];
+          all = all && found;
+        }
+        if (all) target = f2;
+      }
+      if (target < 0 || (g > 0 && target == f)) return -1;  // not the faces of a tetrahedron
+      for (int j = 0; j < NFP; ++j) {
+        int hit = -1;
+        for (int j2 = 0; j2 < NFP; ++j2)
+          if (face_nodes[target * NFP + j2] == perm[g][face_nodes[f * NFP + j]]) hit = j2;
+        fperm[g][f * NFP + j] = target * NFP + hit;
+      }
+    }
+  // }}}
+
+  // {{{ orbits, slots and the symmetric combinations
+  Vec node[NP];                     // by slot
+  int part_of[NP], node_slot[NP];
+  {
+    bool seen[NP] = {};
+    int nfull = 0, npair[4] = {}, nsingle = 0;
+    for (int n = 0; n < NP; ++n) {
+      if (seen[n]) continue;
+      int orbit[4];
+      for (int g = 0; g < 4; ++g) orbit[g] = perm[g][n];
+      for (int g = 0; g < 4; ++g) seen[orbit[g]] = true;
+      int fix = 0, nfix = 0;
+      for (int g = 1; g < 4; ++g)
+        if (orbit[g] == n) fix = g, ++nfix;
+      if (nfix == 0) {
+        for (int r = 0; r < 4; ++r) {
+          const int slot = r == 0 ? nfull : B::DA + (r - 1) * B::DB + nfull;
+          node[slot] = combo(orbit, 4, r);
+          part_of[slot] = r;
+          node_slot[orbit[r]] = slot;
+        }
+        ++nfull;
+      } else if (nfix == 1) {
+        const int pair[2] = {n, orbit[fix == 1 ? 2 : 1]};
+        const int sa = B::NO4 + fix - 1, sb = B::DA + (fix - 1) * B::DB + B::NO4;
+        node[sa] = combo(pair, 2, 0);
+        node[sb] = combo(pair, 2, 1);
+        part_of[sa] = 0;
+        part_of[sb] = fix;
+        node_slot[pair[0]] = sa;
+        node_slot[pair[1]] = sb;
+        ++npair[fix];
+      } else {
+        node[B::DA - 1] = combo(orbit, 1, 0);
+        part_of[B::DA - 1] = 0;
+        node_slot[n] = B::DA - 1;
+        ++nsingle;
+      }
+    }
+    if (nfull != B::NO4 || npair[1] != B::NPR || npair[2] != B::NPR || npair[3] != B::NPR ||
+        nsingle != B::NSG)
+      return -1;
+  }
+  Vec face[NFPT];
+  int face_slot[NFPT];
+  for (int o = 0; o < NFP; ++o) {   // orbit o starts at point o of face 0
+    int orbit[4];
+    for (int g = 0; g < 4; ++g) orbit[g] = fperm[g][o];
+    for (int r = 0; r < 4; ++r) {
+      face[r * NFP + o] = combo(orbit, 4, r);
+      face_slot[orbit[r]] = r * NFP + o;
+    }
+  }
+  // }}}
+
+  // an operator of `cols` columns in the combinations' basis (outputs by node
+  // slot, inputs by slot of `in`), normalised for plain sums on both sides
+  std::vector<long double> half, full;
+  auto to_basis = [&](const Vec* in, int cols, auto at) {
+    half.assign((size_t)NP * cols, 0.0L);
+    full.assign((size_t)NP * cols, 0.0L);
+    for (int i = 0; i < NP; ++i)
+      for (int a = 0; a < node[i].n; ++a)
+        for (int c = 0; c < cols; ++c)
+          half[(size_t)i * cols + c] += node[i].sign[a] * at(node[i].idx[a], c);
+    for (int i = 0; i < NP; ++i)
+      for (int c = 0; c < cols; ++c) {
+        long double s = 0.0L;
+        for (int b = 0; b < in[c].n; ++b)
+          s += in[c].sign[b] * half[(size_t)i * cols + in[c].idx[b]];
+        full[(size_t)i * cols + c] = s / (node[i].n * in[c].n);
+      }
+  };
+  // whether the entries outside the pattern vanish to rounding
+  auto symmetric = [&](int cols, auto inside) {
+    long double big = 0.0L, off = 0.0L;
+    for (int i = 0; i < NP; ++i)
+      for (int c = 0; c < cols; ++c) {
+        const long double x = std::fabs(full[(size_t)i * cols + c]);
+        if (!std::isfinite(x)) return false;
+        long double& m = inside(i, c) ? big : off;
+        if (x > m) m = x;
+      }
+    return off <= kAsymmetry * big;
+  };
+  auto slot0 = [](int r) { return r == 0 ? 0 : B::DA + (r - 1) * B::DB; };
+  auto dim = [](int r) { return r == 0 ? B::DA : B::DB; };
+
+  std::memset(out, 0, O::SIZE);
+  double* ops = reinterpret_cast<double*>(out);
+  for (int k = 1; k < 4; ++k) {
+    // D'_k = -1/2 (D_k - D_other - D_other')
+    to_basis(node, NP, [&](int i, int j) {
+      long double s = 0.0L;
+      for (int r = 0; r < 3; ++r) {
+        const long double d = diff[(size_t)(r * NP + i) * NP + j];
+        s += r == k - 1 ? -0.5L * d : 0.5L * d;
+      }
+      return s;
+    });
+    // order 1: one block per direction (strong: into part 0, weak: from it)
+    if (!symmetric(NP, [&](int i, int j) {
+          const int ri = part_of[i], rj = part_of[j];
+          return (ri ^ rj) == k && (N != 1 || (strong ? ri : rj) == 0);
+        }))
+      return -1;
+    for (int r = 0; r < 4; ++r) {
+      const int pitch = r == 0 ? O::PA : O::PB, s = r ^ k;
+      int row = 0;                  // rows of part r before direction k
+      for (int k2 = 1; k2 < k; ++k2) row += dim(r ^ k2);
+      double* dst = ops + (r == 0 ? 0 : O::VOL0 + (r - 1) * O::VOLB) + row * pitch;
+      for (int j = 0; j < dim(s); ++j)
+        for (int i = 0; i < dim(r); ++i)
+          dst[j * pitch + i] = (double)full[(size_t)(slot0(r) + i) * NP + slot0(s) + j];
+    }
+  }
+  to_basis(face, NFPT,
+           [&](int i, int fj) { return (long double)lift[(size_t)i * NFPT + fj]; });
+  if (!symmetric(NFPT, [&](int i, int c) { return part_of[i] == c / NFP; })) return -1;
+  for (int r = 0; r < 4; ++r) {
+    const int pitch = r == 0 ? O::PA : O::PB;
+    double* dst = ops + (r == 0 ? O::LIFT : O::LIFTB + (r - 1) * NFP * O::PB);
+    for (int o = 0; o < NFP; ++o)
+      for (int i = 0; i < dim(r); ++i)
+        dst[o * pitch + i] = (double)full[(size_t)(slot0(r) + i) * NFPT + r * NFP + o];
+  }
+  int32_t* ns = reinterpret_cast<int32_t*>(out + O::NODE_SLOT);
+  int32_t* fp = reinterpret_cast<int32_t*>(out + O::FACE_POINT);
+  for (int n = 0; n < NP; ++n) ns[n] = node_slot[n];
+  for (int fj = 0; fj < NFPT; ++fj) fp[face_slot[fj]] = fj;
+  return O::SIZE;
+}
+
+}  // namespace
+
+int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
+                 bool strong, unsigned char* out, int out_bytes) {
+  switch (order) {
+    case 1: return pack<1>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 2: return pack<2>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 3: return pack<3>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 4: return pack<4>(diff, lift, face_nodes, strong, out, out_bytes);
+    default: return -1;
+  }
+}
+
+}  // namespace dg

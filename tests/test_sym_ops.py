@@ -1,0 +1,200 @@
+"""The symmetry-adapted operator blocks (``pack_sym_ops``): applied to the
+transformed inputs they reproduce the dense derivative and LIFT products, and
+operators without the tetrahedron's symmetry are refused (such plans keep the
+general kernels).  The block product is restated here in NumPy."""
+
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from actx_dgfem_suite_gb300 import _lib
+from actx_dgfem_suite_gb300.refelem import reference_tet
+
+EPS = np.finfo(np.float64).eps
+
+
+def _pack(order, diff, lift, face_nodes, strong):
+    f = ctypes.CDLL(str(_lib.library_path()))._ZN2dg12pack_sym_opsEiPKdS1_PKibPhi
+    f.restype = ctypes.c_int
+    diff, lift = np.ascontiguousarray(diff), np.ascontiguousarray(lift)
+    fn = np.ascontiguousarray(face_nodes, dtype=np.int32)
+    ptr = [ctypes.c_void_p(x.ctypes.data) for x in (diff, lift, fn)]
+    size = f(ctypes.c_int(order), *ptr, ctypes.c_bool(strong), None, 0)
+    buf = np.zeros(size, dtype=np.uint8)
+    got = f(ctypes.c_int(order), *ptr, ctypes.c_bool(strong),
+            ctypes.c_void_p(buf.ctypes.data), size)
+    return buf if got == size else None
+
+
+class _Blocks:
+    """The operator block of order N read back in the kernel's layout."""
+
+    def __init__(self, order, buf):
+        self.np_ = (order + 1) * (order + 2) * (order + 3) // 6
+        self.nfp = (order + 1) * (order + 2) // 2
+        npr, nsg = int(order % 2 == 0), int(order == 4)
+        self.no4 = (self.np_ - 6 * npr - nsg) // 4
+        self.npr, self.db, self.da = npr, self.no4 + npr, self.no4 + 3 * npr + nsg
+        even = lambda n: (n + 1) & ~1  # noqa: E731
+        pitch = [even(self.da)] + 3 * [even(self.db)]
+        dim = [self.da] + 3 * [self.db]
+        self.slot0 = [0] + [self.da + k * self.db for k in range(3)]
+        x = buf.view(np.float64) if buf.size % 8 == 0 else None
+        pos = 0
+        self.vol, self.lift = {}, {}
+        for r in range(4):
+            for k in range(1, 4):
+                n = dim[r ^ k] * pitch[r]
+                self.vol[r, k] = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
+                pos += n
+        for r in range(4):
+            n = self.nfp * pitch[r]
+            self.lift[r] = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
+            pos += n
+        tab = buf.view(np.int32)
+        pos *= 2
+        self.node_slot = tab[pos:pos + self.np_]
+        pos += (self.np_ + 3) // 4 * 4
+        self.face_point = tab[pos:pos + 4 * self.nfp]
+        self.dim = dim
+
+    def transform(self, x):
+        """In place on slots (last axis); applying it twice scales by 4, 2, 1."""
+        h = np.array([[1, 1, 1, 1], [1, 1, -1, -1], [1, -1, 1, -1], [1, -1, -1, 1.0]])
+        for o in range(self.no4):
+            s = [o] + [self.slot0[k] + o for k in (1, 2, 3)]
+            x[..., s] = x[..., s] @ h
+        for k in range(3 * self.npr):
+            s = [self.no4 + k, self.slot0[k + 1] + self.no4]
+            x[..., s] = x[..., s] @ np.array([[1, 1], [1, -1.0]])
+        return x
+
+    def part(self, r):
+        return slice(self.slot0[r], self.slot0[r] + self.dim[r])
+
+
+@pytest.mark.parametrize("strong", [False, True])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_blocks_reproduce_the_dense_operators(order, strong):
+    ref = reference_tet(order)
+    diff = ref.diff if strong else ref.weak_diff
+    b = _Blocks(order, _pack(order, diff, ref.lift, ref.face_nodes, strong))
+    assert sorted(b.node_slot) == list(range(b.np_))
+    assert sorted(b.face_point) == list(range(4 * b.nfp))
+    rng = np.random.default_rng(order)
+    x = rng.standard_normal((7, b.np_))
+    g = rng.standard_normal((3, 7, 1))           # one metric row per direction
+    xs = np.empty_like(x)
+    xs[:, b.node_slot] = x
+    xs = b.transform(xs)
+    h = [g[1] + g[2], g[0] + g[2], g[0] + g[1]]
+    ys = np.zeros_like(xs)
+    for r in range(4):
+        for k in (1, 2, 3):
+            if order == 1 and (r if strong else r ^ k) != 0:
+                continue                         # not evaluated by the kernel
+            ys[:, b.part(r)] += h[k - 1] * (xs[:, b.part(r ^ k)] @ b.vol[r, k].T)
+    y = b.transform(ys)[:, b.node_slot]
+    dense = sum(g[r] * (x @ diff[r].T) for r in range(3))
+    # sums of 3 Np products of unit-size entries on either side
+    scale = sum(np.abs(g[r]) * (np.abs(x) @ np.abs(diff[r]).T) for r in range(3))
+    assert np.all(np.abs(y - dense) <= 3 * b.np_ * EPS * scale.max())
+
+    f = rng.standard_normal((7, 4 * b.nfp))
+    h4 = np.array([[1, 1, 1, 1], [1, 1, -1, -1], [1, -1, 1, -1], [1, -1, -1, 1.0]])
+    fs = np.einsum("rg,ego->ero", h4, f[:, b.face_point].reshape(7, 4, b.nfp))
+    ys = np.zeros_like(xs)
+    for r in range(4):
+        ys[:, b.part(r)] = fs[:, r] @ b.lift[r].T
+    y = b.transform(ys)[:, b.node_slot]
+    lift = ref.lift.reshape(b.np_, -1)
+    scale = (np.abs(f) @ np.abs(lift).T).max()
+    assert np.all(np.abs(y - f @ lift.T) <= 4 * b.nfp * EPS * scale)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_operators_without_the_symmetry_are_refused(order):
+    ref = reference_tet(order)
+    fn = ref.face_nodes
+    for which in ("diff", "lift", "nodes", "nan"):
+        diff, lift, nodes = ref.weak_diff.copy(), ref.lift.copy(), fn.copy()
+        if which == "diff":
+            diff[1, 0, -1] += 1e-9 * np.abs(diff).max()
+        elif which == "lift":
+            lift.reshape(-1)[3] += 1e-9 * np.abs(lift).max()
+        elif which == "nan":
+            diff[2, -1, 0] = np.nan
+        else:                                    # a face that is not one
+            nodes[0] = nodes[1]
+        assert _pack(order, diff, lift, nodes, False) is None, which
+    # another node order: the symmetry does not hold in this order's group action
+    p = np.roll(np.arange(ref.np_), 1)
+    diff = ref.weak_diff[:, p][:, :, p]
+    lift = ref.lift[p]
+    inv = np.argsort(p)
+    got = _pack(order, diff, lift, inv[fn], False)
+    if got is not None:                          # order 1: any order of four vertices
+        assert order == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("equation,order", [("wave", 1), ("wave", 4), ("euler", 2),
+                                            ("euler", 3), ("maxwell", 3), ("maxwell", 4)])
+def test_asymmetric_operators_take_the_general_kernel(equation, order):
+    """An FP64 plan on the face-shared path whose operators lack the symmetry
+    still evaluates them as given: equal to the fused kernel's result."""
+    import torch
+
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import jittered_box_mesh, make_problem
+    prob = make_problem(equation, jittered_box_mesh(3), order, seed=order)
+    q = torch.from_numpy(prob.fields).cuda()
+    out = []
+    for partner in (True, False):
+        dm = DeviceMesh(prob.disc, "cuda:0", with_partner=partner)
+        for name in ("_weak", "_strong", "_lift"):
+            ops = getattr(dm, name).copy()
+            ops.reshape(-1)[::7] *= 1.01
+            setattr(dm, name, ops)
+        plan = DevicePlan(dm, equation, prob.params, "fp64")
+        out.append(plan.rhs(q))
+        plan.finish()
+    sym = DevicePlan(DeviceMesh(prob.disc, "cuda:0"), equation, prob.params, "fp64").rhs(q)
+    norm = float(torch.linalg.norm(out[1]))
+    assert float(torch.linalg.norm(out[0] - out[1])) <= 1e-12 * norm
+    assert float(torch.linalg.norm(sym - out[1])) > 1e-6 * norm   # not the same operator
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("equation", ["wave", "euler", "maxwell"])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("nel", [1, 15, 16, 17, 31, 32, 33, 65])
+def test_tile_edges_match_the_general_kernel(equation, order, nel):
+    """Element counts around the tile sizes (16 and 32 elements), RHS and RK
+    stage with element scale: equal to the fused general kernel."""
+    import torch
+
+    from actx_dgfem_suite_gb300.mesh import TetMesh
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import jittered_box_mesh, make_problem
+    mesh = jittered_box_mesh(3)
+    mesh = TetMesh(vertices=mesh.vertices, elements=mesh.elements[:nel])
+    prob = make_problem(equation, mesh, order, seed=nel)
+    q = torch.from_numpy(prob.fields).cuda()
+    scale = torch.linspace(0.8, 1.2, nel, dtype=torch.float64, device="cuda")
+    got = []
+    for partner in (True, False):
+        plan = DevicePlan(DeviceMesh(prob.disc, "cuda:0", with_partner=partner), equation,
+                          prob.params, "fp64")
+        r = plan.rhs(q)
+        plan.set_element_scale(scale)
+        res, qo, un = 0.5 * q, torch.empty_like(q), torch.empty_like(q)
+        plan.rk_stage(q, qo, res, 0.3, 0.7, 1e-2, rhs_unscaled=un)
+        plan.finish()
+        got.append((r, res, qo, un))
+    for a, b in zip(*got):
+        # two orders of summation of the same products: 1e-12 as the parity bound
+        assert float(torch.linalg.norm(a - b)) <= 1e-12 * float(torch.linalg.norm(b))
