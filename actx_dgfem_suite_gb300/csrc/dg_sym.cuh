@@ -32,9 +32,9 @@
 //
 // Measured (GB300, CUDA events, whole RHS with its face kernel, dense kernel
 // before -> now): Maxwell P4 584,016 tets 38.9 -> 14.3 ms, Euler P4 118,098 tets
-// 7.08 -> 3.57 ms, wave P3 215,622 tets 2.69 -> 1.27 ms, Euler P2 LSRK step
-// 413,526 tets 16.7 -> 11.6 ms, wave P1 5.14 M tets 5.77 -> 4.56 ms.  The kernel
-// runs at 72-88 % of the FP64 pipe's rate by operation count.
+// 7.08 -> 2.92 ms, wave P3 215,622 tets 2.69 -> 1.26 ms, Euler P2 LSRK step
+// 413,526 tets 16.7 -> 11.1 ms, wave P1 5.14 M tets 5.77 -> 4.56 ms.  ncu: FP64
+// pipe 83 % (wave P1) to 92 % (Maxwell P4) busy.
 //
 // Work split: a tile of E elements with one lane per element and one warp per
 // part rho, so that every operator entry is the same for a whole warp and is
@@ -65,9 +65,9 @@ struct Basis {
 
 // Operator block: doubles in rows of one input each, padded to 16 bytes.
 // Volume blocks of part 0, then 1, 2, 3, each for k = 1, 2, 3 (inputs of part
-// rho xor k); LIFT blocks the same way (NFP inputs).  Then two int32 tables:
-// node -> slot, and the face point of every face slot (part r of orbit o at
-// r NFP + o).
+// rho xor k); LIFT blocks the same way (NFP inputs).  Then three int32 tables:
+// node -> slot, slot -> node, and the face point of every face slot (part r of
+// orbit o at r NFP + o).
 template <int N>
 struct Ops {
   using B = Basis<N>;
@@ -78,27 +78,32 @@ struct Ops {
   static constexpr int LIFTB = LIFT + B::NFP * PA;
   static constexpr int ENTRIES = LIFTB + 3 * B::NFP * PB;
   static constexpr int NODE_SLOT = ENTRIES * 8;             // bytes from here
-  static constexpr int FACE_POINT = NODE_SLOT + pad16(B::NP * 4);
+  static constexpr int SLOT_NODE = NODE_SLOT + pad16(B::NP * 4);
+  static constexpr int FACE_POINT = SLOT_NODE + pad16(B::NP * 4);
   static constexpr int SIZE = FACE_POINT + pad16(B::NFPT * 4);
 };
 
 // Tile shape.  Maxwell's E and H equations have the same form, so the two
-// halves of a warp take one each: 16 elements per tile, and the order-4 tile
-// (49 KB) fits four times on an SM.  Wave and Euler keep all fields in a
-// thread and 32 elements per tile.  Face values and result reuse the state's
-// arrays.
+// halves of a warp take one each, on 16 elements per tile; wave and Euler keep
+// all fields in a thread and 32 elements per tile.  Face values and result
+// reuse the state's arrays; from order 2 on the face values come in two chunks
+// of orbits, so that a tile's shared memory is little more than its state and
+// three to four CTAs share an SM at order 4: their phases (loads, transforms,
+// products) must overlap to keep the FP64 pipe busy.
 template <int N, int EQ>
 struct Tile {
   using B = Basis<N>;
   static constexpr int NF = EqInfo<EQ>::NF;
-  static constexpr int NX = EQ == DG_EULER ? 12 : NF;       // euler: flux components
   static constexpr int GROUPS = EQ == DG_MAXWELL ? 2 : 1;
   static constexpr int NA = NF / GROUPS;                    // fields of a thread
   static constexpr int E = 32 / GROUPS, PE = E + 1;
   static constexpr int BLOCK = 128;
+  // CTAs per SM the registers must allow (order-4 Euler: 168 instead of 186)
+  static constexpr int MIN_CTAS = N == 4 ? 3 : 4;
+  static constexpr int CH = N == 1 ? B::NFP : (B::NFP + 1) / 2;  // orbits of a chunk
   static constexpr int X = Ops<N>::SIZE;
-  static constexpr int X_BYTES = pad16(NX * B::NP * PE * 8);
-  static constexpr int F_BYTES = pad16(NF * B::NFPT * PE * 8);
+  static constexpr int X_BYTES = pad16(NF * B::NP * PE * 8);
+  static constexpr int F_BYTES = pad16(NF * 4 * CH * PE * 8);
   static constexpr int H = X + (X_BYTES > F_BYTES ? X_BYTES : F_BYTES);
   static constexpr int SMEM = H + pad16(9 * PE * 8);
 };
@@ -131,9 +136,10 @@ __device__ __forceinline__ void load_row(const double* p, double (&r)[P]) {
   }
 }
 
-// Volume term of part rho (D outputs, row pitch P).  x: the thread's element
-// in shared memory; h: metric of the three directions (pitch PE per entry);
-// f0: first input field (Maxwell); sgn: Maxwell's curl sign, wave's -c.
+// Volume term of part rho (D outputs, row pitch P), wave and Maxwell.  x: the
+// thread's element in shared memory; h: metric of the three directions (pitch
+// PE per entry); f0: first input field (Maxwell); sgn: Maxwell's curl sign,
+// wave's -c.
 template <int N, int EQ, int D, int P>
 __device__ __forceinline__ void volume(const double* __restrict__ x,
                                        const double* __restrict__ h,
@@ -176,22 +182,6 @@ __device__ __forceinline__ void volume(const double* __restrict__ x,
         acc[2][i] = fma(h1, g[i], acc[2][i]);
         acc[3][i] = fma(h2, g[i], acc[3][i]);
       }
-    } else if constexpr (EQ == DG_EULER) {
-      // arrays 0-2: m; 3-5: (E + p) u; 6-11: m u + p (xx, xy, xz, yy, yz, zz)
-      constexpr int S[5][3] = {{0, 1, 2}, {3, 4, 5}, {6, 7, 8}, {7, 9, 10}, {8, 10, 11}};
-#pragma unroll 1
-      for (int j = 0; j < din; ++j, row += P, xs += PE) {
-        double v[12], t[P];
-#pragma unroll
-        for (int m = 0; m < 12; ++m) v[m] = xs[m * FS];
-        load_row<P>(row, t);
-#pragma unroll
-        for (int f = 0; f < 5; ++f) {
-          const double w = fma(h0, v[S[f][0]], fma(h1, v[S[f][1]], h2 * v[S[f][2]]));
-#pragma unroll
-          for (int i = 0; i < D; ++i) acc[f][i] = fma(t[i], w, acc[f][i]);
-        }
-      }
     } else {
       const double* xf = xs + f0 * FS;
 #pragma unroll 1
@@ -213,19 +203,17 @@ __device__ __forceinline__ void volume(const double* __restrict__ x,
   }
 }
 
-// LIFT of part rho: f is the thread's element at its part's first face slot
-// (and first output field).
-template <int N, int EQ, int D, int P>
-__device__ __forceinline__ void lift(const double* __restrict__ f,
-                                     const double* __restrict__ row,
-                                     double (&acc)[Tile<N, EQ>::NA][D]) {
-  using B = Basis<N>;
-  constexpr int PE = Tile<N, EQ>::PE, FS = B::NFPT * PE, NA = Tile<N, EQ>::NA;
+// acc += block * fields for `rows` inputs: x is the thread's element at the
+// first input of the first field, FS the field stride.
+template <int NA, int D, int P, int PE, int FS>
+__device__ __forceinline__ void block_product(const double* __restrict__ x,
+                                              const double* __restrict__ row, int rows,
+                                              double (&acc)[NA][D]) {
 #pragma unroll 1
-  for (int o = 0; o < B::NFP; ++o, row += P, f += PE) {
+  for (int j = 0; j < rows; ++j, row += P, x += PE) {
     double v[NA], t[P];
 #pragma unroll
-    for (int m = 0; m < NA; ++m) v[m] = f[m * FS];
+    for (int m = 0; m < NA; ++m) v[m] = x[m * FS];
     load_row<P>(row, t);
 #pragma unroll
     for (int m = 0; m < NA; ++m)
@@ -256,78 +244,94 @@ __device__ __forceinline__ void transform(double* x, int narrays) {
   }
 }
 
-// Euler: node state (arrays 0-4), pressure (5) and 1/rho (6) to the twelve
-// flux components, transformed, in place.
-template <int N, int PE, int E, int BLOCK>
-__device__ __forceinline__ void euler_inputs(double* x) {
+// Euler: the five fluxes along direction k (metric row h_k), transformed.  With
+// U = h.m / rho: h.m, (E + p) U and m_c U + p h_c, 12 operations per node.  The
+// state is read from memory once per direction (twice from L2): with the
+// twelve flux components in shared memory instead (82 operations per node with
+// the metric combinations, here 66) one CTA fitted on an SM at order 4 and the
+// FP64 pipe was 74 % busy (kernel at P4, 118,098 tets: 2.89 ms, now 2.24; RK
+// stage at P2, 413,526 tets: 1.47 ms, now 1.37).
+// Orbits of the same length go to the same warps (an FP64 instruction costs the
+// pipe a whole warp's time however many of its lanes are active).
+template <int N>
+__device__ __forceinline__ void euler_inputs(const RhsArgs& a, int64_t e0, int ecount, int k,
+                                             const int* __restrict__ slot_node,
+                                             const double* __restrict__ sH, double* sX) {
   using B = Basis<N>;
-  constexpr int NO = B::NO4 + 3 * B::NPR + B::NSG, FS = B::NP * PE;
-  const int le = threadIdx.x % E;
-  for (int o = threadIdx.x / E; o < NO; o += BLOCK / E) {
-    const int pair = o - B::NO4;                 // 0-2: pairs, 3: the centroid
-    const int cnt = NO == B::NO4 || pair < 0 ? 4 : (pair < 3 ? 2 : 1);
-    double* p[4];
-    p[0] = x + o * PE + le;
-    p[1] = x + (pair < 0 ? B::DA + o : B::DA + pair * B::DB + B::NO4) * PE + le;
-    p[2] = x + (B::DA + B::DB + o) * PE + le;
-    p[3] = x + (B::DA + 2 * B::DB + o) * PE + le;
-    double m[4][3], u[4][3], pr[4], ep[4];
+  using T = Tile<N, DG_EULER>;
+  constexpr int PE = T::PE, XS = B::NP * PE, DA = B::DA, DB = B::DB, NO4 = B::NO4;
+  const int64_t nelnp = a.nel * B::NP;
+  // the orbit of CNT nodes at the given slots, element el of the tile
+  auto orbit = [&](auto tag, int el, int s0, int s1, int s2, int s3) {
+    constexpr int CNT = decltype(tag)::value;
+    const int slot[4] = {s0, s1, s2, s3};
+    const double* h = sH + k * 3 * PE + el;
+    const double h0 = h[0], h1 = h[PE], h2 = h[2 * PE];
+    double f[5][CNT];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      if (n >= cnt) break;
-      const double rinv = p[n][6 * FS];
-      pr[n] = p[n][5 * FS];
-      ep[n] = p[n][FS] + pr[n];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        m[n][c] = p[n][(2 + c) * FS];
-        u[n][c] = m[n][c] * rinv;
+    for (int n = 0; n < CNT; ++n) {
+      double en = 0.0, m0 = 0.0, m1 = 0.0, m2 = 0.0, p = 0.0, rinv = 0.0;
+      if (el < ecount) {
+        const int64_t g = (e0 + el) * B::NP + slot_node[slot[n]];
+        const double* q = a.q + nelnp + g;
+        en = __ldg(q);
+        m0 = __ldg(q + nelnp);
+        m1 = __ldg(q + 2 * nelnp);
+        m2 = __ldg(q + 3 * nelnp);
+        p = __ldg(a.aux + g);
+        rinv = __ldg(a.aux + nelnp + g);
       }
+      const double hm = fma(h0, m0, fma(h1, m1, h2 * m2));
+      const double u = hm * rinv;
+      f[0][n] = hm;
+      f[1][n] = (en + p) * u;
+      f[2][n] = fma(m0, u, p * h0);
+      f[3][n] = fma(m1, u, p * h1);
+      f[4][n] = fma(m2, u, p * h2);
     }
-    auto put = [&](int arr, auto val) {
-      if (cnt == 4) {
-        double v0 = val(0), v1 = val(1), v2 = val(2), v3 = val(3);
-        butterfly(v0, v1, v2, v3);
-        p[0][arr * FS] = v0;
-        p[1][arr * FS] = v1;
-        p[2][arr * FS] = v2;
-        p[3][arr * FS] = v3;
-      } else if (cnt == 2) {
-        const double v0 = val(0), v1 = val(1);
-        p[0][arr * FS] = v0 + v1;
-        p[1][arr * FS] = v0 - v1;
-      } else {
-        p[0][arr * FS] = val(0);
+    double* x = sX + el;
+#pragma unroll
+    for (int m = 0; m < 5; ++m, x += XS) {
+      if constexpr (CNT == 4) {
+        butterfly(f[m][0], f[m][1], f[m][2], f[m][3]);
+      } else if constexpr (CNT == 2) {
+        const double s = f[m][0] + f[m][1], d = f[m][0] - f[m][1];
+        f[m][0] = s;
+        f[m][1] = d;
       }
-    };
 #pragma unroll
-    for (int c = 0; c < 3; ++c) put(c, [&](int n) { return m[n][c]; });
-#pragma unroll
-    for (int c = 0; c < 3; ++c) put(3 + c, [&](int n) { return ep[n] * u[n][c]; });
-    int arr = 6;
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int d = c; d < 3; ++d, ++arr)
-        put(arr, [&](int n) {
-          return c == d ? fma(m[n][c], u[n][d], pr[n]) : m[n][c] * u[n][d];
-        });
+      for (int n = 0; n < CNT; ++n) x[slot[n] * PE] = f[m][n];
+    }
+  };
+  for (int idx = threadIdx.x; idx < T::E * NO4; idx += T::BLOCK) {
+    const int el = idx / NO4, o = idx - el * NO4;
+    orbit(std::integral_constant<int, 4>{}, el, o, DA + o, DA + DB + o, DA + 2 * DB + o);
   }
+  if constexpr (B::NPR > 0)  // backwards, so that other warps take these
+    for (int idx = T::BLOCK - 1 - threadIdx.x; idx < T::E * 3; idx += T::BLOCK) {
+      const int el = idx / 3, d = idx - el * 3;
+      orbit(std::integral_constant<int, 2>{}, el, NO4 + d, DA + d * DB + NO4, 0, 0);
+    }
+  if constexpr (B::NSG > 0)
+    for (int el = threadIdx.x; el < T::E; el += T::BLOCK)
+      orbit(std::integral_constant<int, 1>{}, el, DA - 1, 0, 0, 0);
 }
 
 template <int N, int EQ, bool STAGE>
-__global__ void __launch_bounds__(Tile<N, EQ>::BLOCK) dg_rhs_sym_kernel(const RhsArgs a) {
+__global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
+    dg_rhs_sym_kernel(const RhsArgs a) {
   using T = Tile<N, EQ>;
   using O = Ops<N>;
   using B = Basis<N>;
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT, NF = T::NF, NA = T::NA;
   constexpr int E = T::E, PE = T::PE, BLOCK = T::BLOCK;
-  constexpr int XS = NP * PE, FS = NFPT * PE;  // array strides
+  constexpr int XS = NP * PE, CH = T::CH, FS = 4 * CH * PE;  // array strides
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t bar;
   __shared__ int ops_ok;
   const double* ops = reinterpret_cast<const double*>(smem);
   const int* node_slot = reinterpret_cast<const int*>(smem + O::NODE_SLOT);
+  [[maybe_unused]] const int* slot_node = reinterpret_cast<const int*>(smem + O::SLOT_NODE);
   const int* face_point = reinterpret_cast<const int*>(smem + O::FACE_POINT);
   double* sX = reinterpret_cast<double*>(smem + T::X);
   double* sH = reinterpret_cast<double*>(smem + T::H);
@@ -358,23 +362,20 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK) dg_rhs_sym_kernel(const Rh
     const int64_t e0 = tile * E;
     const int ecount = (nel - e0) < (int64_t)E ? (int)(nel - e0) : E;
 
-    // {{{ state and metric -> shared memory, then the volume term's inputs
+    // {{{ metric and (wave, Maxwell) state -> shared memory, transformed
     {
-      const double* qk = a.q + e0 * NP;
-      for (int rem = t; rem < E * NP; rem += BLOCK) {
-        const int el = rem / NP;
-        double* x = sX + node_slot[rem - el * NP] * PE + el;
-        const bool in = rem < ecount * NP;
-        double v[NF];
+      if constexpr (EQ != DG_EULER) {
+        const double* qk = a.q + e0 * NP;
+        for (int rem = t; rem < E * NP; rem += BLOCK) {
+          const int el = rem / NP;
+          double* x = sX + node_slot[rem - el * NP] * PE + el;
+          const bool in = rem < ecount * NP;
+          double v[NF];
 #pragma unroll
-        for (int k = 0; k < NF; ++k) v[k] = in ? __ldg(qk + k * nelnp + rem) : 0.0;
-        if constexpr (EQ == DG_EULER) {
-          const double* ax = a.aux + e0 * NP + rem;
-          x[5 * XS] = in ? __ldg(ax) : 0.0;
-          x[6 * XS] = in ? __ldg(ax + nelnp) : 0.0;
+          for (int k = 0; k < NF; ++k) v[k] = in ? __ldg(qk + k * nelnp + rem) : 0.0;
+#pragma unroll
+          for (int k = 0; k < NF; ++k) x[k * XS] = v[k];
         }
-#pragma unroll
-        for (int k = 0; k < NF; ++k) x[k * XS] = v[k];
       }
       const double* mt = a.metric + e0 * 9;
       for (int idx = t; idx < 9 * E; idx += BLOCK) {
@@ -386,9 +387,10 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK) dg_rhs_sym_kernel(const Rh
       }
     }
     __syncthreads();
-    if constexpr (EQ == DG_EULER) euler_inputs<N, PE, E, BLOCK>(sX);
-    else transform<N, PE, E, BLOCK>(sX, NF);
-    __syncthreads();
+    if constexpr (EQ != DG_EULER) {
+      transform<N, PE, E, BLOCK>(sX, NF);
+      __syncthreads();
+    }
     // }}}
 
     // {{{ volume and LIFT blocks, one part per warp.  The parts differ in size
@@ -400,12 +402,13 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK) dg_rhs_sym_kernel(const Rh
     const double sgn = EQ == DG_MAXWELL ? (grp == 0 ? 1.0 : -1.0)
                                         : (EQ == DG_WAVE ? -a.p0 : 1.0);
 
-    // the tile's face values, transformed on the way in
-    auto load_faces = [&]() {
+    // orbits o0 .. o0 + CH - 1 of the tile's face values, transformed
+    auto load_faces = [&](int o0) {
       const int64_t nfpt_all = nel * NFPT;
       const double* fk = a.flux_in + e0 * NFPT;
-      for (int idx = t; idx < E * NFP; idx += BLOCK) {
-        const int el = idx / NFP, o = idx - el * NFP;
+      for (int idx = t; idx < E * CH; idx += BLOCK) {
+        const int el = idx / CH, oc = idx - el * CH, o = o0 + oc;
+        if (NFP % CH != 0 && o >= NFP) continue;
         // the orbit's four points, one per face
         const int p0 = face_point[o], p1 = face_point[NFP + o],
                   p2 = face_point[2 * NFP + o], p3 = face_point[3 * NFP + o];
@@ -423,7 +426,7 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK) dg_rhs_sym_kernel(const Rh
         for (int k = 0; k < NF; ++k) {
           butterfly(v[k][0], v[k][1], v[k][2], v[k][3]);
 #pragma unroll
-          for (int r = 0; r < 4; ++r) sX[k * FS + (r * NFP + o) * PE + el] = v[k][r];
+          for (int r = 0; r < 4; ++r) sX[k * FS + (r * CH + oc) * PE + el] = v[k][r];
         }
       }
     };
@@ -435,12 +438,30 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK) dg_rhs_sym_kernel(const Rh
       for (int m = 0; m < NA; ++m)
 #pragma unroll
         for (int i = 0; i < D; ++i) acc[m][i] = 0.0;
-      volume<N, EQ, D, P>(sX + le, sH + le, vops, rho, f_in, sgn, acc);
-      cta_sync<BLOCK>();  // the state's slots are free
-      load_faces();
-      cta_sync<BLOCK>();
-      lift<N, EQ, D, P>(sX + f_out * FS + rho * NFP * PE + le, lops, acc);
-      cta_sync<BLOCK>();  // every warp has read its inputs
+      if constexpr (EQ == DG_EULER) {
+#pragma unroll 1
+        for (int k = 0; k < 3; ++k) {
+          euler_inputs<N>(a, e0, ecount, k, slot_node, sH, sX);
+          cta_sync<BLOCK>();
+          const int sig = rho ^ (k + 1), din = sig == 0 ? B::DA : B::DB;
+          if (N != 1 || sig == 0)  // order 1: weak derivatives leave part A only
+            block_product<NA, D, P, PE, XS>(
+                sX + (sig == 0 ? 0 : B::DA + (sig - 1) * B::DB) * PE + le, vops, din, acc);
+          vops += din * P;
+          cta_sync<BLOCK>();       // the inputs' slots are free
+        }
+      } else {
+        volume<N, EQ, D, P>(sX + le, sH + le, vops, rho, f_in, sgn, acc);
+        cta_sync<BLOCK>();         // the state's slots are free
+      }
+#pragma unroll 1
+      for (int o0 = 0; o0 < NFP; o0 += CH) {
+        load_faces(o0);
+        cta_sync<BLOCK>();
+        block_product<NA, D, P, PE, FS>(sX + f_out * FS + rho * CH * PE + le, lops + o0 * P,
+                                        NFP - o0 < CH ? NFP - o0 : CH, acc);
+        cta_sync<BLOCK>();         // every warp has read its inputs
+      }
       [[maybe_unused]] const double post = grp == 0 ? a.k[4] : a.k[5];  // 1/eps, 1/mu
 #pragma unroll
       for (int m = 0; m < NA; ++m)

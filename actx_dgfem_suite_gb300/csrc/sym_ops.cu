@@ -218,7 +218,9 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
   }
   int32_t* ns = reinterpret_cast<int32_t*>(out + O::NODE_SLOT);
   int32_t* fp = reinterpret_cast<int32_t*>(out + O::FACE_POINT);
+  int32_t* sn = reinterpret_cast<int32_t*>(out + O::SLOT_NODE);
   for (int n = 0; n < NP; ++n) ns[n] = node_slot[n];
+  for (int n = 0; n < NP; ++n) sn[node_slot[n]] = n;
   for (int fj = 0; fj < NFPT; ++fj) fp[face_slot[fj]] = fj;
   return O::SIZE;
 }

@@ -58,6 +58,8 @@ class _Blocks:
         pos *= 2
         self.node_slot = tab[pos:pos + self.np_]
         pos += (self.np_ + 3) // 4 * 4
+        self.slot_node = tab[pos:pos + self.np_]
+        pos += (self.np_ + 3) // 4 * 4
         self.face_point = tab[pos:pos + 4 * self.nfp]
         self.dim = dim
 
@@ -83,6 +85,7 @@ def test_blocks_reproduce_the_dense_operators(order, strong):
     diff = ref.diff if strong else ref.weak_diff
     b = _Blocks(order, _pack(order, diff, ref.lift, ref.face_nodes, strong))
     assert sorted(b.node_slot) == list(range(b.np_))
+    assert list(b.slot_node[b.node_slot]) == list(range(b.np_))
     assert sorted(b.face_point) == list(range(4 * b.nfp))
     rng = np.random.default_rng(order)
     x = rng.standard_normal((7, b.np_))
