@@ -254,6 +254,9 @@ struct dg_plan {
   void* d_adj_ops = nullptr;
   uint32_t adj_ops_bytes = 0;
   int adj_grid = 0;
+  void* d_adj_sym_ops = nullptr;  // symmetric operators: dg_sym_adjoint.cuh
+  uint32_t adj_sym_ops_bytes = 0;
+  int adj_sym_grid = 0;
 };
 
 namespace {
@@ -1029,6 +1032,31 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     const int64_t atiles = (p->nel + ashape.elems_per_tile - 1) / ashape.elems_per_tile;
     const int64_t afull = (int64_t)nsm * ashape.blocks_per_sm;
     p->adj_grid = (int)(atiles < afull ? atiles : afull);
+
+    std::vector<unsigned char> sops(
+        dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes, nullptr, 0));
+    const int sbytes = dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes, sops.data(),
+                                            (int)sops.size());
+    if (sbytes > 0) {  // the operators have the symmetry
+      dg::LaunchShape sshape;
+      err = equation == DG_WAVE ? dg::adjoint_sym_shape_wave(N, &sshape)
+                                : dg::vjp_sym_shape_euler(N, &sshape);
+      if (err == cudaSuccess) err = cudaMalloc(&p->d_adj_sym_ops, sbytes);
+      if (err == cudaSuccess)
+        err = cudaMemcpy(p->d_adj_sym_ops, sops.data(), sbytes, cudaMemcpyHostToDevice);
+      if (err != cudaSuccess) {
+        dg_plan_destroy(p);
+        return cuda_fail(err, "symmetry-adapted adjoint configuration");
+      }
+      if (sbytes != sshape.ops_bytes || sshape.blocks_per_sm < 1) {
+        dg_plan_destroy(p);
+        return fail(DG_ERR_CUDA, "symmetry-adapted adjoint: layout mismatch or does not fit");
+      }
+      p->adj_sym_ops_bytes = static_cast<uint32_t>(sbytes);
+      const int64_t stiles = (p->nel + sshape.elems_per_tile - 1) / sshape.elems_per_tile;
+      const int64_t sfull = (int64_t)nsm * sshape.blocks_per_sm;
+      p->adj_sym_grid = (int)(stiles < sfull ? stiles : sfull);
+    }
   }
   *plan_out = p;
   return DG_OK;
@@ -1304,6 +1332,9 @@ dg::VjpArgs vjp_args(const dg_plan* p, const double* q, const double* x, double*
   a.nowned = p->nowned;
   a.ops = p->d_adj_ops;
   a.ops_bytes = p->adj_ops_bytes;
+  a.sym_ops = p->d_adj_sym_ops;
+  a.sym_ops_bytes = p->adj_sym_ops_bytes;
+  a.sym_grid = p->adj_sym_grid;
   a.nel = p->nel;
   a.status = p->d_status;
   a.gamma = p->params[0];
@@ -1375,6 +1406,9 @@ int dg_rhs_adjoint(dg_plan* p, const double* x, double* y, double* face_scratch,
   a.face_partner = p->face_partner;
   a.ops = p->d_adj_ops;
   a.ops_bytes = p->adj_ops_bytes;
+  a.sym_ops = p->d_adj_sym_ops;
+  a.sym_ops_bytes = p->adj_sym_ops_bytes;
+  a.sym_grid = p->adj_sym_grid;
   a.nel = p->nel;
   a.status = p->d_status;
   cudaError_t err = dg::adjoint_launch_wave(p->order, a, p->adj_grid, p->nsm,
@@ -1420,6 +1454,9 @@ int dg_rhs_adjoint_stage(dg_plan* p, const double* x, double xscale, double* lam
   a.face_partner = p->face_partner;
   a.ops = p->d_adj_ops;
   a.ops_bytes = p->adj_ops_bytes;
+  a.sym_ops = p->d_adj_sym_ops;
+  a.sym_ops_bytes = p->adj_sym_ops_bytes;
+  a.sym_grid = p->adj_sym_grid;
   a.nel = p->nel;
   a.status = p->d_status;
   a.xscale = xscale;
@@ -1672,7 +1709,7 @@ int dg_plan_destroy(dg_plan* p) {
   for (void* b : {(void*)p->d_owned, (void*)p->d_flux, (void*)p->d_aux,
                   (void*)p->d_tc_ops, p->d_tcm_ops[0], p->d_tcm_ops[1],
                   p->d_tcm_ops[2] != p->d_tcm_ops[1] ? p->d_tcm_ops[2] : nullptr,
-                  (void*)p->d_pres, p->d_sym_ops})
+                  (void*)p->d_pres, p->d_sym_ops, p->d_adj_sym_ops})
     if (b && cudaFree(b) != cudaSuccess) code = DG_ERR_CUDA;
   delete p;
   if (code != DG_OK) return fail(code, "cudaFree failed");

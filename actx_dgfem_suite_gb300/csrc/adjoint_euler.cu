@@ -2,6 +2,7 @@
 // orders 1..4: see dg_adjoint_euler.cuh.
 #include "dg_adjoint_euler.cuh"
 #include "dg_launch.h"
+#include "dg_sym_adjoint.cuh"
 
 namespace dg {
 namespace {
@@ -23,6 +24,22 @@ cudaError_t vjp_shape_n(LaunchShape* out) {
 }
 
 template <int N>
+cudaError_t vjp_sym_shape_n(LaunchShape* out) {
+  using T = sym::AdjTile<N, DG_EULER>;
+  auto* fn = sym::dg_euler_vjp_sym_kernel<N>;
+  cudaError_t err =
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
+  if (err != cudaSuccess) return err;
+  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out->blocks_per_sm, fn, T::BLOCK,
+                                                      T::SMEM);
+  out->smem_bytes = T::SMEM;
+  out->elems_per_tile = T::E;
+  out->ops_bytes = T::O::SIZE;
+  out->threads = T::BLOCK;
+  return err;
+}
+
+template <int N>
 cudaError_t vjp_launch_n(const VjpArgs& a, int grid, int nsm, bool stage, cudaStream_t s) {
   constexpr int NP = Shape<N>::NP, NFP = Shape<N>::NFP;
   const int64_t nodes = a.nel * NP;
@@ -33,7 +50,11 @@ cudaError_t vjp_launch_n(const VjpArgs& a, int grid, int nsm, bool stage, cudaSt
       a.q, const_cast<double*>(a.aux), (uint32_t)nodes, a.gamma);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  dg_euler_vjp_volume<N><<<grid, kBlock, VjpTile<N>::SMEM_BYTES, s>>>(a);
+  using S = sym::AdjTile<N, DG_EULER>;
+  if (a.sym_ops)
+    sym::dg_euler_vjp_sym_kernel<N><<<a.sym_grid, S::BLOCK, S::SMEM, s>>>(a);
+  else
+    dg_euler_vjp_volume<N><<<grid, kBlock, VjpTile<N>::SMEM_BYTES, s>>>(a);
   err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   int64_t fb = (a.nowned * NFP + kFaceBlock - 1) / kFaceBlock;
@@ -57,6 +78,16 @@ cudaError_t vjp_shape_euler(int order, LaunchShape* out) {
     case 2: return vjp_shape_n<2>(out);
     case 3: return vjp_shape_n<3>(out);
     case 4: return vjp_shape_n<4>(out);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t vjp_sym_shape_euler(int order, LaunchShape* out) {
+  switch (order) {
+    case 1: return vjp_sym_shape_n<1>(out);
+    case 2: return vjp_sym_shape_n<2>(out);
+    case 3: return vjp_sym_shape_n<3>(out);
+    case 4: return vjp_sym_shape_n<4>(out);
     default: return cudaErrorInvalidValue;
   }
 }

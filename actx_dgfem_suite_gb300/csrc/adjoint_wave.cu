@@ -1,6 +1,7 @@
 // Adjoint (transpose) kernels of the FP64 wave RHS, orders 1..4.
 #include "dg_adjoint.cuh"
 #include "dg_launch.h"
+#include "dg_sym_adjoint.cuh"
 
 namespace dg {
 namespace {
@@ -26,9 +27,35 @@ cudaError_t adj_shape_n(LaunchShape* out) {
   return cudaSuccess;
 }
 
+template <int N>
+cudaError_t adj_sym_shape_n(LaunchShape* out) {
+  using T = sym::AdjTile<N, DG_WAVE>;
+  out->blocks_per_sm = 1 << 30;
+  for (int stage = 0; stage < 2; ++stage) {  // both forms, the smaller occupancy
+    auto* fn = stage ? sym::dg_wave_adjoint_sym_kernel<N, true>
+                     : sym::dg_wave_adjoint_sym_kernel<N, false>;
+    cudaError_t err =
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
+    int b = 0;
+    if (err == cudaSuccess)
+      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, T::BLOCK, T::SMEM);
+    if (err != cudaSuccess) return err;
+    if (b < out->blocks_per_sm) out->blocks_per_sm = b;
+  }
+  out->smem_bytes = T::SMEM;
+  out->elems_per_tile = T::E;
+  out->ops_bytes = T::O::SIZE;
+  out->threads = T::BLOCK;
+  return cudaSuccess;
+}
+
 template <int N, bool STAGE>
 cudaError_t adj_launch_n(const AdjArgs& a, int grid, int nsm, cudaStream_t s) {
-  dg_wave_adjoint_volume<N, STAGE><<<grid, kBlock, AdjTile<N>::SMEM_BYTES, s>>>(a);
+  using S = sym::AdjTile<N, DG_WAVE>;
+  if (a.sym_ops)
+    sym::dg_wave_adjoint_sym_kernel<N, STAGE><<<a.sym_grid, S::BLOCK, S::SMEM, s>>>(a);
+  else
+    dg_wave_adjoint_volume<N, STAGE><<<grid, kBlock, AdjTile<N>::SMEM_BYTES, s>>>(a);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   const int64_t nodes = a.nel * Shape<N>::NP;
@@ -47,6 +74,16 @@ cudaError_t adjoint_shape_wave(int order, LaunchShape* out) {
     case 2: return adj_shape_n<2>(out);
     case 3: return adj_shape_n<3>(out);
     case 4: return adj_shape_n<4>(out);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t adjoint_sym_shape_wave(int order, LaunchShape* out) {
+  switch (order) {
+    case 1: return adj_sym_shape_n<1>(out);
+    case 2: return adj_sym_shape_n<2>(out);
+    case 3: return adj_sym_shape_n<3>(out);
+    case 4: return adj_sym_shape_n<4>(out);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -53,6 +53,9 @@ struct AdjArgs {
   uint32_t ops_bytes;
   int64_t nel;
   int* status;
+  const void* sym_ops;      // symmetry-adapted operator block (sym::AdjOps), or NULL
+  uint32_t sym_ops_bytes;
+  int sym_grid;
   // STAGE (fused reverse RK stage) only
   double xscale;            // rbar_s = xscale x
   double* lam;              // (4, Nel, Np), updated in place

@@ -44,6 +44,9 @@ struct VjpArgs {
   int64_t nowned;
   const void* ops;          // adjoint operator block (AdjOpsLayout)
   uint32_t ops_bytes;
+  const void* sym_ops;      // symmetry-adapted operator block (sym::AdjOps), or NULL
+  uint32_t sym_ops_bytes;
+  int sym_grid;
   int64_t nel;
   int* status;
   double gamma;

@@ -107,6 +107,11 @@ int pack_tcm_ops(int order, const double* diff, const double* lift,
 int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
                  bool strong, unsigned char* out, int out_bytes);
 
+// The same for the adjoint kernels (sym::AdjOps): transposed weak derivatives
+// and transposed LIFT.
+int pack_sym_adj_ops(int order, const double* weak, const double* lift,
+                     const int32_t* face_nodes, unsigned char* out, int out_bytes);
+
 // Triangle meshes (rhs_2d.cu): shape query and launch of dg_rhs2d_kernel
 // for mode MODE_RHS or MODE_STAGE (FP64), and the operator block
 // [Wt (2 Np Np) | Lt (3 Nfp Np) | int32 edge nodes (3 Nfp)] packed from the
@@ -124,8 +129,12 @@ int set_error(int code, const char* msg);
 
 // Adjoint of the FP64 wave RHS: shape of the volume kernel, and the two
 // launches (volume transpose + lifted face adjoints, then the per-node
-// transposed flux/gather); `nsm` caps the second grid.
+// transposed flux/gather); `nsm` caps the second grid.  With AdjArgs::sym_ops
+// (VjpArgs::sym_ops for Euler) the volume kernel is the one in the
+// symmetry-adapted basis, on sym_grid CTAs; adjoint_sym_shape_*: its shape.
 cudaError_t adjoint_shape_wave(int order, LaunchShape* out);
+cudaError_t adjoint_sym_shape_wave(int order, LaunchShape* out);
+cudaError_t vjp_sym_shape_euler(int order, LaunchShape* out);
 cudaError_t adjoint_launch_wave(int order, const AdjArgs& a, int grid, int nsm,
                                 cudaStream_t s);
 // The same two launches as one fused reverse LSRK stage (AdjArgs' stage

@@ -67,7 +67,14 @@ struct Basis {
 // Volume blocks of part 0, then 1, 2, 3, each for k = 1, 2, 3 (inputs of part
 // rho xor k); LIFT blocks the same way (NFP inputs).  Then three int32 tables:
 // node -> slot, slot -> node, and the face point of every face slot (part r of
-// orbit o at r NFP + o).
+// orbit o at r NFP + o).  AdjOps: the transposed derivatives' blocks in the same
+// place and the transposed LIFT blocks, in chunks of CH orbits: the chunk's
+// rows of part 0 (DA inputs), then of parts 1, 2, 3, each CH entries padded.
+template <int N>
+constexpr int chunk_orbits() {  // orbits of face values held at a time
+  return N == 1 ? Basis<N>::NFP : (Basis<N>::NFP + 1) / 2;
+}
+
 template <int N>
 struct Ops {
   using B = Basis<N>;
@@ -78,6 +85,19 @@ struct Ops {
   static constexpr int LIFTB = LIFT + B::NFP * PA;
   static constexpr int ENTRIES = LIFTB + 3 * B::NFP * PB;
   static constexpr int NODE_SLOT = ENTRIES * 8;             // bytes from here
+  static constexpr int SLOT_NODE = NODE_SLOT + pad16(B::NP * 4);
+  static constexpr int FACE_POINT = SLOT_NODE + pad16(B::NP * 4);
+  static constexpr int SIZE = FACE_POINT + pad16(B::NFPT * 4);
+};
+
+template <int N>
+struct AdjOps {
+  using B = Basis<N>;
+  static constexpr int CH = chunk_orbits<N>(), NCH = (B::NFP + CH - 1) / CH;
+  static constexpr int PC = (CH + 1) & ~1;
+  static constexpr int LIFT = Ops<N>::LIFT;                 // entries before LIFT^T
+  static constexpr int CHUNK = B::NP * PC;                  // entries of a chunk
+  static constexpr int NODE_SLOT = (LIFT + NCH * CHUNK) * 8;
   static constexpr int SLOT_NODE = NODE_SLOT + pad16(B::NP * 4);
   static constexpr int FACE_POINT = SLOT_NODE + pad16(B::NP * 4);
   static constexpr int SIZE = FACE_POINT + pad16(B::NFPT * 4);
@@ -100,7 +120,7 @@ struct Tile {
   static constexpr int BLOCK = 128;
   // CTAs per SM the registers must allow (order-4 Euler: 168 instead of 186)
   static constexpr int MIN_CTAS = N == 4 ? 3 : 4;
-  static constexpr int CH = N == 1 ? B::NFP : (B::NFP + 1) / 2;  // orbits of a chunk
+  static constexpr int CH = chunk_orbits<N>();
   static constexpr int X = Ops<N>::SIZE;
   static constexpr int X_BYTES = pad16(NF * B::NP * PE * 8);
   static constexpr int F_BYTES = pad16(NF * 4 * CH * PE * 8);
@@ -139,22 +159,21 @@ __device__ __forceinline__ void load_row(const double* p, double (&r)[P]) {
 // Volume term of part rho (D outputs, row pitch P), wave and Maxwell.  x: the
 // thread's element in shared memory; h: metric of the three directions (pitch
 // PE per entry); f0: first input field (Maxwell); sgn: Maxwell's curl sign,
-// wave's -c.
-template <int N, int EQ, int D, int P>
+// wave's -c.  At order 1 one block per direction is not zero: into part A for
+// strong (and transposed weak) derivatives, from part A for weak ones.
+template <int N, int EQ, int D, int P, bool INTO_A = EQ == DG_MAXWELL>
 __device__ __forceinline__ void volume(const double* __restrict__ x,
                                        const double* __restrict__ h,
                                        const double* __restrict__ row, int rho, int f0,
                                        double sgn, double (&acc)[Tile<N, EQ>::NA][D]) {
   using B = Basis<N>;
   constexpr int PE = Tile<N, EQ>::PE, FS = B::NP * PE;  // array stride
-  constexpr bool STRONG = EQ == DG_MAXWELL;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int sig = rho ^ (k + 1);
     const int din = sig == 0 ? B::DA : B::DB;
     const double* xs = x + (sig == 0 ? 0 : B::DA + (sig - 1) * B::DB) * PE;
-    // order 1: strong derivatives reach part A only, weak ones leave it only
-    if (N == 1 && (STRONG ? rho != 0 : sig != 0)) {
+    if (N == 1 && (INTO_A ? rho : sig) != 0) {
       row += din * P;
       continue;
     }

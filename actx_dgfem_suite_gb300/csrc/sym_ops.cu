@@ -3,6 +3,7 @@
 // LIFT.
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "dg_launch.h"
@@ -36,11 +37,14 @@ Vec combo(const int* orbit, int n, int part) {
   return v;
 }
 
-template <int N>
-int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool strong,
+// ADJ: the blocks of the transposed operators (sym::AdjOps); `into_a`: which
+// order-1 blocks may be non-zero (those into part A, else those from it).
+template <int N, bool ADJ>
+int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool into_a,
          unsigned char* out, int out_bytes) {
   using B = sym::Basis<N>;
-  using O = sym::Ops<N>;
+  using F = sym::Ops<N>;
+  using O = std::conditional_t<ADJ, sym::AdjOps<N>, sym::Ops<N>>;
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT;
   if (!out) return O::SIZE;
   if (out_bytes < O::SIZE) return -1;
@@ -185,22 +189,21 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
     to_basis(node, NP, [&](int i, int j) {
       long double s = 0.0L;
       for (int r = 0; r < 3; ++r) {
-        const long double d = diff[(size_t)(r * NP + i) * NP + j];
+        const long double d = diff[(size_t)(r * NP + (ADJ ? j : i)) * NP + (ADJ ? i : j)];
         s += r == k - 1 ? -0.5L * d : 0.5L * d;
       }
       return s;
     });
-    // order 1: one block per direction (strong: into part 0, weak: from it)
     if (!symmetric(NP, [&](int i, int j) {
           const int ri = part_of[i], rj = part_of[j];
-          return (ri ^ rj) == k && (N != 1 || (strong ? ri : rj) == 0);
+          return (ri ^ rj) == k && (N != 1 || (into_a ? ri : rj) == 0);
         }))
       return -1;
     for (int r = 0; r < 4; ++r) {
-      const int pitch = r == 0 ? O::PA : O::PB, s = r ^ k;
+      const int pitch = r == 0 ? F::PA : F::PB, s = r ^ k;
       int row = 0;                  // rows of part r before direction k
       for (int k2 = 1; k2 < k; ++k2) row += dim(r ^ k2);
-      double* dst = ops + (r == 0 ? 0 : O::VOL0 + (r - 1) * O::VOLB) + row * pitch;
+      double* dst = ops + (r == 0 ? 0 : F::VOL0 + (r - 1) * F::VOLB) + row * pitch;
       for (int j = 0; j < dim(s); ++j)
         for (int i = 0; i < dim(r); ++i)
           dst[j * pitch + i] = (double)full[(size_t)(slot0(r) + i) * NP + slot0(s) + j];
@@ -209,13 +212,16 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
   to_basis(face, NFPT,
            [&](int i, int fj) { return (long double)lift[(size_t)i * NFPT + fj]; });
   if (!symmetric(NFPT, [&](int i, int c) { return part_of[i] == c / NFP; })) return -1;
-  for (int r = 0; r < 4; ++r) {
-    const int pitch = r == 0 ? O::PA : O::PB;
-    double* dst = ops + (r == 0 ? O::LIFT : O::LIFTB + (r - 1) * NFP * O::PB);
+  for (int r = 0; r < 4; ++r)
     for (int o = 0; o < NFP; ++o)
-      for (int i = 0; i < dim(r); ++i)
-        dst[o * pitch + i] = (double)full[(size_t)(slot0(r) + i) * NFPT + r * NFP + o];
-  }
+      for (int i = 0; i < dim(r); ++i) {
+        const double x = (double)full[(size_t)(slot0(r) + i) * NFPT + r * NFP + o];
+        if constexpr (ADJ)
+          ops[O::LIFT + (o / O::CH) * O::CHUNK + (slot0(r) + i) * O::PC + o % O::CH] = x;
+        else
+          ops[(r == 0 ? F::LIFT : F::LIFTB + (r - 1) * NFP * F::PB) +
+              o * (r == 0 ? F::PA : F::PB) + i] = x;
+      }
   int32_t* ns = reinterpret_cast<int32_t*>(out + O::NODE_SLOT);
   int32_t* fp = reinterpret_cast<int32_t*>(out + O::FACE_POINT);
   int32_t* sn = reinterpret_cast<int32_t*>(out + O::SLOT_NODE);
@@ -230,10 +236,21 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
 int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
                  bool strong, unsigned char* out, int out_bytes) {
   switch (order) {
-    case 1: return pack<1>(diff, lift, face_nodes, strong, out, out_bytes);
-    case 2: return pack<2>(diff, lift, face_nodes, strong, out, out_bytes);
-    case 3: return pack<3>(diff, lift, face_nodes, strong, out, out_bytes);
-    case 4: return pack<4>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 1: return pack<1, false>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 2: return pack<2, false>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 3: return pack<3, false>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 4: return pack<4, false>(diff, lift, face_nodes, strong, out, out_bytes);
+    default: return -1;
+  }
+}
+
+int pack_sym_adj_ops(int order, const double* weak, const double* lift,
+                     const int32_t* face_nodes, unsigned char* out, int out_bytes) {
+  switch (order) {
+    case 1: return pack<1, true>(weak, lift, face_nodes, true, out, out_bytes);
+    case 2: return pack<2, true>(weak, lift, face_nodes, true, out, out_bytes);
+    case 3: return pack<3, true>(weak, lift, face_nodes, true, out, out_bytes);
+    case 4: return pack<4, true>(weak, lift, face_nodes, true, out, out_bytes);
     default: return -1;
   }
 }

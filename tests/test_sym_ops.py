@@ -16,23 +16,27 @@ from actx_dgfem_suite_gb300.refelem import reference_tet
 EPS = np.finfo(np.float64).eps
 
 
-def _pack(order, diff, lift, face_nodes, strong):
-    f = ctypes.CDLL(str(_lib.library_path()))._ZN2dg12pack_sym_opsEiPKdS1_PKibPhi
+def _pack(order, diff, lift, face_nodes, strong=None):
+    """The block of the forward (``strong`` given) or adjoint operators."""
+    lib = ctypes.CDLL(str(_lib.library_path()))
+    if strong is None:
+        f, extra = lib._ZN2dg16pack_sym_adj_opsEiPKdS1_PKiPhi, []
+    else:
+        f, extra = lib._ZN2dg12pack_sym_opsEiPKdS1_PKibPhi, [ctypes.c_bool(strong)]
     f.restype = ctypes.c_int
     diff, lift = np.ascontiguousarray(diff), np.ascontiguousarray(lift)
     fn = np.ascontiguousarray(face_nodes, dtype=np.int32)
-    ptr = [ctypes.c_void_p(x.ctypes.data) for x in (diff, lift, fn)]
-    size = f(ctypes.c_int(order), *ptr, ctypes.c_bool(strong), None, 0)
+    args = [ctypes.c_int(order)] + [ctypes.c_void_p(x.ctypes.data) for x in (diff, lift, fn)]
+    size = f(*args, *extra, None, 0)
     buf = np.zeros(size, dtype=np.uint8)
-    got = f(ctypes.c_int(order), *ptr, ctypes.c_bool(strong),
-            ctypes.c_void_p(buf.ctypes.data), size)
+    got = f(*args, *extra, ctypes.c_void_p(buf.ctypes.data), size)
     return buf if got == size else None
 
 
 class _Blocks:
     """The operator block of order N read back in the kernel's layout."""
 
-    def __init__(self, order, buf):
+    def __init__(self, order, buf, adjoint=False):
         self.np_ = (order + 1) * (order + 2) * (order + 3) // 6
         self.nfp = (order + 1) * (order + 2) // 2
         npr, nsg = int(order % 2 == 0), int(order == 4)
@@ -50,7 +54,17 @@ class _Blocks:
                 n = dim[r ^ k] * pitch[r]
                 self.vol[r, k] = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
                 pos += n
-        for r in range(4):
+        if adjoint:                              # chunks of orbits, rows by node slot
+            ch = self.nfp if order == 1 else (self.nfp + 1) // 2
+            nch = -(-self.nfp // ch)
+            n = nch * self.np_ * even(ch)
+            t = x[pos:pos + n].reshape(nch, self.np_, even(ch))[:, :, :ch]
+            t = t.transpose(1, 0, 2).reshape(self.np_, -1)
+            assert not t[:, self.nfp:].any()
+            for r in range(4):
+                self.lift[r] = t[self.slot0[r]:self.slot0[r] + dim[r], :self.nfp].T
+            pos += n
+        for r in range(0 if adjoint else 4):
             n = self.nfp * pitch[r]
             self.lift[r] = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
             pos += n
@@ -116,6 +130,25 @@ def test_blocks_reproduce_the_dense_operators(order, strong):
     lift = ref.lift.reshape(b.np_, -1)
     scale = (np.abs(f) @ np.abs(lift).T).max()
     assert np.all(np.abs(y - f @ lift.T) <= 4 * b.nfp * EPS * scale)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_adjoint_blocks_are_the_transposed_blocks(order):
+    ref = reference_tet(order)
+    args = (order, ref.weak_diff, ref.lift, ref.face_nodes)
+    fwd = _Blocks(order, _pack(*args, strong=False))
+    adj = _Blocks(order, _pack(*args), adjoint=True)
+    assert np.array_equal(fwd.node_slot, adj.node_slot)
+    assert np.array_equal(fwd.face_point, adj.face_point)
+    for r in range(4):
+        assert np.array_equal(adj.lift[r], fwd.lift[r].T)
+        for k in (1, 2, 3):
+            # the same sums rounded once to FP64, in another order of summation
+            assert np.allclose(adj.vol[r, k], fwd.vol[r ^ k, k].T, rtol=0,
+                               atol=2 * EPS * np.abs(ref.weak_diff).max())
+    bad = ref.weak_diff.copy()
+    bad[0, 1, 0] += 1e-9
+    assert _pack(order, bad, ref.lift, ref.face_nodes) is None
 
 
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
@@ -201,3 +234,46 @@ def test_tile_edges_match_the_general_kernel(equation, order, nel):
     for a, b in zip(*got):
         # two orders of summation of the same products: 1e-12 as the parity bound
         assert float(torch.linalg.norm(a - b)) <= 1e-12 * float(torch.linalg.norm(b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("equation", ["wave", "euler"])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("nel", [1, 31, 32, 33, 65])
+def test_adjoint_tile_edges_match_the_dense_kernels(equation, order, nel):
+    """Transposed Jacobian and fused reverse stage with element scale around the
+    tile size, against the dense kernels: those run on operators moved off the
+    symmetry by 1e-11, which moves results by no more than that."""
+    import torch
+
+    from actx_dgfem_suite_gb300.mesh import TetMesh
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import jittered_box_mesh, make_problem
+    mesh = jittered_box_mesh(3)
+    mesh = TetMesh(vertices=mesh.vertices, elements=mesh.elements[:nel])
+    prob = make_problem(equation, mesh, order, seed=nel)
+    q = torch.from_numpy(prob.fields).cuda()
+    g = torch.Generator(device="cuda").manual_seed(nel)
+    x = torch.randn(q.shape, dtype=q.dtype, device=q.device, generator=g)
+    lq = torch.randn(q.shape, dtype=q.dtype, device=q.device, generator=g)
+    scale = torch.linspace(0.8, 1.2, nel, dtype=torch.float64, device="cuda")
+    got = []
+    for off in (0.0, 1e-11):
+        dm = DeviceMesh(prob.disc, "cuda:0")
+        dm._weak = dm._weak.copy()
+        dm._weak.reshape(-1)[1] += off * abs(dm._weak).max()
+        plan = DevicePlan(dm, equation, prob.params, "fp64")
+        y = plan.vjp(q, x)
+        plan.set_element_scale(scale)
+        lam, rbar, scr = 0.3 * x, torch.empty_like(x), torch.empty_like(x)
+        out = [y, lam, rbar]
+        if equation == "wave":
+            cbar = torch.ones(nel, dtype=torch.float64, device="cuda")
+            plan.adjoint_stage(x, 0.7, lam, rbar, lq, cbar, 0.4, 0.9, 1e-2, scr)
+            out.append(cbar)
+        else:
+            plan.vjp_stage(q, x, 0.7, lam, rbar, 0.4, 0.9, 1e-2, scr)
+        plan.finish()
+        got.append(out)
+    for a, b in zip(*got):
+        assert float(torch.linalg.norm(a - b)) <= 1e-10 * float(torch.linalg.norm(b))
