@@ -100,7 +100,7 @@ class CompiledRHS:
 
     def _upload(self, host: torch.Tensor) -> torch.Tensor:
         dev = self.actx.device
-        cur = torch.cuda.current_stream(dev)
+        cur = torch.cuda.current_stream(dev.index)
         if (self._in_buf is None or self._in_buf.shape != host.shape):
             self._in_buf = torch.empty(host.shape, dtype=torch.float64, device=dev)
             self._in_free = None
@@ -143,7 +143,7 @@ class CompiledRHS:
         state = args[self.op.state_argnum]
         q = self.stage(state)
         res = self.plan.rhs(q, out)
-        cur = torch.cuda.current_stream(self.actx.device)
+        cur = torch.cuda.current_stream(self.actx.device.index)
         done = torch.cuda.Event()
         done.record(cur)
         if q is self._in_buf:

@@ -23,12 +23,6 @@ NFIELDS = {"wave": 4, "euler": 5, "maxwell": 6}
 NFIELDS_2D = {"wave": 3, "euler": 4, "maxwell": 3}
 
 
-def _stream_handle(stream) -> ctypes.c_void_p:
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(stream.cuda_stream)
-
-
 class DeviceMesh:
     """Geometry, gather index and reference operators of one discretisation,
     uploaded once.
@@ -144,6 +138,10 @@ class DevicePlan:
             raise ValueError("triangle-mesh plans evaluate in FP64 only")
         self.nfields = (NFIELDS_2D if self.dim == 2 else NFIELDS)[equation]
         self.params = tuple(float(p) for p in params)
+        #: (nfields, Nel, Np) of a state
+        self.shape = (self.nfields, mesh.nelements, mesh.np_)
+        self._device = mesh.device
+        self._device_index = mesh.device.index
         L = _lib.lib()
         handle = ctypes.c_void_p()
         parr = (ctypes.c_double * max(1, len(self.params)))(*self.params)
@@ -160,9 +158,12 @@ class DevicePlan:
         self._handle = handle
         self._lib = L
 
-    @property
-    def shape(self) -> tuple[int, int, int]:
-        return (self.nfields, self.mesh.nelements, self.mesh.np_)
+    def _stream(self, stream) -> int:
+        """The handle of ``stream`` or of the current one (by device index: the
+        lookup without one costs several microseconds, a tenth of a small RHS)."""
+        if stream is None:
+            stream = torch.cuda.current_stream(self._device_index)
+        return stream.cuda_stream
 
     def info(self) -> dict:
         nel = ctypes.c_int64()
@@ -186,9 +187,9 @@ class DevicePlan:
         return self.info()["launches_per_rhs"]
 
     def _check_tensor(self, x: torch.Tensor, name: str):
-        if x.dtype != torch.float64 or x.device != self.mesh.device:
-            raise TypeError(f"{name} must be float64 on {self.mesh.device}")
-        if tuple(x.shape) != self.shape or not x.is_contiguous():
+        if x.dtype != torch.float64 or x.device != self._device:
+            raise TypeError(f"{name} must be float64 on {self._device}")
+        if x.shape != self.shape or not x.is_contiguous():
             raise ValueError(f"{name} must be a contiguous {self.shape} tensor, "
                              f"got {tuple(x.shape)}")
 
@@ -199,9 +200,8 @@ class DevicePlan:
             out = torch.empty_like(q)
         else:
             self._check_tensor(out, "out")
-        _lib.check(self._lib.dg_rhs(self._handle, ctypes.c_void_p(q.data_ptr()),
-                                    ctypes.c_void_p(out.data_ptr()),
-                                    _stream_handle(stream)))
+        _lib.check(self._lib.dg_rhs(self._handle, q.data_ptr(), out.data_ptr(),
+                                    self._stream(stream)))
         return out
 
     def rk_stage(self, q_in: torch.Tensor, q_out: torch.Tensor,
@@ -214,11 +214,10 @@ class DevicePlan:
         rptr = None
         if rhs_unscaled is not None:
             self._check_tensor(rhs_unscaled, "rhs_unscaled")
-            rptr = ctypes.c_void_p(rhs_unscaled.data_ptr())
+            rptr = rhs_unscaled.data_ptr()
         _lib.check(self._lib.dg_rk_stage(
-            self._handle, ctypes.c_void_p(q_in.data_ptr()),
-            ctypes.c_void_p(q_out.data_ptr()), ctypes.c_void_p(res.data_ptr()),
-            float(a), float(b), float(dt), rptr, _stream_handle(stream)))
+            self._handle, q_in.data_ptr(), q_out.data_ptr(), res.data_ptr(),
+            float(a), float(b), float(dt), rptr, self._stream(stream)))
 
     def set_element_scale(self, scale: torch.Tensor | None) -> None:
         """Multiply each element's RHS by ``scale[e]`` (kept referenced)."""
@@ -250,7 +249,7 @@ class DevicePlan:
             raise ValueError(f"scratch needs {n} float64 entries")
         _lib.check(self._lib.dg_rhs_adjoint(
             self._handle, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()),
-            ctypes.c_void_p(scratch.data_ptr()), _stream_handle(stream)))
+            ctypes.c_void_p(scratch.data_ptr()), self._stream(stream)))
         return out
 
     def adjoint_stage(self, x: torch.Tensor, xscale: float, lam: torch.Tensor,
@@ -271,11 +270,11 @@ class DevicePlan:
                                  or not cbar.is_contiguous()):
             raise ValueError("cbar must be a contiguous float64 (Nel,) tensor on the "
                              "plan's device")
-        ptr = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())  # noqa: E731
+        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
         _lib.check(self._lib.dg_rhs_adjoint_stage(
             self._handle, ptr(x), float(xscale), ptr(lam), ptr(rbar_out), ptr(lq),
             ptr(cbar), float(a), float(b), float(dt), ptr(y_scratch),
-            _stream_handle(stream)))
+            self._stream(stream)))
 
     #: launch variants: bit 0 tensor-core products (fp32-mixed), bit 1 one CTA per
     #: tile; 4 and 5 the tcgen05 kernel (exact digit pairs, 3xTF32), 6 the
@@ -311,7 +310,7 @@ class DevicePlan:
         if ref is None:
             _lib.check(self._lib.dg_plan_autotune(
                 self._handle, ctypes.c_void_p(q.data_ptr()),
-                ctypes.c_void_p(out.data_ptr()), int(reps), _stream_handle(stream),
+                ctypes.c_void_p(out.data_ptr()), int(reps), self._stream(stream),
                 ctypes.byref(chosen), ms))
             errs = None
         else:
@@ -322,7 +321,7 @@ class DevicePlan:
             _lib.check(self._lib.dg_plan_autotune_bounded(
                 self._handle, ctypes.c_void_p(q.data_ptr()),
                 ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(ref.data_ptr()),
-                float(max_rel_l2), int(reps), _stream_handle(stream),
+                float(max_rel_l2), int(reps), self._stream(stream),
                 ctypes.byref(chosen), ms, errs))
         res = {"chosen": chosen.value,
                "ms": {self.VARIANTS[v]: (float(ms[v]) if ms[v] >= 0 else None)
@@ -343,8 +342,8 @@ class DevicePlan:
         else:
             self._check_tensor(out, "out")
         _lib.check(self._lib.dg_rhs_vjp(
-            self._handle, ctypes.c_void_p(q.data_ptr()), ctypes.c_void_p(x.data_ptr()),
-            ctypes.c_void_p(out.data_ptr()), _stream_handle(stream)))
+            self._handle, q.data_ptr(), x.data_ptr(), out.data_ptr(),
+            self._stream(stream)))
         return out
 
     def vjp_stage(self, q: torch.Tensor, x: torch.Tensor, xscale: float,
@@ -358,13 +357,13 @@ class DevicePlan:
             self._check_tensor(t, name)
         if rbar_out is not None:
             self._check_tensor(rbar_out, "rbar_out")
-        ptr = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())  # noqa: E731
+        ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
         _lib.check(self._lib.dg_rhs_vjp_stage(
             self._handle, ptr(q), ptr(x), float(xscale), ptr(lam), ptr(rbar_out),
-            float(a), float(b), float(dt), ptr(y_scratch), _stream_handle(stream)))
+            float(a), float(b), float(dt), ptr(y_scratch), self._stream(stream)))
 
     def finish(self, stream=None) -> None:
-        _lib.check(self._lib.dg_finish(self._handle, _stream_handle(stream)))
+        _lib.check(self._lib.dg_finish(self._handle, self._stream(stream)))
 
     def close(self) -> None:
         if getattr(self, "_handle", None) is not None and self._handle.value:
