@@ -241,6 +241,16 @@ struct dg_plan {
   dg::LaunchShape tcb_shape[2];
   int tcb_grid[2] = {0, 0};
   int64_t tcb_ntiles[2] = {0, 0};
+  // mixed precision, wave and Euler: the CUDA-core kernel (dg_mixed.cuh) of
+  // variants 0 and 2
+  bool mix = false;
+  void* d_mix_ops = nullptr;
+  uint32_t mix_ops_bytes = 0;
+  dg::LaunchShape mix_shape;
+  int mix_grid = 0;
+  int64_t mix_ntiles = 0;
+  float4* d_nodes = nullptr;   // Euler: FP32 node records, filled before each RHS
+  int nodes_grid = 0;
   // symmetry-adapted kernel (dg_sym.cuh): the face-shared path's main kernel
   // for operators that have the tetrahedron's symmetry
   bool sym = false;
@@ -279,6 +289,7 @@ dg::RhsArgs base_args(const dg_plan* p) {
   a.flux_in = p->split ? p->d_flux : nullptr;
   a.aux = p->split ? p->d_aux : nullptr;
   a.pres = p->d_pres;
+  a.nodes = p->d_nodes;
   return a;
 }
 
@@ -387,6 +398,9 @@ bool is_shape_variant(int v) { return v >= kFirstShapeVariant && v < DG_NUM_VARI
 int shape_index(int v) { return (v - kFirstShapeVariant) / 2; }
 constexpr int kShapeModeBits[2] = {dg::MODE_B128, dg::MODE_B512};
 
+// The plan's variant runs dg_rhs_mixed_kernel.
+bool uses_mix(const dg_plan* p) { return p->mix && (p->variant | 2) == 2; }
+
 // Mode bits and grid of the main kernel under the plan's variant.
 int main_mode(const dg_plan* p, int base) {
   if (is_shape_variant(p->variant))
@@ -399,6 +413,11 @@ int main_grid(const dg_plan* p) {
     if ((p->variant - kFirstShapeVariant) & 1)
       return (int)(p->tcb_ntiles[k] < 0x7fffffff ? p->tcb_ntiles[k] : 0x7fffffff);
     return p->tcb_grid[k];
+  }
+  if (uses_mix(p)) {
+    if (p->variant & 2)
+      return (int)(p->mix_ntiles < 0x7fffffff ? p->mix_ntiles : 0x7fffffff);
+    return p->mix_grid;
   }
   if (p->sym) {
     if (p->variant & 2)
@@ -778,7 +797,10 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
   // the persistent grid fits the modes the plan launches: RHS and RK stage,
   // in the face-shared form on the split path
   dg::LaunchShape shape;
-  const int base_mode = split ? dg::MODE_SPLIT : dg::MODE_RHS;
+  // (wave and Euler in mixed precision: of the mma.sync variants; the CUDA-core
+  // variants have their own kernel)
+  const bool mix = kprec == 1 && equation != DG_MAXWELL;
+  const int base_mode = split ? dg::MODE_SPLIT : (mix ? dg::MODE_TC : dg::MODE_RHS);
   cudaError_t err = shape_of(equation, N, kprec, base_mode, &shape);
   if (err == cudaSuccess) {
     dg::LaunchShape other;
@@ -906,6 +928,41 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
       const int64_t mfull = (int64_t)nsm * m0.blocks_per_sm;
       p->tcm_grid[k] = (int)(mtiles < mfull ? mtiles : mfull);
     }
+  }
+  if (mix) {
+    dg::LaunchShape x0, x1;
+    err = equation == DG_WAVE ? dg::mixed_shape_wave(N, false, &x0)
+                              : dg::mixed_shape_euler(N, false, &x0);
+    if (err == cudaSuccess)
+      err = equation == DG_WAVE ? dg::mixed_shape_wave(N, true, &x1)
+                                : dg::mixed_shape_euler(N, true, &x1);
+    std::vector<unsigned char> xops(
+        dg::pack_mixed_ops(N, diff, mesh->lift, mesh->face_nodes, nullptr, 0));
+    const int xbytes = dg::pack_mixed_ops(N, diff, mesh->lift, mesh->face_nodes, xops.data(),
+                                          (int)xops.size());
+    if (err == cudaSuccess && equation == DG_EULER)
+      err = cudaMalloc(&p->d_nodes, (size_t)p->nel * np * 32);
+    if (err == cudaSuccess) err = cudaMalloc(&p->d_mix_ops, xops.size());
+    if (err == cudaSuccess)
+      err = cudaMemcpy(p->d_mix_ops, xops.data(), xops.size(), cudaMemcpyHostToDevice);
+    if (err != cudaSuccess) {
+      dg_plan_destroy(p);
+      return cuda_fail(err, "mixed-precision kernel configuration");
+    }
+    if (x1.blocks_per_sm < x0.blocks_per_sm) x0.blocks_per_sm = x1.blocks_per_sm;
+    if (xbytes != x0.ops_bytes || x0.blocks_per_sm < 1) {
+      dg_plan_destroy(p);
+      return fail(DG_ERR_CUDA, "mixed-precision kernel: layout mismatch or does not fit");
+    }
+    p->mix = true;
+    p->mix_ops_bytes = static_cast<uint32_t>(xbytes);
+    p->mix_shape = x0;
+    p->mix_ntiles = (p->nel + x0.elems_per_tile - 1) / x0.elems_per_tile;
+    const int64_t xfull = (int64_t)nsm * x0.blocks_per_sm;
+    p->mix_grid = (int)(p->mix_ntiles < xfull ? p->mix_ntiles : xfull);
+    const int64_t nblocks = (p->nel * np + 255) / 256;
+    const int64_t nfull = (int64_t)nsm * 8;
+    p->nodes_grid = (int)(nblocks < nfull ? nblocks : nfull);
   }
   p->face_partner = mesh->face_partner;
 
@@ -1290,6 +1347,16 @@ int autotune_impl(dg_plan* p, const double* q, double* rhs, const double* ref,
   return code;
 }
 
+// The mixed-precision variants' per-node table of state q, where they have one.
+cudaError_t launch_tables(const dg_plan* p, const double* q, cudaStream_t s) {
+  const int64_t n = p->nel * p->np;
+  if (uses_mix(p) && p->d_nodes)
+    return dg::mixed_nodes_euler(q, p->d_nodes, n, p->params[0], p->nodes_grid, s);
+  if (p->d_pres)
+    return dg::pressure_launch_euler(q, p->d_pres, n, p->params[0], p->pres_grid, s);
+  return cudaSuccess;
+}
+
 // The main kernel (volume and LIFT, with the fluxes where they are fused)
 // under the plan's precision, path and variant: RHS or RK stage.
 cudaError_t launch_main(const dg_plan* p, dg::RhsArgs a, bool stage, cudaStream_t s) {
@@ -1305,6 +1372,13 @@ cudaError_t launch_main(const dg_plan* p, dg::RhsArgs a, bool stage, cudaStream_
     a.ops_bytes = p->tcm_ops_bytes[k];
     return tcm_launch_of(p->equation, p->order, tcm_mode(k) | (stage ? 1 : 0), a,
                          p->tcm_grid[k], s);
+  }
+  if (uses_mix(p)) {
+    a.ops = p->d_mix_ops;
+    a.ops_bytes = p->mix_ops_bytes;
+    return p->equation == DG_WAVE
+               ? dg::mixed_launch_wave(p->order, stage, a, main_grid(p), s)
+               : dg::mixed_launch_euler(p->order, stage, a, main_grid(p), s);
   }
   if (p->sym) {
     a.ops = p->d_sym_ops;
@@ -1546,12 +1620,9 @@ int dg_rhs(dg_plan* p, const double* q, double* rhs, void* stream) {
     cudaError_t err = launch_faces(p, q, s);
     if (err != cudaSuccess) return cuda_fail(err, "face kernel launch");
   }
-  if (p->d_pres) {
-    cudaError_t err = dg::pressure_launch_euler(q, p->d_pres, p->nel * p->np,
-                                                p->params[0], p->pres_grid, s);
-    if (err != cudaSuccess) return cuda_fail(err, "pressure kernel launch");
-  }
-  cudaError_t err = launch_main(p, a, false, s);
+  cudaError_t err = launch_tables(p, q, s);
+  if (err != cudaSuccess) return cuda_fail(err, "node table launch");
+  err = launch_main(p, a, false, s);
   if (err != cudaSuccess) return cuda_fail(err, "rhs launch");
   return DG_OK;
 }
@@ -1589,12 +1660,9 @@ int dg_rk_stage(dg_plan* p, const double* q_in, double* q_out, double* res,
     cudaError_t err = launch_faces(p, q_in, s);
     if (err != cudaSuccess) return cuda_fail(err, "face kernel launch");
   }
-  if (p->d_pres) {
-    cudaError_t err = dg::pressure_launch_euler(q_in, p->d_pres, p->nel * p->np,
-                                                p->params[0], p->pres_grid, s);
-    if (err != cudaSuccess) return cuda_fail(err, "pressure kernel launch");
-  }
-  cudaError_t err = launch_main(p, a, true, s);
+  cudaError_t err = launch_tables(p, q_in, s);
+  if (err != cudaSuccess) return cuda_fail(err, "node table launch");
+  err = launch_main(p, a, true, s);
   if (err != cudaSuccess) return cuda_fail(err, "rk stage launch");
   return DG_OK;
 }
@@ -1709,7 +1777,8 @@ int dg_plan_destroy(dg_plan* p) {
   for (void* b : {(void*)p->d_owned, (void*)p->d_flux, (void*)p->d_aux,
                   (void*)p->d_tc_ops, p->d_tcm_ops[0], p->d_tcm_ops[1],
                   p->d_tcm_ops[2] != p->d_tcm_ops[1] ? p->d_tcm_ops[2] : nullptr,
-                  (void*)p->d_pres, p->d_sym_ops, p->d_adj_sym_ops})
+                  (void*)p->d_pres, p->d_sym_ops, p->d_adj_sym_ops,
+                  p->d_mix_ops, (void*)p->d_nodes})
     if (b && cudaFree(b) != cudaSuccess) code = DG_ERR_CUDA;
   delete p;
   if (code != DG_OK) return fail(code, "cudaFree failed");
@@ -1812,13 +1881,15 @@ int dg_plan_info(const dg_plan* p, int64_t* nelements, int32_t* order,
     *block = p->tc ? p->tc_shape.threads
                    : (m4 ? p->tcm_shape[k].threads
                          : (mb ? p->tcb_shape[kb].threads
-                               : (p->sym ? p->sym_shape.threads : dg::kBlock)));
+                               : (uses_mix(p) ? p->mix_shape.threads
+                                              : (p->sym ? p->sym_shape.threads : dg::kBlock))));
   if (smem_bytes)
     *smem_bytes = p->tc ? p->tc_shape.smem_bytes
                         : (m4 ? p->tcm_shape[k].smem_bytes
                               : (mb ? p->tcb_shape[kb].smem_bytes
-                                    : (p->sym ? p->sym_shape.smem_bytes
-                                                   : p->shape.smem_bytes)));
+                                    : (uses_mix(p) ? p->mix_shape.smem_bytes
+                                                   : (p->sym ? p->sym_shape.smem_bytes
+                                                             : p->shape.smem_bytes))));
   return DG_OK;
 }
 

@@ -112,6 +112,22 @@ int pack_sym_ops(int order, const double* diff, const double* lift, const int32_
 int pack_sym_adj_ops(int order, const double* weak, const double* lift,
                      const int32_t* face_nodes, unsigned char* out, int out_bytes);
 
+// Mixed precision on the CUDA cores, wave and Euler (dg_mixed.cuh): shape and
+// launch (stage: fused RK stage) of the main kernel, Euler's launch before it that
+// fills the FP32 node records (32 bytes per node), and the FP32 operator block
+// (mix::Ops); returns the block size (out == NULL: size only, -1 if out_bytes is
+// short).
+cudaError_t mixed_shape_wave(int order, bool stage, LaunchShape* out);
+cudaError_t mixed_launch_wave(int order, bool stage, const RhsArgs& a, int grid,
+                              cudaStream_t s);
+cudaError_t mixed_shape_euler(int order, bool stage, LaunchShape* out);
+cudaError_t mixed_launch_euler(int order, bool stage, const RhsArgs& a, int grid,
+                               cudaStream_t s);
+cudaError_t mixed_nodes_euler(const double* q, float4* rec, int64_t nelnp, double gamma,
+                              int grid, cudaStream_t s);
+int pack_mixed_ops(int order, const double* diff, const double* lift,
+                   const int32_t* face_nodes, unsigned char* out, int out_bytes);
+
 // Triangle meshes (rhs_2d.cu): shape query and launch of dg_rhs2d_kernel
 // for mode MODE_RHS or MODE_STAGE (FP64), and the operator block
 // [Wt (2 Np Np) | Lt (3 Nfp Np) | int32 edge nodes (3 Nfp)] packed from the
