@@ -446,7 +446,15 @@ cudaError_t launch_faces(const dg_plan* p, const double* q, cudaStream_t s) {
   f.p0 = p->params[0];
   f.p1 = p->params[1];
   f.p2 = p->params[2];
-  for (int k = 0; k < 6; ++k) f.k[k] = p->k[k];
+  if (p->equation == DG_WAVE) {
+    f.c[0] = 0.5 * p->params[0];
+  } else if (p->equation == DG_MAXWELL) {
+    const double z = p->k[0], y = p->k[1], ce = p->k[2], ch = p->k[3], alpha = p->params[0];
+    f.c[0] = -ce * z;
+    f.c[1] = ce * alpha;
+    f.c[2] = -ch * y;
+    f.c[3] = -ch * alpha;
+  }
   return face_launch_of(p->equation, p->order, f, p->face_grid, p->aux_grid, s);
 }
 

@@ -18,6 +18,12 @@
 //       dg_rhs_sym_kernel (dg_sym.cuh) for operators with the tetrahedron's
 //       symmetry, dg_rhs_kernel with MODE_SPLIT for any others.
 //
+// What bounds it: the FP64 pipe (79-85 % busy), so each flux is written for the
+// fewest FP64 operations that keep jumps as differences of traces: wave 26 per
+// pair of points, Euler 50, Maxwell 62.  Measured (GB300, ncu, against 30 / 55 /
+// 68 before): wave P1 at 5.14 M tets 1.91 -> 1.75 ms, Euler P2 at 413,526 tets 617
+// -> 569 us, Maxwell P4 at 584,016 tets 2.09 ms either way.
+//
 // Face values live in HBM as (nfields, Nel, 4 Nfp) doubles, face point
 // (e, f, j) at e * 4 Nfp + f Nfp + j -- the fused kernel's shared-memory
 // flux layout -- already multiplied by sJ/J and signed as that kernel's.
@@ -46,7 +52,10 @@ struct FaceArgs {
   int64_t nowned;
   int* status;
   double p0, p1, p2;          // equation parameters
-  double k[6];                // maxwell: z, 1/z, -1/(2z), 1/(2/z), 1/eps, 1/mu
+  // flux constants, folded on the host (every FP64 multiply counts here): wave c/2;
+  // maxwell, with z the impedance, ce = -1/(2z), ch = z/2: -ce z, ce alpha, -ch / z,
+  // -ch alpha
+  double c[4];
 };
 
 // Pressure, 1/rho and |u| + c of every node (the per-trace quantities of the
@@ -131,10 +140,9 @@ __global__ void __launch_bounds__(kFaceBlock) dg_face_flux_kernel(const FaceArgs
         qe[k] = bdry ? 0.0 : __ldg(qx);
       }
     }
-    // own[k]: value for this face point; part[k]: for the glued face point
-    // (before each side's sJ/J and a common factor fs)
+    // own[k]: value for this face point; part[k]: for the glued face point, each
+    // with its side's sJ/J
     double own[NF], part[NF];
-    double fs = 1.0;
 
     if constexpr (EQ == DG_WAVE) {
       if (bdry) {  // Dirichlet mirror: exterior (-u, v)
@@ -144,18 +152,22 @@ __global__ void __launch_bounds__(kFaceBlock) dg_face_flux_kernel(const FaceArgs
         qe[3] = qi[3];
       }
       // F_u = c (avg(v).n + (u+ - u-)/2) = c/2 ((v- + v+).n + u+ - u-),
-      // F_v = c (avg(u) + (v+ - v-).n/2) n = c/2 (u- + u+ + (v+ - v-).n) n;
-      // c/2 goes into the side scales
-      const double sv = fma(qi[1] + qe[1], nx, fma(qi[2] + qe[2], ny, (qi[3] + qe[3]) * nz));
+      // F_v = c (avg(u) + (v+ - v-).n/2) n = c/2 (u- + u+ + (v+ - v-).n) n, the
+      // sums as 2 x interior + jump; c/2 goes into the side scales
+      const double du = qe[0] - qi[0];
       const double dv = fma(qe[1] - qi[1], nx, fma(qe[2] - qi[2], ny, (qe[3] - qi[3]) * nz));
-      const double gv = (qi[0] + qe[0]) + dv;
-      own[0] = sv + (qe[0] - qi[0]);
-      own[1] = gv * nx;
-      own[2] = gv * ny;
-      own[3] = gv * nz;
-#pragma unroll
-      for (int k = 0; k < NF; ++k) part[k] = -own[k];
-      fs = 0.5 * a.p0;
+      const double vn = fma(qi[1], nx, fma(qi[2], ny, qi[3] * nz));
+      const double su = du + fma(2.0, vn, dv), gv = fma(2.0, qi[0], du) + dv;
+      const double so = a.c[0] * scale_o, sp = -a.c[0] * scale_p;
+      const double go = so * gv, gp = sp * gv;
+      own[0] = so * su;
+      own[1] = go * nx;
+      own[2] = go * ny;
+      own[3] = go * nz;
+      part[0] = sp * su;
+      part[1] = gp * nx;
+      part[2] = gp * ny;
+      part[3] = gp * nz;
     } else if constexpr (EQ == DG_EULER) {
       const double* an = a.aux;
       const double pi = __ldg(an + ii), ri = __ldg(an + nelnp + ii),
@@ -176,30 +188,24 @@ __global__ void __launch_bounds__(kFaceBlock) dg_face_flux_kernel(const FaceArgs
         re = __ldg(an + nelnp + gi);
         le = __ldg(an + 2 * (size_t)nelnp + gi);
       }
-      // F(q).n of one side: with m.n first, u.n = (m.n) / rho costs one
-      // product (the velocity itself is not needed here)
-      double fn_i[5], fn_e[5];
-      auto side = [&](const double* qq, double p, double rinv, double* fn) {
-        const double mn = fma(qq[2], nx, fma(qq[3], ny, qq[4] * nz));
-        const double un = mn * rinv;
-        fn[0] = mn;
-        fn[1] = un * (qq[1] + p);
-        fn[2] = fma(qq[2], un, p * nx);
-        fn[3] = fma(qq[3], un, p * ny);
-        fn[4] = fma(qq[4], un, p * nz);
-      };
-      side(qi, pi, ri, fn_i);
-      side(qe, pe, re, fn_e);
-      // f_k = 1/2 (F_i + F_e).n - 1/2 lam (q_e - q_i) n.n = 1/2 t_k; the 1/2
-      // and the sign go into the per-side scale factors below
+      // (F- + F+).n through m.n and u.n = (m.n) / rho of both sides
+      const double mi = fma(qi[2], nx, fma(qi[3], ny, qi[4] * nz));
+      const double me = fma(qe[2], nx, fma(qe[3], ny, qe[4] * nz));
+      const double ui = mi * ri, ue = me * re, ps = pi + pe;
       const double lnn = fmax(li, le) * fma(nx, nx, fma(ny, ny, nz * nz));
+      const double sum[5] = {mi + me, fma(ue, qe[1] + pe, ui * (qi[1] + pi)),
+                             fma(qe[2], ue, fma(qi[2], ui, ps * nx)),
+                             fma(qe[3], ue, fma(qi[3], ui, ps * ny)),
+                             fma(qe[4], ue, fma(qi[4], ui, ps * nz))};
+      // f_k = 1/2 (F- + F+).n - 1/2 lam (q+ - q-) n.n = 1/2 t_k; the glued side
+      // sees -f_k
+      const double so = -0.5 * scale_o, sp = 0.5 * scale_p;
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
-        const double tk = fma(-lnn, qe[k] - qi[k], fn_i[k] + fn_e[k]);
-        own[k] = -tk;
-        part[k] = tk;
+        const double tk = fma(-lnn, qe[k] - qi[k], sum[k]);
+        own[k] = so * tk;
+        part[k] = sp * tk;
       }
-      fs = 0.5;
     } else {  // DG_MAXWELL
       if (bdry) {  // PEC: exterior (-E, H)
         qe[0] = -qi[0];
@@ -209,8 +215,6 @@ __global__ void __launch_bounds__(kFaceBlock) dg_face_flux_kernel(const FaceArgs
         qe[4] = qi[4];
         qe[5] = qi[5];
       }
-      const double alpha = a.p0;
-      const double z = a.k[0], y = a.k[1], ce = a.k[2], ch = a.k[3];
       const double je[3] = {qe[0] - qi[0], qe[1] - qi[1], qe[2] - qi[2]};
       const double jh[3] = {qe[3] - qi[3], qe[4] - qi[4], qe[5] - qi[5]};
       const double n[3] = {nx, ny, nz};
@@ -221,34 +225,33 @@ __global__ void __launch_bounds__(kFaceBlock) dg_face_flux_kernel(const FaceArgs
       };
       // fe = n x (z jh - alpha n x je) = Ae + Be, fh = n x (y je + alpha n x jh)
       // = Ah + Bh; swapping the sides keeps Ae, Ah and negates Be, Bh.  With
-      // the constants folded: -ce fe = k1 (n x jh) + k2 (n x n x je),
-      // -ch fh = k3 (n x je) + k4 (n x n x jh)
+      // the constants folded: -ce fe = c0 (n x jh) + c1 (n x n x je),
+      // -ch fh = c2 (n x je) + c3 (n x n x jh).  (The side's scale folded into the
+      // constants saves six more multiplies per point but measured 5 % slower: 60
+      // registers, four CTAs per SM instead of five.)
       double nxe[3], nxh[3], nnxe[3], nnxh[3];
       cross(n, je, nxe);
       cross(n, jh, nxh);
       cross(n, nxe, nnxe);
       cross(n, nxh, nnxh);
-      const double k1 = -ce * z, k2 = ce * alpha, k3 = -ch * y, k4 = -ch * alpha;
 #pragma unroll
       for (int x = 0; x < 3; ++x) {
-        const double ae = k1 * nxh[x], be = k2 * nnxe[x];
-        const double ah = k3 * nxe[x], bh = k4 * nnxh[x];
-        own[x] = ae + be;
-        own[3 + x] = ah + bh;
-        part[x] = ae - be;
-        part[3 + x] = ah - bh;
+        const double ae = a.c[0] * nxh[x], be = a.c[1] * nnxe[x];
+        const double ah = a.c[2] * nxe[x], bh = a.c[3] * nnxh[x];
+        own[x] = scale_o * (ae + be);
+        own[3 + x] = scale_o * (ah + bh);
+        part[x] = scale_p * (ae - be);
+        part[3 + x] = scale_p * (ah - bh);
       }
     }
 
-    const double so = fs * scale_o;
-    const double sp = fs * scale_p;
     double* out = a.flux + fp;
 #pragma unroll
-    for (int k = 0; k < NF; ++k, out += nfp_all) out[0] = so * own[k];
+    for (int k = 0; k < NF; ++k, out += nfp_all) out[0] = own[k];
     if (pp >= 0) {
       double* outp = a.flux + (uint32_t)pp;
 #pragma unroll
-      for (int k = 0; k < NF; ++k, outp += nfp_all) outp[0] = sp * part[k];
+      for (int k = 0; k < NF; ++k, outp += nfp_all) outp[0] = part[k];
     }
   }
 }

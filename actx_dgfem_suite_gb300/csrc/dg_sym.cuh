@@ -502,25 +502,35 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
     __syncthreads();
     // }}}
 
-    // {{{ back to nodes, then store or fold into the RK stage
+    // {{{ back to nodes, then store or fold into the RK stage (all loads of a node
+    // before its stores, which the compiler must assume to alias them)
     transform<N, PE, E, BLOCK>(sX, NF);
     __syncthreads();
     for (int rem = t; rem < ecount * NP; rem += BLOCK) {
       const int el = rem / NP;
       const double* y = sX + node_slot[rem - el * NP] * PE + el;
-      int64_t gidx = e0 * NP + rem;
+      const int64_t gidx = e0 * NP + rem;
+      [[maybe_unused]] double res[NF], qn[NF];
+      if constexpr (STAGE) {
 #pragma unroll
-      for (int k = 0; k < NF; ++k, gidx += nelnp) {
+        for (int k = 0; k < NF; ++k) {
+          res[k] = a.rk_a != 0.0 ? a.res[gidx + k * nelnp] : 0.0;
+          qn[k] = __ldg(a.q + gidx + k * nelnp);
+        }
+      }
+      const double scale = a.elem_scale ? __ldg(a.elem_scale + e0 + el) : 1.0;
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
         double val = y[k * XS];
         if constexpr (STAGE)
-          if (a.rhs_unscaled) a.rhs_unscaled[gidx] = val;
-        if (a.elem_scale) val *= __ldg(a.elem_scale + e0 + el);
+          if (a.rhs_unscaled) a.rhs_unscaled[gidx + k * nelnp] = val;
+        if (a.elem_scale) val *= scale;
         if constexpr (!STAGE) {
-          a.rhs[gidx] = val;
+          a.rhs[gidx + k * nelnp] = val;
         } else {
-          const double r = (a.rk_a != 0.0 ? a.rk_a * a.res[gidx] : 0.0) + a.rk_dt * val;
-          a.res[gidx] = r;
-          a.q_out[gidx] = __ldg(a.q + gidx) + a.rk_b * r;
+          const double r = (a.rk_a != 0.0 ? a.rk_a * res[k] : 0.0) + a.rk_dt * val;
+          a.res[gidx + k * nelnp] = r;
+          a.q_out[gidx + k * nelnp] = qn[k] + a.rk_b * r;
         }
       }
     }
