@@ -251,8 +251,9 @@ struct dg_plan {
   int64_t mix_ntiles = 0;
   float4* d_nodes = nullptr;   // Euler: FP32 node records, filled before each RHS
   int nodes_grid = 0;
-  // symmetry-adapted kernel (dg_sym.cuh): the face-shared path's main kernel
-  // for operators that have the tetrahedron's symmetry
+  // symmetry-adapted kernel (dg_sym.cuh, dg_sym2d.cuh): the main kernel of the
+  // face-shared path and of triangle meshes for operators that have the element's
+  // symmetry
   bool sym = false;
   void* d_sym_ops = nullptr;
   uint32_t sym_ops_bytes = 0;
@@ -1222,6 +1223,41 @@ int dg_plan_create_2d(dg_plan** plan_out, int32_t equation,
   const int64_t full_stage = (int64_t)nsm * other.blocks_per_sm;
   p->grid = (int)(p->ntiles < full ? p->ntiles : full);
   p->grid_stage = (int)(p->ntiles < full_stage ? p->ntiles : full_stage);
+
+  std::vector<unsigned char> sops(
+      dg::pack_sym_ops_2d(N, diff, mesh->lift, mesh->face_nodes, nullptr, 0));
+  const int sbytes = dg::pack_sym_ops_2d(N, diff, mesh->lift, mesh->face_nodes, sops.data(),
+                                         (int)sops.size());
+  // The symmetry-adapted kernel's tile of 32 elements takes longer from start to end
+  // than the dense kernel's smaller ones, which pays once SMs hold more than one.
+  // Measured (dense / symmetric, us): at 32 elements per SM wave P4 21 / 31, Euler P4
+  // 47 / 59, wave P2 10 / 14; at 48 wave P4 31 / 31, Euler P4 69 / 60, wave P3 19 / 21,
+  // wave P2 16 / 14; at 84 wave P4 50 / 41, Euler P3 86 / 56; order 1 at any size
+  // (wave 10 / 9, Euler 24 / 15 at 800 elements).
+  const bool fills = N == 1 || p->nel >= (int64_t)48 * nsm;
+  if (sbytes > 0 && fills) {  // the operators have the symmetry
+    dg::LaunchShape s0, s1;
+    err = dg::sym_shape_2d(equation, N, dg::MODE_RHS, &s0);
+    if (err == cudaSuccess) err = dg::sym_shape_2d(equation, N, dg::MODE_STAGE, &s1);
+    if (err == cudaSuccess) err = cudaMalloc(&p->d_sym_ops, sbytes);
+    if (err == cudaSuccess)
+      err = cudaMemcpy(p->d_sym_ops, sops.data(), sbytes, cudaMemcpyHostToDevice);
+    if (err != cudaSuccess) {
+      dg_plan_destroy(p);
+      return cuda_fail(err, "symmetry-adapted 2D kernel configuration");
+    }
+    if (sbytes != s0.ops_bytes || s0.blocks_per_sm < 1 || s1.blocks_per_sm < 1) {
+      dg_plan_destroy(p);
+      return fail(DG_ERR_CUDA, "symmetry-adapted 2D kernel: layout mismatch or does not fit");
+    }
+    p->sym = true;
+    p->sym_ops_bytes = static_cast<uint32_t>(sbytes);
+    p->sym_shape = s0;
+    p->sym_ntiles = (p->nel + s0.elems_per_tile - 1) / s0.elems_per_tile;
+    const int64_t f0 = (int64_t)nsm * s0.blocks_per_sm, f1 = (int64_t)nsm * s1.blocks_per_sm;
+    p->sym_grid = (int)(p->sym_ntiles < f0 ? p->sym_ntiles : f0);
+    p->grid_stage = (int)(p->sym_ntiles < f1 ? p->sym_ntiles : f1);
+  }
   *plan_out = p;
   return DG_OK;
 }
@@ -1395,6 +1431,17 @@ cudaError_t launch_main(const dg_plan* p, dg::RhsArgs a, bool stage, cudaStream_
   }
   const int base = (stage ? dg::MODE_STAGE : dg::MODE_RHS) | (p->split ? dg::MODE_SPLIT : 0);
   return launch_of(p->equation, p->order, prec, main_mode(p, base), a, main_grid(p), s);
+}
+
+// Triangle meshes: the one launch of an RHS or RK stage.
+cudaError_t launch_2d_of(const dg_plan* p, int mode, dg::RhsArgs a, cudaStream_t s) {
+  const bool stage = mode == dg::MODE_STAGE;
+  if (!p->sym)
+    return dg::launch_2d(p->equation, p->order, mode, a, stage ? p->grid_stage : p->grid, s);
+  a.ops = p->d_sym_ops;
+  a.ops_bytes = p->sym_ops_bytes;
+  return dg::sym_launch_2d(p->equation, p->order, mode, a, stage ? p->grid_stage : p->sym_grid,
+                           s);
 }
 
 dg::VjpArgs vjp_args(const dg_plan* p, const double* q, const double* x, double* y) {
@@ -1620,7 +1667,7 @@ int dg_rhs(dg_plan* p, const double* q, double* rhs, void* stream) {
   a.rhs = rhs;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (p->dim == 2) {
-    cudaError_t err = dg::launch_2d(p->equation, p->order, dg::MODE_RHS, a, p->grid, s);
+    cudaError_t err = launch_2d_of(p, dg::MODE_RHS, a, s);
     if (err != cudaSuccess) return cuda_fail(err, "rhs launch");
     return DG_OK;
   }
@@ -1660,7 +1707,7 @@ int dg_rk_stage(dg_plan* p, const double* q_in, double* q_out, double* res,
   }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (p->dim == 2) {
-    cudaError_t err = dg::launch_2d(p->equation, p->order, dg::MODE_STAGE, a, p->grid_stage, s);
+    cudaError_t err = launch_2d_of(p, dg::MODE_STAGE, a, s);
     if (err != cudaSuccess) return cuda_fail(err, "rk stage launch");
     return DG_OK;
   }

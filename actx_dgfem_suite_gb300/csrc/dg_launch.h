@@ -139,6 +139,16 @@ cudaError_t launch_2d(int eq, int order, int mode, const RhsArgs& a, int grid,
 int pack_ops_2d(int order, const double* diff, const double* lift,
                 const int32_t* face_nodes, unsigned char* out, int out_bytes);
 
+// The same in the triangle's symmetry-adapted basis (sym_2d.cu, dg_sym2d.cuh), for
+// operators that pack_sym_ops_2d accepts; it returns the block size (out == NULL:
+// size only) or -1 when they do not have the symmetry to rounding (or out_bytes is
+// short).
+cudaError_t sym_shape_2d(int eq, int order, int mode, LaunchShape* out);
+cudaError_t sym_launch_2d(int eq, int order, int mode, const RhsArgs& a, int grid,
+                          cudaStream_t s);
+int pack_sym_ops_2d(int order, const double* diff, const double* lift,
+                    const int32_t* face_nodes, unsigned char* out, int out_bytes);
+
 // Record `msg` as the calling thread's last error (dg_last_error) and
 // return `code`; shared by the translation units behind the C ABI.
 int set_error(int code, const char* msg);

@@ -277,3 +277,165 @@ def test_adjoint_tile_edges_match_the_dense_kernels(equation, order, nel):
         got.append(out)
     for a, b in zip(*got):
         assert float(torch.linalg.norm(a - b)) <= 1e-10 * float(torch.linalg.norm(b))
+
+
+@pytest.mark.parametrize("strong", [False, True])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_triangle_blocks_reproduce_the_dense_operators(order, strong):
+    """``pack_sym_ops_2d``: even and odd blocks under the swap of vertices 1 and
+    2; operators off the symmetry are refused."""
+    from actx_dgfem_suite_gb300.refelem import reference_tri
+    f = ctypes.CDLL(str(_lib.library_path()))._ZN2dg15pack_sym_ops_2dEiPKdS1_PKiPhi
+    f.restype = ctypes.c_int
+
+    def pack(diff, lift, fnodes):
+        arrs = [np.ascontiguousarray(diff), np.ascontiguousarray(lift),
+                np.ascontiguousarray(fnodes, dtype=np.int32)]
+        args = [ctypes.c_int(order)] + [ctypes.c_void_p(x.ctypes.data) for x in arrs]
+        buf = np.zeros(f(*args, None, 0), dtype=np.uint8)
+        got = f(*args, ctypes.c_void_p(buf.ctypes.data), buf.size)
+        return buf if got == buf.size else None
+
+    ref = reference_tri(order)
+    diff = ref.diff if strong else ref.weak_diff
+    npn, nfpt = ref.np_, 3 * ref.nfp
+    buf = pack(diff, ref.lift, ref.face_nodes)
+    nfx, ffx = order // 2 + 1, int(order % 2 == 0)
+    npr, fpr = (npn - nfx) // 2, (nfpt - ffx) // 2
+    dim, fdim = (npr + nfx, npr), (fpr + ffx, fpr)
+    pitch = [(d + 1) & ~1 for d in dim]
+    x, pos = buf.view(np.float64), 0
+    vol, lft = {}, {}
+    for r in range(2):
+        for k in range(2):
+            n = dim[r ^ k] * pitch[r]
+            vol[r, k] = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
+            pos += n
+    for r in range(2):
+        n = fdim[r] * pitch[r]
+        lft[r] = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
+        pos += n
+    tab, pos = buf.view(np.int32), 2 * pos
+    tables = []
+    for n in (npn, npn, nfpt, nfpt):
+        tables.append(tab[pos:pos + n])
+        pos += (n + 3) // 4 * 4
+    node_slot, slot_node, edge_slot, edge_node = tables
+    assert list(slot_node[node_slot]) == list(range(npn))
+    assert sorted(edge_slot) == list(range(nfpt))
+    assert np.array_equal(edge_node, ref.face_nodes.reshape(-1))
+
+    def mirror(v, pairs, even):
+        u, w = v[:, :pairs].copy(), v[:, even:even + pairs].copy()
+        v[:, :pairs], v[:, even:even + pairs] = u + w, u - w
+        return v
+
+    rng = np.random.default_rng(order)
+    q, e = rng.standard_normal((7, npn)), rng.standard_normal((7, nfpt))
+    g = rng.standard_normal((2, 7, 1))
+    part = [slice(0, dim[0]), slice(dim[0], npn)]
+    fpart = [slice(0, fdim[0]), slice(fdim[0], nfpt)]
+    qs, es = np.empty_like(q), np.empty_like(e)
+    qs[:, node_slot], es[:, edge_slot] = q, e
+    mirror(qs, npr, dim[0])
+    mirror(es, fpr, fdim[0])
+    h = [g[0] + g[1], g[0] - g[1]]
+    y, z = np.zeros_like(qs), np.zeros_like(qs)
+    for r in range(2):
+        for k in range(2):
+            y[:, part[r]] += h[k] * (qs[:, part[r ^ k]] @ vol[r, k].T)
+        z[:, part[r]] = es[:, fpart[r]] @ lft[r].T
+    y, z = (mirror(v, npr, dim[0])[:, node_slot] for v in (y, z))
+    dense = g[0] * (q @ diff[0].T) + g[1] * (q @ diff[1].T)
+    size = sum(np.abs(g[r]) * (np.abs(q) @ np.abs(diff[r]).T) for r in range(2)).max()
+    assert np.all(np.abs(y - dense) <= 3 * npn * EPS * size)
+    lift = ref.lift.reshape(npn, -1)
+    assert np.all(np.abs(z - e @ lift.T) <= 4 * nfpt * EPS * (np.abs(e) @ np.abs(lift).T).max())
+    for which in range(3):
+        d, li, fn = diff.copy(), ref.lift.copy(), ref.face_nodes.copy()
+        if which == 0:
+            d[0, 0, 1] += 1e-9 * np.abs(d).max()
+        elif which == 1:
+            li.reshape(-1)[1] = np.nan
+        else:
+            fn[0] = fn[2][::-1] if order > 1 else fn[2]
+        assert pack(d, li, fn) is None, which
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("equation", ["wave", "euler", "maxwell"])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("nel", [0, 1, 31, 33, 146])
+def test_triangle_tile_edges_match_the_dense_kernel(equation, order, nel):
+    """Element counts around the 32-element tile on a mesh whose elements are
+    shuffled (glued sides inside and outside the tiles), RHS and RK stage: the
+    dense kernel runs on operators moved off the symmetry by 1e-11."""
+    import torch
+
+    from actx_dgfem_suite_gb300.mesh import TriMesh
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import jittered_square_mesh, make_problem_2d
+    # the kernel serves meshes from 48 elements per SM on
+    nel += 48 * torch.cuda.get_device_properties(0).multi_processor_count
+    mesh = jittered_square_mesh(61)
+    el = mesh.elements
+    if nel % 2:
+        el = np.roll(el, nel % 3, axis=1)[np.random.default_rng(nel).permutation(len(el))]
+    assert nel <= len(el)
+    prob = make_problem_2d(equation, TriMesh(vertices=mesh.vertices, elements=el[:nel]), order,
+                           seed=nel)
+    q = torch.from_numpy(prob.fields).cuda()
+    scale = torch.linspace(0.8, 1.2, nel, dtype=torch.float64, device="cuda")
+    got = []
+    for off in (0.0, 1e-11):
+        dm = DeviceMesh(prob.disc, "cuda:0")
+        for name in ("_weak", "_strong"):
+            ops = getattr(dm, name).copy()
+            ops.reshape(-1)[1] += off * abs(ops).max()
+            setattr(dm, name, ops)
+        plan = DevicePlan(dm, equation, prob.params, "fp64")
+        r = plan.rhs(q)
+        plan.set_element_scale(scale)
+        res, qo, un = 0.5 * q, torch.empty_like(q), torch.empty_like(q)
+        plan.rk_stage(q, qo, res, 0.3, 0.7, 1e-2, rhs_unscaled=un)
+        plan.finish()
+        got.append((r, res, qo, un, plan.info()["block"]))
+    assert got[0][4] != got[1][4]                # two different kernels
+    for a, b in zip(got[0][:4], got[1][:4]):
+        assert float(torch.linalg.norm(a - b)) <= 1e-10 * float(torch.linalg.norm(b))
+
+
+@pytest.mark.gpu
+def test_triangles_glued_with_a_turn_are_not_shared():
+    """Sides glued by the gather index whose normals are not opposite (a periodic
+    sector) keep one flux per side, inside a tile too."""
+    import torch
+
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import jittered_square_mesh, make_problem_2d
+    prob = make_problem_2d("euler", jittered_square_mesh(61), 2, seed=1)
+    q = torch.from_numpy(prob.fields).cuda()
+    got, blocks = [], []
+    for off in (0.0, 1e-11):
+        dm = DeviceMesh(prob.disc, "cuda:0")
+        gather = dm.gather.cpu().numpy().view(np.uint32).copy()
+        nodes, npn = prob.disc.ref.face_nodes, prob.disc.np_
+        free = [(e, f) for e in range(prob.disc.nelements) for f in range(3)
+                if gather[e, f, 0] >> 31]
+        turned = 0
+        for (e, f), (e2, f2) in zip(free[::2], free[1::2]):
+            if e != e2 and abs((prob.disc.normal[e, f] + prob.disc.normal[e2, f2])).max() > 0.1:
+                gather[e, f] = e2 * npn + nodes[f2][::-1]
+                gather[e2, f2] = e * npn + nodes[f][::-1]
+                turned += 1
+        assert turned > 0
+        dm.gather = torch.from_numpy(gather.view(np.int32)).cuda()
+        ops = dm._weak.copy()
+        ops.reshape(-1)[1] += off * abs(ops).max()
+        dm._weak = ops
+        plan = DevicePlan(dm, "euler", prob.params, "fp64")
+        got.append(plan.rhs(q))
+        plan.finish()
+        blocks.append(plan.info()["block"])
+    assert blocks[0] != blocks[1]
+    assert float(torch.linalg.norm(got[0] - got[1])) <= 1e-10 * float(torch.linalg.norm(got[1]))
