@@ -806,10 +806,7 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
   // the persistent grid fits the modes the plan launches: RHS and RK stage,
   // in the face-shared form on the split path
   dg::LaunchShape shape;
-  // (wave and Euler in mixed precision: of the mma.sync variants; the CUDA-core
-  // variants have their own kernel)
-  const bool mix = kprec == 1 && equation != DG_MAXWELL;
-  const int base_mode = split ? dg::MODE_SPLIT : (mix ? dg::MODE_TC : dg::MODE_RHS);
+  const int base_mode = split ? dg::MODE_SPLIT : dg::MODE_RHS;
   cudaError_t err = shape_of(equation, N, kprec, base_mode, &shape);
   if (err == cudaSuccess) {
     dg::LaunchShape other;
@@ -938,6 +935,19 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
       p->tcm_grid[k] = (int)(mtiles < mfull ? mtiles : mfull);
     }
   }
+  // Wave and Euler, mixed precision: dg_rhs_mixed_kernel (dg_mixed.cuh) on meshes
+  // that fill its 32-element tiles, else dg_rhs_kernel, whose tiles of 256 / Np
+  // elements finish sooner (one tile takes 7-11 us against 12-25).  The limits are
+  // where the RK stage's times cross, in elements per SM.  Measured (us, dg_rhs_kernel /
+  // dg_rhs_mixed_kernel): wave P1 at 316 14 / 16, at 546 23 / 22; wave P2 at 316
+  // 36 / 38, at 546 80 / 77; wave P3 at 68 21 / 23, at 162 44 / 40; wave P4 at 68
+  // 40 / 45, at 162 108 / 84; Euler P1 at 546 38 / 51, at 867 72 / 67; Euler P2 at 68
+  // 24 / 24, at 162 45 / 34; Euler P3 at 39 24 / 27, at 68 34 / 34, at 162 78 / 68.
+  // Both kernels give the same bits.
+  constexpr int kMixedPerSm[2][4] = {{540, 350, 120, 120}, {800, 100, 72, 72}};
+  const bool mix =
+      kprec == 1 && equation != DG_MAXWELL &&
+      p->nel >= (int64_t)kMixedPerSm[equation == DG_EULER ? 1 : 0][N - 1] * nsm;
   if (mix) {
     dg::LaunchShape x0, x1;
     err = equation == DG_WAVE ? dg::mixed_shape_wave(N, false, &x0)
@@ -997,11 +1007,20 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
   }
 
   if (split && !tc) {
+    // Wave and Euler from order 2 on: on meshes of fewer elements the general kernel's
+    // tiles of 256 / Np elements finish sooner than tiles of 32 (one tile per SM and
+    // less).  Measured (RHS, us, general / symmetric): at 1,296 elements, 8.5 per SM,
+    // wave P3 29 / 36, Euler P3 51 / 68, wave P4 72 / 72, Euler P4 132 / 135; at 3,072
+    // wave P3 51 / 38, Euler P3 91 / 75, Euler P4 250 / 142.  Order 1 and Maxwell (tiles
+    // of 16): no slower at any size (Maxwell P3 at 162 elements 55 / 36).
+    const int per_sm = equation == DG_MAXWELL || N == 1 ? 0 : (N == 4 ? 9 : 13);
     const bool strong = equation == DG_MAXWELL;
     std::vector<unsigned char> sops(
         dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong, nullptr, 0));
-    const int bytes = dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong,
-                                       sops.data(), (int)sops.size());
+    const int bytes = p->nel < (int64_t)per_sm * nsm
+                          ? 0
+                          : dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong,
+                                             sops.data(), (int)sops.size());
     if (bytes > 0) {  // the operators have the symmetry
       dg::LaunchShape s0, s1;
       err = sym_shape_of(equation, N, false, &s0);
@@ -1099,10 +1118,16 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     const int64_t afull = (int64_t)nsm * ashape.blocks_per_sm;
     p->adj_grid = (int)(atiles < afull ? atiles : afull);
 
+    // as for the RHS, with two phases per tile: measured (vjp, us, dense / symmetric)
+    // Euler P2 at 6,000 elements 103 / 109, at 10,368 162 / 151; Euler P3 at 3,072
+    // 129 / 142, at 6,000 245 / 209; Euler P4 at 1,296 174 / 222, at 3,072 256 / 241
+    const int per_sm = N <= 2 ? 48 : (N == 3 ? 32 : 16);
     std::vector<unsigned char> sops(
         dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes, nullptr, 0));
-    const int sbytes = dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes, sops.data(),
-                                            (int)sops.size());
+    const int sbytes = p->nel < (int64_t)per_sm * nsm
+                           ? 0
+                           : dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes,
+                                                  sops.data(), (int)sops.size());
     if (sbytes > 0) {  // the operators have the symmetry
       dg::LaunchShape sshape;
       err = equation == DG_WAVE ? dg::adjoint_sym_shape_wave(N, &sshape)

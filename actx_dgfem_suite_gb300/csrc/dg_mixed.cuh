@@ -1,6 +1,7 @@
 // Mixed-precision RHS of the wave and Euler equations on the CUDA cores
 // (sm_103a): FP32 derivative, flux and LIFT arithmetic on an FP64 state,
-// variants 0 (persistent) and 2 (one CTA per tile).
+// variants 0 (persistent) and 2 (one CTA per tile) of meshes that fill its tiles
+// (dg_plan_create; dg_rhs_kernel serves smaller ones).
 //
 // One lane per element and R = 5 rows of the operators per warp (P2-P4; 2 at P1),
 // so that operator entries are warp-uniform broadcasts shared by all fields of a
@@ -20,7 +21,7 @@
 // The arithmetic is that of dg_rhs_kernel in FP32, operation for operation: the
 // sums run over four columns at a time from the last to the first, derivatives
 // along t before s before r, LIFT continues the volume sum, so results are bit
-// for bit those of the one-thread-per-(element, node) kernel this one replaced.
+// for bit the same and the choice between the kernels is one of speed alone.
 //
 // What bounds it: instruction issue (55 % of the slots at Euler P3) and the
 // gathers' latency; hence loads issued ahead for R nodes and two face points at a

@@ -283,8 +283,6 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
   static_assert(!(SPLIT && T::MIXED), "the face-shared path is FP64 only");
   static_assert(!TCM || T::MIXED, "tensor-core products are a mixed-precision mode");
   static_assert(BLOCK == kBlock || TCM, "other tile shapes are MODE_TC variants");
-  static_assert(!T::MIXED || TCM || EQ == DG_MAXWELL,
-                "wave and Euler in FP32 on the CUDA cores: dg_rhs_mixed_kernel");
   static_assert(T::E >= 1, "at least one element per tile");
   constexpr int NP = T::NP, NFPT = T::NFPT, NF = T::NF, E = T::E;
   constexpr int ROW = T::ROW, FROW = T::FROW;  // shared-memory row pitches
@@ -515,30 +513,60 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
         auto row = [&](const Real* base, int r) {
           return reinterpret_cast<const float4*>(base + (r * E + el) * ROW);
         };
-        float d[6][3];
+        if constexpr (EQ == DG_WAVE) {
+          const float4* uv = row(sQr, 0);
+          const float4 *a0 = row(sAux, 0), *a1 = row(sAux, 1), *a2 = row(sAux, 2);
+          float ur0 = 0.f, ur1 = 0.f, ur2 = 0.f, dv = 0.f;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) d[k][0] = d[k][1] = d[k][2] = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < ROW / 4; ++jj) {
-          const float4 w0 = w0v[jj], w1 = w1v[jj], w2 = w2v[jj];
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            const float4 qv = row(sQr, k)[jj];
-            d[k][0] = dot4(w0, qv, d[k][0]);
-            d[k][1] = dot4(w1, qv, d[k][1]);
-            d[k][2] = dot4(w2, qv, d[k][2]);
+          for (int jj = 0; jj < ROW / 4; ++jj) {
+            const float4 w0 = w0v[jj], w1 = w1v[jj], w2 = w2v[jj], u = uv[jj];
+            ur0 = dot4(w0, u, ur0);
+            ur1 = dot4(w1, u, ur1);
+            ur2 = dot4(w2, u, ur2);
+            dv = dot4(w0, a0[jj], dot4(w1, a1[jj], dot4(w2, a2[jj], dv)));
           }
+          const Real c = p0;
+          vol[0] = -c * dv;
+#pragma unroll
+          for (int x = 0; x < 3; ++x)
+            vol[1 + x] = -c * fma(G[0 * 3 + x], ur0,
+                                  fma(G[1 * 3 + x], ur1, G[2 * 3 + x] * ur2));
+        } else if constexpr (EQ == DG_EULER) {
+#pragma unroll
+          for (int jj = 0; jj < ROW / 4; ++jj) {
+            const float4 w0 = w0v[jj], w1 = w1v[jj], w2 = w2v[jj];
+#pragma unroll
+            for (int k = 0; k < 5; ++k)
+              vol[k] = dot4(w0, row(sAux, k * 3 + 0)[jj],
+                            dot4(w1, row(sAux, k * 3 + 1)[jj],
+                                 dot4(w2, row(sAux, k * 3 + 2)[jj], vol[k])));
+          }
+        } else {  // DG_MAXWELL
+          float d[6][3];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) d[k][0] = d[k][1] = d[k][2] = 0.f;
+#pragma unroll
+          for (int jj = 0; jj < ROW / 4; ++jj) {
+            const float4 w0 = w0v[jj], w1 = w1v[jj], w2 = w2v[jj];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+              const float4 qv = row(sQr, k)[jj];
+              d[k][0] = dot4(w0, qv, d[k][0]);
+              d[k][1] = dot4(w1, qv, d[k][1]);
+              d[k][2] = dot4(w2, qv, d[k][2]);
+            }
+          }
+          auto dx = [&](int k, int x) {
+            return fma(G[0 * 3 + x], d[k][0],
+                       fma(G[1 * 3 + x], d[k][1], G[2 * 3 + x] * d[k][2]));
+          };
+          vol[0] = dx(5, 1) - dx(4, 2);
+          vol[1] = dx(3, 2) - dx(5, 0);
+          vol[2] = dx(4, 0) - dx(3, 1);
+          vol[3] = -(dx(2, 1) - dx(1, 2));
+          vol[4] = -(dx(0, 2) - dx(2, 0));
+          vol[5] = -(dx(1, 0) - dx(0, 1));
         }
-        auto dx = [&](int k, int x) {
-          return fma(G[0 * 3 + x], d[k][0],
-                     fma(G[1 * 3 + x], d[k][1], G[2 * 3 + x] * d[k][2]));
-        };
-        vol[0] = dx(5, 1) - dx(4, 2);
-        vol[1] = dx(3, 2) - dx(5, 0);
-        vol[2] = dx(4, 0) - dx(3, 1);
-        vol[3] = -(dx(2, 1) - dx(1, 2));
-        vol[4] = -(dx(0, 2) - dx(2, 0));
-        vol[5] = -(dx(1, 0) - dx(0, 1));
       } else if constexpr (EQ == DG_WAVE) {
         const Real c = p0;
         const Real* u = sQr + el * NP;

@@ -118,8 +118,9 @@ struct Tile {
   static constexpr int NA = NF / GROUPS;                    // fields of a thread
   static constexpr int E = 32 / GROUPS, PE = E + 1;
   static constexpr int BLOCK = 128;
-  // CTAs per SM the registers must allow (order-4 Euler: 168 instead of 186)
-  static constexpr int MIN_CTAS = N == 4 ? 3 : 4;
+  // CTAs per SM the registers must allow (order-4 Euler: 168 instead of 186; order-1
+  // Euler: 64 instead of 92)
+  static constexpr int MIN_CTAS = N == 4 ? 3 : (N == 1 && EQ == DG_EULER ? 8 : 4);
   static constexpr int CH = chunk_orbits<N>();
   static constexpr int X = Ops<N>::SIZE;
   static constexpr int X_BYTES = pad16(NF * B::NP * PE * 8);

@@ -62,19 +62,12 @@ cudaError_t launch_impl(const RhsArgs& a, int grid, cudaStream_t s) {
   }
 }
 
-// FP32 arithmetic on the CUDA cores: Maxwell here, wave and Euler in
-// dg_rhs_mixed_kernel (dg_mixed.cuh)
-template <int EQ, typename Real>
-constexpr bool kPlainModes = std::is_same<Real, double>::value || EQ == DG_MAXWELL;
-
 template <int N, int EQ, typename Real>
 cudaError_t shape_mode(int mode, LaunchShape* out) {
-  if constexpr (kPlainModes<EQ, Real>) {
-    switch (mode) {
-      case MODE_RHS: return shape_impl<N, EQ, Real, MODE_RHS>(out);
-      case MODE_STAGE: return shape_impl<N, EQ, Real, MODE_STAGE>(out);
-      default: break;
-    }
+  switch (mode) {
+    case MODE_RHS: return shape_impl<N, EQ, Real, MODE_RHS>(out);
+    case MODE_STAGE: return shape_impl<N, EQ, Real, MODE_STAGE>(out);
+    default: break;
   }
   if constexpr (std::is_same<Real, double>::value) {
     switch (mode) {
@@ -100,12 +93,10 @@ cudaError_t shape_mode(int mode, LaunchShape* out) {
 
 template <int N, int EQ, typename Real>
 cudaError_t launch_mode(int mode, const RhsArgs& a, int grid, cudaStream_t s) {
-  if constexpr (kPlainModes<EQ, Real>) {
-    switch (mode) {
-      case MODE_RHS: return launch_impl<N, EQ, Real, MODE_RHS>(a, grid, s);
-      case MODE_STAGE: return launch_impl<N, EQ, Real, MODE_STAGE>(a, grid, s);
-      default: break;
-    }
+  switch (mode) {
+    case MODE_RHS: return launch_impl<N, EQ, Real, MODE_RHS>(a, grid, s);
+    case MODE_STAGE: return launch_impl<N, EQ, Real, MODE_STAGE>(a, grid, s);
+    default: break;
   }
   if constexpr (std::is_same<Real, double>::value) {
     switch (mode) {

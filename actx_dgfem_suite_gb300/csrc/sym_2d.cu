@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "dg_launch.h"
+#include "dg_pair.h"
 #include "dg_sym2d.cuh"
 
 namespace dg {
@@ -151,23 +152,23 @@ int pack(const double* diff, const double* lift, const int32_t* edge_nodes, unsi
 
   // the operator in the basis of sums and differences, normalised for plain sums
   // on both sides; false unless the entries outside the pattern vanish
-  std::vector<long double> full;
+  std::vector<double> full;
   auto to_basis = [&](const Vec* in, int cols, int even, int flip, auto at) {
-    full.assign((size_t)NP * cols, 0.0L);
-    long double big = 0.0L, off = 0.0L;
+    full.assign((size_t)NP * cols, 0.0);
+    double big = 0.0, off = 0.0;
     for (int i = 0; i < NP; ++i)
       for (int c = 0; c < cols; ++c) {
-        long double s = 0.0L;
+        Pair s;
         for (int a = 0; a < node[i].n; ++a)
           for (int b = 0; b < in[c].n; ++b)
-            s += (long double)((a ? node[i].sign : 1) * (b ? in[c].sign : 1)) *
-                 at(node[i].idx[a], in[c].idx[b]);
-        s /= node[i].n * in[c].n;
-        full[(size_t)i * cols + c] = s;
-        if (!std::isfinite(s)) return false;
+            s.add((a ? node[i].sign : 1) * (b ? in[c].sign : 1),
+                  at(node[i].idx[a], in[c].idx[b]));
+        const double x = s.hi / (node[i].n * in[c].n);  // powers of two
+        full[(size_t)i * cols + c] = x;
+        if (!std::isfinite(x)) return false;
         const bool inside = ((i >= B::DE) ^ (c >= even)) == (flip != 0);
-        long double& m = inside ? big : off;
-        if (std::fabs(s) > m) m = std::fabs(s);
+        double& m = inside ? big : off;
+        if (std::fabs(x) > m) m = std::fabs(x);
       }
     return off <= kAsymmetry * big;
   };
@@ -176,8 +177,9 @@ int pack(const double* diff, const double* lift, const int32_t* edge_nodes, unsi
   for (int k = 0; k < 2; ++k) {
     // D' = (D_1 + D_2) / 2 and (D_1 - D_2) / 2
     if (!to_basis(node, NP, B::DE, k, [&](int i, int j) {
-          const long double d1 = diff[(size_t)i * NP + j], d2 = diff[(size_t)(NP + i) * NP + j];
-          return 0.5L * (k == 0 ? d1 + d2 : d1 - d2);
+          Pair s;
+          s.add(0.5, diff[(size_t)i * NP + j]);
+          return s.add(k == 0 ? 0.5 : -0.5, diff[(size_t)(NP + i) * NP + j]);
         }))
       return -1;
     for (int r = 0; r < 2; ++r) {
@@ -188,18 +190,18 @@ int pack(const double* diff, const double* lift, const int32_t* edge_nodes, unsi
       for (int j = 0; j < din; ++j)
         for (int i = 0; i < d; ++i)
           dst[j * pitch + i] =
-              (double)full[(size_t)(r * B::DE + i) * NP + s * B::DE + j];
+              full[(size_t)(r * B::DE + i) * NP + s * B::DE + j];
     }
   }
   if (!to_basis(edge, NFPT, B::FE, 0,
-                [&](int i, int fj) { return (long double)lift[(size_t)i * NFPT + fj]; }))
+                [&](int i, int fj) { return Pair(lift[(size_t)i * NFPT + fj]); }))
     return -1;
   for (int r = 0; r < 2; ++r) {
     const int pitch = r == 0 ? O::PE : O::PO, d = r == 0 ? B::DE : B::DO;
     double* dst = ops + (r == 0 ? O::LIFT0 : O::LIFT1);
     for (int o = 0; o < (r == 0 ? B::FE : B::FO); ++o)
       for (int i = 0; i < d; ++i)
-        dst[o * pitch + i] = (double)full[(size_t)(r * B::DE + i) * NFPT + r * B::FE + o];
+        dst[o * pitch + i] = full[(size_t)(r * B::DE + i) * NFPT + r * B::FE + o];
   }
   int32_t* ns = reinterpret_cast<int32_t*>(out + O::NODE_SLOT);
   int32_t* sn = reinterpret_cast<int32_t*>(out + O::SLOT_NODE);

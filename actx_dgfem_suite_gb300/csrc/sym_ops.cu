@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "dg_launch.h"
+#include "dg_pair.h"
 #include "dg_sym.cuh"
 
 namespace dg {
@@ -137,6 +138,14 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
         nsingle != B::NSG)
       return -1;
   }
+  // the combinations that each node enters, and with which sign
+  int nslots[NP] = {}, slots[NP][4], signs[NP][4];
+  for (int i = 0; i < NP; ++i)
+    for (int a = 0; a < node[i].n; ++a) {
+      const int n = node[i].idx[a];
+      slots[n][nslots[n]] = i;
+      signs[n][nslots[n]++] = node[i].sign[a];
+    }
   Vec face[NFPT];
   int face_slot[NFPT];
   for (int o = 0; o < NFP; ++o) {   // orbit o starts at point o of face 0
@@ -151,30 +160,33 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
 
   // an operator of `cols` columns in the combinations' basis (outputs by node
   // slot, inputs by slot of `in`), normalised for plain sums on both sides
-  std::vector<long double> half, full;
+  std::vector<Pair> half;
+  std::vector<double> full;
   auto to_basis = [&](const Vec* in, int cols, auto at) {
-    half.assign((size_t)NP * cols, 0.0L);
-    full.assign((size_t)NP * cols, 0.0L);
-    for (int i = 0; i < NP; ++i)
-      for (int a = 0; a < node[i].n; ++a)
-        for (int c = 0; c < cols; ++c)
-          half[(size_t)i * cols + c] += node[i].sign[a] * at(node[i].idx[a], c);
+    half.assign((size_t)NP * cols, Pair());
+    full.assign((size_t)NP * cols, 0.0);
+    for (int n = 0; n < NP; ++n)
+      for (int c = 0; c < cols; ++c) {
+        const Pair x = at(n, c);
+        for (int k = 0; k < nslots[n]; ++k)
+          half[(size_t)slots[n][k] * cols + c].add(signs[n][k], x);
+      }
     for (int i = 0; i < NP; ++i)
       for (int c = 0; c < cols; ++c) {
-        long double s = 0.0L;
+        Pair s;
         for (int b = 0; b < in[c].n; ++b)
-          s += in[c].sign[b] * half[(size_t)i * cols + in[c].idx[b]];
-        full[(size_t)i * cols + c] = s / (node[i].n * in[c].n);
+          s.add(in[c].sign[b], half[(size_t)i * cols + in[c].idx[b]]);
+        full[(size_t)i * cols + c] = s.hi / (node[i].n * in[c].n);  // powers of two
       }
   };
   // whether the entries outside the pattern vanish to rounding
   auto symmetric = [&](int cols, auto inside) {
-    long double big = 0.0L, off = 0.0L;
+    double big = 0.0, off = 0.0;
     for (int i = 0; i < NP; ++i)
       for (int c = 0; c < cols; ++c) {
-        const long double x = std::fabs(full[(size_t)i * cols + c]);
+        const double x = std::fabs(full[(size_t)i * cols + c]);
         if (!std::isfinite(x)) return false;
-        long double& m = inside(i, c) ? big : off;
+        double& m = inside(i, c) ? big : off;
         if (x > m) m = x;
       }
     return off <= kAsymmetry * big;
@@ -187,11 +199,10 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
   for (int k = 1; k < 4; ++k) {
     // D'_k = -1/2 (D_k - D_other - D_other')
     to_basis(node, NP, [&](int i, int j) {
-      long double s = 0.0L;
-      for (int r = 0; r < 3; ++r) {
-        const long double d = diff[(size_t)(r * NP + (ADJ ? j : i)) * NP + (ADJ ? i : j)];
-        s += r == k - 1 ? -0.5L * d : 0.5L * d;
-      }
+      Pair s;
+      for (int r = 0; r < 3; ++r)
+        s.add(r == k - 1 ? -0.5 : 0.5,
+              diff[(size_t)(r * NP + (ADJ ? j : i)) * NP + (ADJ ? i : j)]);
       return s;
     });
     if (!symmetric(NP, [&](int i, int j) {
@@ -206,16 +217,16 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
       double* dst = ops + (r == 0 ? 0 : F::VOL0 + (r - 1) * F::VOLB) + row * pitch;
       for (int j = 0; j < dim(s); ++j)
         for (int i = 0; i < dim(r); ++i)
-          dst[j * pitch + i] = (double)full[(size_t)(slot0(r) + i) * NP + slot0(s) + j];
+          dst[j * pitch + i] = full[(size_t)(slot0(r) + i) * NP + slot0(s) + j];
     }
   }
   to_basis(face, NFPT,
-           [&](int i, int fj) { return (long double)lift[(size_t)i * NFPT + fj]; });
+           [&](int i, int fj) { return Pair(lift[(size_t)i * NFPT + fj]); });
   if (!symmetric(NFPT, [&](int i, int c) { return part_of[i] == c / NFP; })) return -1;
   for (int r = 0; r < 4; ++r)
     for (int o = 0; o < NFP; ++o)
       for (int i = 0; i < dim(r); ++i) {
-        const double x = (double)full[(size_t)(slot0(r) + i) * NFPT + r * NFP + o];
+        const double x = full[(size_t)(slot0(r) + i) * NFPT + r * NFP + o];
         if constexpr (ADJ)
           ops[O::LIFT + (o / O::CH) * O::CHUNK + (slot0(r) + i) * O::PC + o % O::CH] = x;
         else

@@ -207,16 +207,20 @@ def test_asymmetric_operators_take_the_general_kernel(equation, order):
 @pytest.mark.gpu
 @pytest.mark.parametrize("equation", ["wave", "euler", "maxwell"])
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
-@pytest.mark.parametrize("nel", [1, 15, 16, 17, 31, 32, 33, 65])
-def test_tile_edges_match_the_general_kernel(equation, order, nel):
-    """Element counts around the tile sizes (16 and 32 elements), RHS and RK
-    stage with element scale: equal to the fused general kernel."""
+@pytest.mark.parametrize("extra", [0, 1, 15, 17, 31, 33])
+def test_tile_edges_match_the_general_kernel(equation, order, extra):
+    """Element counts around the tile sizes (16 and 32 elements) from the smallest
+    mesh that takes the kernel, RHS and RK stage with element scale: equal to the
+    fused general kernel."""
     import torch
 
     from actx_dgfem_suite_gb300.mesh import TetMesh
     from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
     from tests._helpers import jittered_box_mesh, make_problem
-    mesh = jittered_box_mesh(3)
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    nel = 1 if order == 1 or equation == "maxwell" else (9 if order == 4 else 13) * nsm
+    nel += extra
+    mesh = jittered_box_mesh(3 if nel < 100 else 7)
     mesh = TetMesh(vertices=mesh.vertices, elements=mesh.elements[:nel])
     prob = make_problem(equation, mesh, order, seed=nel)
     q = torch.from_numpy(prob.fields).cuda()
@@ -230,6 +234,7 @@ def test_tile_edges_match_the_general_kernel(equation, order, nel):
         res, qo, un = 0.5 * q, torch.empty_like(q), torch.empty_like(q)
         plan.rk_stage(q, qo, res, 0.3, 0.7, 1e-2, rhs_unscaled=un)
         plan.finish()
+        assert (plan.info()["block"] == 128) == partner
         got.append((r, res, qo, un))
     for a, b in zip(*got):
         # two orders of summation of the same products: 1e-12 as the parity bound
@@ -239,17 +244,20 @@ def test_tile_edges_match_the_general_kernel(equation, order, nel):
 @pytest.mark.gpu
 @pytest.mark.parametrize("equation", ["wave", "euler"])
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
-@pytest.mark.parametrize("nel", [1, 31, 32, 33, 65])
-def test_adjoint_tile_edges_match_the_dense_kernels(equation, order, nel):
+@pytest.mark.parametrize("extra", [0, 1, 31, 33])
+def test_adjoint_tile_edges_match_the_dense_kernels(equation, order, extra):
     """Transposed Jacobian and fused reverse stage with element scale around the
-    tile size, against the dense kernels: those run on operators moved off the
-    symmetry by 1e-11, which moves results by no more than that."""
+    tile size, from the smallest mesh that takes the kernels, against the dense
+    kernels: those run on operators moved off the symmetry by 1e-11, which moves
+    results by no more than that."""
     import torch
 
     from actx_dgfem_suite_gb300.mesh import TetMesh
     from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
     from tests._helpers import jittered_box_mesh, make_problem
-    mesh = jittered_box_mesh(3)
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    nel = (48, 48, 32, 16)[order - 1] * nsm + extra
+    mesh = jittered_box_mesh(11)
     mesh = TetMesh(vertices=mesh.vertices, elements=mesh.elements[:nel])
     prob = make_problem(equation, mesh, order, seed=nel)
     q = torch.from_numpy(prob.fields).cuda()
