@@ -31,9 +31,9 @@
 // others keep dg_rhs_kernel.
 //
 // Measured (GB300, CUDA events, whole RHS with its face kernel, dense kernel
-// before -> now): Maxwell P4 584,016 tets 38.9 -> 14.3 ms, Euler P4 118,098 tets
-// 7.08 -> 2.92 ms, wave P3 215,622 tets 2.69 -> 1.26 ms, Euler P2 LSRK step
-// 413,526 tets 16.7 -> 11.1 ms, wave P1 5.14 M tets 5.77 -> 4.56 ms.  ncu: FP64
+// before -> now): Maxwell P4 584,016 tets 38.9 -> 13.1 ms, Euler P4 118,098 tets
+// 7.08 -> 2.88 ms, wave P3 215,622 tets 2.69 -> 1.24 ms, Euler P2 LSRK step
+// 413,526 tets 16.7 -> 10.8 ms, wave P1 5.14 M tets 5.77 -> 4.17 ms.  ncu: FP64
 // pipe 83 % (wave P1) to 92 % (Maxwell P4) busy.
 //
 // Work split: a tile of E elements with one lane per element and one warp per
@@ -75,13 +75,24 @@ constexpr int chunk_orbits() {  // orbits of face values held at a time
   return N == 1 ? Basis<N>::NFP : (Basis<N>::NFP + 1) / 2;
 }
 
-template <int N>
+// Strong derivatives (RED; Maxwell from order 2 on): every D'_k maps into the
+// polynomials of degree N - 1, RA and RB of them in parts A and B_k, so the blocks
+// go to coefficients in an orthonormal basis of that space and one more block per
+// part takes the summed coefficients to the nodes: at order 4 175 multiply-adds per
+// field and direction plus 175 per field instead of 304 per field and direction
+// (Maxwell P4, 584,016 tets, whole RHS: 14.3 -> 13.1 ms).
+template <int N, bool RED = false>
 struct Ops {
   using B = Basis<N>;
+  static constexpr int RA = RED ? Basis<N - RED>::DA : B::DA;
+  static constexpr int RB = RED ? Basis<N - RED>::DB : B::DB;
   static constexpr int PA = (B::DA + 1) & ~1, PB = (B::DB + 1) & ~1;
-  static constexpr int VOL0 = 3 * B::DB * PA;               // entries of part 0
-  static constexpr int VOLB = (B::DA + 2 * B::DB) * PB;     // of each part B_k
-  static constexpr int LIFT = VOL0 + 3 * VOLB;
+  static constexpr int PRA = (RA + 1) & ~1, PRB = (RB + 1) & ~1;
+  static constexpr int VOL0 = 3 * B::DB * PRA;              // entries of part 0
+  static constexpr int VOLB = (B::DA + 2 * B::DB) * PRB;    // of each part B_k
+  static constexpr int EXP = VOL0 + 3 * VOLB;               // RED: coefficients -> nodes
+  static constexpr int EXPB = EXP + (RED ? RA * PA : 0);
+  static constexpr int LIFT = EXPB + (RED ? 3 * RB * PB : 0);
   static constexpr int LIFTB = LIFT + B::NFP * PA;
   static constexpr int ENTRIES = LIFTB + 3 * B::NFP * PB;
   static constexpr int NODE_SLOT = ENTRIES * 8;             // bytes from here
@@ -113,6 +124,7 @@ struct AdjOps {
 template <int N, int EQ>
 struct Tile {
   using B = Basis<N>;
+  using O = Ops<N, EQ == DG_MAXWELL && N != 1>;
   static constexpr int NF = EqInfo<EQ>::NF;
   static constexpr int GROUPS = EQ == DG_MAXWELL ? 2 : 1;
   static constexpr int NA = NF / GROUPS;                    // fields of a thread
@@ -122,7 +134,7 @@ struct Tile {
   // Euler: 64 instead of 92)
   static constexpr int MIN_CTAS = N == 4 ? 3 : (N == 1 && EQ == DG_EULER ? 8 : 4);
   static constexpr int CH = chunk_orbits<N>();
-  static constexpr int X = Ops<N>::SIZE;
+  static constexpr int X = O::SIZE;
   static constexpr int X_BYTES = pad16(NF * B::NP * PE * 8);
   static constexpr int F_BYTES = pad16(NF * 4 * CH * PE * 8);
   static constexpr int H = X + (X_BYTES > F_BYTES ? X_BYTES : F_BYTES);
@@ -242,8 +254,10 @@ __device__ __forceinline__ void block_product(const double* __restrict__ x,
   }
 }
 
-// In-place (inverse) transform of `narrays` node arrays of a tile.
-template <int N, int PE, int E, int BLOCK>
+// In-place (inverse) transform of `narrays` node arrays of a tile.  A_ONLY (order 1,
+// weak derivatives): the volume term reads part A alone, 3 of the butterfly's 8
+// additions (with the same for Euler below; wave P1, 5.14 M tets: 4.36 -> 4.17 ms).
+template <int N, int PE, int E, int BLOCK, bool A_ONLY = false>
 __device__ __forceinline__ void transform(double* x, int narrays) {
   using B = Basis<N>;
   constexpr int NO = B::NO4 + 3 * B::NPR;
@@ -253,7 +267,10 @@ __device__ __forceinline__ void transform(double* x, int narrays) {
     double* p = x + f * (B::NP * PE) + le;
     if (o < B::NO4) {
       double* b = p + (B::DA + o) * PE;
-      butterfly(p[o * PE], b[0], b[B::DB * PE], b[2 * B::DB * PE]);
+      if constexpr (A_ONLY)
+        p[o * PE] = (p[o * PE] + b[0]) + (b[B::DB * PE] + b[2 * B::DB * PE]);
+      else
+        butterfly(p[o * PE], b[0], b[B::DB * PE], b[2 * B::DB * PE]);
     } else {  // the pair of direction o - NO4 + 1
       double& u = p[o * PE];
       double& v = p[(B::DA + (o - B::NO4) * B::DB + B::NO4) * PE];
@@ -312,7 +329,10 @@ __device__ __forceinline__ void euler_inputs(const RhsArgs& a, int64_t e0, int e
     double* x = sX + el;
 #pragma unroll
     for (int m = 0; m < 5; ++m, x += XS) {
-      if constexpr (CNT == 4) {
+      if constexpr (N == 1) {  // order 1 reads part A alone
+        x[slot[0] * PE] = (f[m][0] + f[m][1]) + (f[m][2] + f[m][3]);
+        continue;
+      } else if constexpr (CNT == 4) {
         butterfly(f[m][0], f[m][1], f[m][2], f[m][3]);
       } else if constexpr (CNT == 2) {
         const double s = f[m][0] + f[m][1], d = f[m][0] - f[m][1];
@@ -341,7 +361,7 @@ template <int N, int EQ, bool STAGE>
 __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
     dg_rhs_sym_kernel(const RhsArgs a) {
   using T = Tile<N, EQ>;
-  using O = Ops<N>;
+  using O = typename T::O;
   using B = Basis<N>;
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT, NF = T::NF, NA = T::NA;
   constexpr int E = T::E, PE = T::PE, BLOCK = T::BLOCK;
@@ -408,7 +428,7 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
     }
     __syncthreads();
     if constexpr (EQ != DG_EULER) {
-      transform<N, PE, E, BLOCK>(sX, NF);
+      transform<N, PE, E, BLOCK, N == 1 && EQ == DG_WAVE>(sX, NF);
       __syncthreads();
     }
     // }}}
@@ -451,8 +471,9 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
       }
     };
 
-    auto part = [&](auto dtag, auto ptag, int slot0, const double* vops, const double* lops) {
-      constexpr int D = decltype(dtag)::value, P = decltype(ptag)::value;
+    auto part = [&](auto dtag, auto rtag, int slot0, const double* vops,
+                    [[maybe_unused]] const double* xops, const double* lops) {
+      constexpr int D = decltype(dtag)::value, P = (D + 1) & ~1;
       double acc[NA][D];
 #pragma unroll
       for (int m = 0; m < NA; ++m)
@@ -470,6 +491,24 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
           vops += din * P;
           cta_sync<BLOCK>();       // the inputs' slots are free
         }
+      } else if constexpr (EQ == DG_MAXWELL && N != 1) {
+        constexpr int R = decltype(rtag)::value, PR = (R + 1) & ~1;
+        double c[NA][R];           // coefficients of degree N - 1, then to the nodes
+#pragma unroll
+        for (int m = 0; m < NA; ++m)
+#pragma unroll
+          for (int i = 0; i < R; ++i) c[m][i] = 0.0;
+        volume<N, EQ, R, PR>(sX + le, sH + le, vops, rho, f_in, sgn, c);
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          double t[P];
+          load_row<P>(xops + j * P, t);
+#pragma unroll
+          for (int m = 0; m < NA; ++m)
+#pragma unroll
+            for (int i = 0; i < D; ++i) acc[m][i] = fma(t[i], c[m][j], acc[m][i]);
+        }
+        cta_sync<BLOCK>();         // the state's slots are free
       } else {
         volume<N, EQ, D, P>(sX + le, sH + le, vops, rho, f_in, sgn, acc);
         cta_sync<BLOCK>();         // the state's slots are free
@@ -492,13 +531,14 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
     };
     using IA = std::integral_constant<int, B::DA>;
     using IB = std::integral_constant<int, B::DB>;
-    using PA = std::integral_constant<int, O::PA>;
-    using PB = std::integral_constant<int, O::PB>;
-    if (B::DA != B::DB && rho == 0)
-      part(IA{}, PA{}, 0, ops, ops + O::LIFT);
+    using RA = std::integral_constant<int, O::RA>;
+    using RB = std::integral_constant<int, O::RB>;
+    if ((B::DA != B::DB || O::RA != O::RB) && rho == 0)
+      part(IA{}, RA{}, 0, ops, ops + O::EXP, ops + O::LIFT);
     else
-      part(IB{}, PB{}, rho == 0 ? 0 : B::DA + (rho - 1) * B::DB,
+      part(IB{}, RB{}, rho == 0 ? 0 : B::DA + (rho - 1) * B::DB,
            ops + (rho == 0 ? 0 : O::VOL0 + (rho - 1) * O::VOLB),
+           ops + (rho == 0 ? O::EXP : O::EXPB + (rho - 1) * (O::RB * O::PB)),
            ops + (rho == 0 ? O::LIFT : O::LIFTB + (rho - 1) * (NFP * O::PB)));
     __syncthreads();
     // }}}

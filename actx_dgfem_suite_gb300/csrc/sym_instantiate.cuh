@@ -23,7 +23,7 @@ struct SymKernel {
     out->smem_bytes = T::SMEM;
     out->blocks_per_sm = nb;
     out->elems_per_tile = T::E;
-    out->ops_bytes = sym::Ops<N>::SIZE;
+    out->ops_bytes = T::O::SIZE;
     out->threads = T::BLOCK;
     return err;
   }

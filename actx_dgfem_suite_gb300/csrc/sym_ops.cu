@@ -38,14 +38,62 @@ Vec combo(const int* orbit, int n, int part) {
   return v;
 }
 
-// ADJ: the blocks of the transposed operators (sym::AdjOps); `into_a`: which
-// order-1 blocks may be non-zero (those into part A, else those from it).
-template <int N, bool ADJ>
+double dot(const double* a, const double* b, int n) {  // rounded once
+  Pair s;
+  for (int k = 0; k < n; ++k) {
+    const double p = a[k] * b[k];
+    s.add(1.0, p).add(1.0, std::fma(a[k], b[k], -p));
+  }
+  return s.hi;
+}
+
+// Orthonormal basis q (rank x n) of the range of the columns x (cols x n):
+// Gram-Schmidt with the largest remaining column next, each orthogonalised twice.
+// False unless the columns have that rank to rounding.
+bool range_basis(std::vector<double> x, int cols, int n, int rank, double* q) {
+  auto norm = [&](int c) { return std::sqrt(dot(&x[c * n], &x[c * n], n)); };
+  double big = 0.0;
+  for (int c = 0; c < cols; ++c) big = std::fmax(big, norm(c));
+  for (int r = 0; r <= rank; ++r) {
+    int best = 0;
+    double len = -1.0;
+    for (int c = 0; c < cols; ++c) {
+      const double l = norm(c);
+      if (l > len) {
+        len = l;
+        best = c;
+      }
+    }
+    if (r == rank) return len <= 1e-13 * big;
+    if (!(len > 1e-6 * big)) return false;
+    double* v = q + r * n;
+    std::memcpy(v, &x[best * n], n * sizeof(double));
+    for (int pass = 0; pass < 2; ++pass) {
+      for (int p = 0; p < r; ++p) {
+        const double h = dot(q + p * n, v, n);
+        for (int k = 0; k < n; ++k) v[k] = std::fma(-h, q[p * n + k], v[k]);
+      }
+      const double l = std::sqrt(dot(v, v, n));
+      for (int k = 0; k < n; ++k) v[k] /= l;
+    }
+    for (int c = 0; c < cols; ++c)
+      for (int pass = 0; pass < 2; ++pass) {
+        const double h = dot(v, &x[c * n], n);
+        for (int k = 0; k < n; ++k) x[c * n + k] = std::fma(-h, v[k], x[c * n + k]);
+      }
+  }
+  return false;
+}
+
+// ADJ: the blocks of the transposed operators (sym::AdjOps); RED: derivatives
+// through coefficients of degree N - 1 (sym::Ops); `into_a`: which order-1 blocks
+// may be non-zero (those into part A, else those from it).
+template <int N, bool ADJ, bool RED = false>
 int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool into_a,
          unsigned char* out, int out_bytes) {
   using B = sym::Basis<N>;
-  using F = sym::Ops<N>;
-  using O = std::conditional_t<ADJ, sym::AdjOps<N>, sym::Ops<N>>;
+  using F = sym::Ops<N, RED>;
+  using O = std::conditional_t<ADJ, sym::AdjOps<N>, F>;
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT;
   if (!out) return O::SIZE;
   if (out_bytes < O::SIZE) return -1;
@@ -196,6 +244,7 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
 
   std::memset(out, 0, O::SIZE);
   double* ops = reinterpret_cast<double*>(out);
+  std::vector<double> block[4][3];  // of part r and direction k + 1, by columns
   for (int k = 1; k < 4; ++k) {
     // D'_k = -1/2 (D_k - D_other - D_other')
     to_basis(node, NP, [&](int i, int j) {
@@ -210,15 +259,29 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
           return (ri ^ rj) == k && (N != 1 || (into_a ? ri : rj) == 0);
         }))
       return -1;
-    for (int r = 0; r < 4; ++r) {
-      const int pitch = r == 0 ? F::PA : F::PB, s = r ^ k;
-      int row = 0;                  // rows of part r before direction k
-      for (int k2 = 1; k2 < k; ++k2) row += dim(r ^ k2);
-      double* dst = ops + (r == 0 ? 0 : F::VOL0 + (r - 1) * F::VOLB) + row * pitch;
-      for (int j = 0; j < dim(s); ++j)
+    for (int r = 0; r < 4; ++r)
+      for (int j = 0; j < dim(r ^ k); ++j)
         for (int i = 0; i < dim(r); ++i)
-          dst[j * pitch + i] = full[(size_t)(slot0(r) + i) * NP + slot0(s) + j];
+          block[r][k - 1].push_back(full[(size_t)(slot0(r) + i) * NP + slot0(r ^ k) + j]);
+  }
+  for (int r = 0; r < 4; ++r) {
+    const int d = dim(r), rows = r == 0 ? F::RA : F::RB;  // outputs of a block
+    std::vector<double> q((size_t)rows * d);
+    if constexpr (RED) {
+      std::vector<double> all;
+      for (int k = 0; k < 3; ++k) all.insert(all.end(), block[r][k].begin(), block[r][k].end());
+      if (!range_basis(all, (int)all.size() / d, d, rows, q.data())) return -1;
+      double* dst = ops + (r == 0 ? F::EXP : F::EXPB + (r - 1) * (F::RB * F::PB));
+      for (int j = 0; j < rows; ++j)
+        for (int i = 0; i < d; ++i) dst[j * (r == 0 ? F::PA : F::PB) + i] = q[j * d + i];
     }
+    const int pitch = r == 0 ? F::PRA : F::PRB;
+    double* dst = ops + (r == 0 ? 0 : F::VOL0 + (r - 1) * F::VOLB);
+    for (int k = 0; k < 3; ++k)
+      for (int j = 0; j < dim(r ^ (k + 1)); ++j, dst += pitch)
+        for (int i = 0; i < rows; ++i)
+          dst[i] = RED ? dot(&q[(size_t)i * d], &block[r][k][(size_t)j * d], d)
+                       : block[r][k][(size_t)j * d + i];
   }
   to_basis(face, NFPT,
            [&](int i, int fj) { return Pair(lift[(size_t)i * NFPT + fj]); });
@@ -246,11 +309,14 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
 
 int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
                  bool strong, unsigned char* out, int out_bytes) {
-  switch (order) {
+  switch (strong && order > 1 ? -order : order) {
     case 1: return pack<1, false>(diff, lift, face_nodes, strong, out, out_bytes);
-    case 2: return pack<2, false>(diff, lift, face_nodes, strong, out, out_bytes);
-    case 3: return pack<3, false>(diff, lift, face_nodes, strong, out, out_bytes);
-    case 4: return pack<4, false>(diff, lift, face_nodes, strong, out, out_bytes);
+    case 2: return pack<2, false>(diff, lift, face_nodes, false, out, out_bytes);
+    case 3: return pack<3, false>(diff, lift, face_nodes, false, out, out_bytes);
+    case 4: return pack<4, false>(diff, lift, face_nodes, false, out, out_bytes);
+    case -2: return pack<2, false, true>(diff, lift, face_nodes, true, out, out_bytes);
+    case -3: return pack<3, false, true>(diff, lift, face_nodes, true, out, out_bytes);
+    case -4: return pack<4, false, true>(diff, lift, face_nodes, true, out, out_bytes);
     default: return -1;
   }
 }

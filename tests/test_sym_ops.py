@@ -36,7 +36,7 @@ def _pack(order, diff, lift, face_nodes, strong=None):
 class _Blocks:
     """The operator block of order N read back in the kernel's layout."""
 
-    def __init__(self, order, buf, adjoint=False):
+    def __init__(self, order, buf, adjoint=False, reduced=False):
         self.np_ = (order + 1) * (order + 2) * (order + 3) // 6
         self.nfp = (order + 1) * (order + 2) // 2
         npr, nsg = int(order % 2 == 0), int(order == 4)
@@ -49,11 +49,20 @@ class _Blocks:
         x = buf.view(np.float64) if buf.size % 8 == 0 else None
         pos = 0
         self.vol, self.lift = {}, {}
+        # derivatives through coefficients of one degree less: their number per part
+        rank = {2: (1, 1), 3: (4, 2), 4: (5, 5)}[order] if reduced else (dim[0], dim[1])
+        rank = [rank[0]] + 3 * [rank[1]]
         for r in range(4):
             for k in range(1, 4):
-                n = dim[r ^ k] * pitch[r]
-                self.vol[r, k] = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
+                n = dim[r ^ k] * even(rank[r])
+                self.vol[r, k] = x[pos:pos + n].reshape(-1, even(rank[r]))[:, :rank[r]].T
                 pos += n
+        for r in range(4 if reduced else 0):
+            n = rank[r] * pitch[r]
+            expand = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
+            pos += n
+            for k in range(1, 4):
+                self.vol[r, k] = expand @ self.vol[r, k]
         if adjoint:                              # chunks of orbits, rows by node slot
             ch = self.nfp if order == 1 else (self.nfp + 1) // 2
             nch = -(-self.nfp // ch)
@@ -97,7 +106,8 @@ class _Blocks:
 def test_blocks_reproduce_the_dense_operators(order, strong):
     ref = reference_tet(order)
     diff = ref.diff if strong else ref.weak_diff
-    b = _Blocks(order, _pack(order, diff, ref.lift, ref.face_nodes, strong))
+    b = _Blocks(order, _pack(order, diff, ref.lift, ref.face_nodes, strong),
+                reduced=strong and order > 1)
     assert sorted(b.node_slot) == list(range(b.np_))
     assert list(b.slot_node[b.node_slot]) == list(range(b.np_))
     assert sorted(b.face_point) == list(range(4 * b.nfp))
@@ -149,6 +159,13 @@ def test_adjoint_blocks_are_the_transposed_blocks(order):
     bad = ref.weak_diff.copy()
     bad[0, 1, 0] += 1e-9
     assert _pack(order, bad, ref.lift, ref.face_nodes) is None
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_strong_operators_that_keep_the_degree_are_refused(order):
+    """Weak derivatives have the symmetry, but reach all of degree N."""
+    ref = reference_tet(order)
+    assert _pack(order, ref.weak_diff, ref.lift, ref.face_nodes, True) is None
 
 
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
