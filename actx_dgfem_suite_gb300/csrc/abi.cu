@@ -1014,13 +1014,13 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     // wave P3 51 / 38, Euler P3 91 / 75, Euler P4 250 / 142.  Order 1 and Maxwell (tiles
     // of 16): no slower at any size (Maxwell P3 at 162 elements 55 / 36).
     const int per_sm = equation == DG_MAXWELL || N == 1 ? 0 : (N == 4 ? 9 : 13);
-    const bool strong = equation == DG_MAXWELL;
+    const bool strong = equation == DG_MAXWELL, reduce = equation != DG_EULER;
     std::vector<unsigned char> sops(
-        dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong, nullptr, 0));
+        dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong, reduce, nullptr, 0));
     const int bytes = p->nel < (int64_t)per_sm * nsm
                           ? 0
                           : dg::pack_sym_ops(N, diff, mesh->lift, mesh->face_nodes, strong,
-                                             sops.data(), (int)sops.size());
+                                             reduce, sops.data(), (int)sops.size());
     if (bytes > 0) {  // the operators have the symmetry
       dg::LaunchShape s0, s1;
       err = sym_shape_of(equation, N, false, &s0);
@@ -1123,11 +1123,13 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     // 129 / 142, at 6,000 245 / 209; Euler P4 at 1,296 174 / 222, at 3,072 256 / 241
     const int per_sm = N <= 2 ? 48 : (N == 3 ? 32 : 16);
     std::vector<unsigned char> sops(
-        dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes, nullptr, 0));
+        dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes, equation == DG_WAVE, nullptr,
+                             0));
     const int sbytes = p->nel < (int64_t)per_sm * nsm
                            ? 0
                            : dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes,
-                                                  sops.data(), (int)sops.size());
+                                                  equation == DG_WAVE, sops.data(),
+                                                  (int)sops.size());
     if (sbytes > 0) {  // the operators have the symmetry
       dg::LaunchShape sshape;
       err = equation == DG_WAVE ? dg::adjoint_sym_shape_wave(N, &sshape)

@@ -101,16 +101,17 @@ int pack_tcm_ops(int order, const double* diff, const double* lift,
                  bool tf32);
 
 // Operator block of the symmetry-adapted kernels (sym::Ops in dg_sym.cuh);
-// `strong`: diff holds strong derivatives.  Returns the block size (out ==
-// NULL: size only), or -1 when the operators do not have the tetrahedron's
-// four-group symmetry to rounding (or out_bytes is short).
+// `strong`: diff holds strong derivatives; `reduce`: products through coefficients of
+// one degree less (wave and Maxwell).  Returns the block size (out == NULL: size
+// only), or -1 when the operators do not have the tetrahedron's four-group symmetry
+// or, with `reduce`, do not lower the degree to rounding (or out_bytes is short).
 int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
-                 bool strong, unsigned char* out, int out_bytes);
+                 bool strong, bool reduce, unsigned char* out, int out_bytes);
 
 // The same for the adjoint kernels (sym::AdjOps): transposed weak derivatives
 // and transposed LIFT.
 int pack_sym_adj_ops(int order, const double* weak, const double* lift,
-                     const int32_t* face_nodes, unsigned char* out, int out_bytes);
+                     const int32_t* face_nodes, bool reduce, unsigned char* out, int out_bytes);
 
 // Mixed precision on the CUDA cores, wave and Euler (dg_mixed.cuh): shape and
 // launch (stage: fused RK stage) of the main kernel, Euler's launch before it that

@@ -23,6 +23,8 @@
 //   order 1 / 2 / 3 / 4       16 / 100 / 400 / 1225 dense     48 / 240 / 800 / 2100
 //                              1 /  24 / 100 /  304 here      12 /  60 / 200 /  525
 //
+// (wave and Maxwell fewer still: see Ops).
+//
 // The direction metric follows from the element's dr/dx:
 // sum_r g_r D_r = sum_k h_k D'_k with h_1 = g_2 + g_3 (cyclic) and
 // D'_k = -1/2 D_{d_k}; the host folds all constants and the butterflies'
@@ -32,7 +34,7 @@
 //
 // Measured (GB300, CUDA events, whole RHS with its face kernel, dense kernel
 // before -> now): Maxwell P4 584,016 tets 38.9 -> 13.1 ms, Euler P4 118,098 tets
-// 7.08 -> 2.88 ms, wave P3 215,622 tets 2.69 -> 1.24 ms, Euler P2 LSRK step
+// 7.08 -> 2.88 ms, wave P3 215,622 tets 2.69 -> 1.17 ms, Euler P2 LSRK step
 // 413,526 tets 16.7 -> 10.8 ms, wave P1 5.14 M tets 5.77 -> 4.17 ms.  ncu: FP64
 // pipe 83 % (wave P1) to 92 % (Maxwell P4) busy.
 //
@@ -75,38 +77,64 @@ constexpr int chunk_orbits() {  // orbits of face values held at a time
   return N == 1 ? Basis<N>::NFP : (Basis<N>::NFP + 1) / 2;
 }
 
-// Strong derivatives (RED; Maxwell from order 2 on): every D'_k maps into the
-// polynomials of degree N - 1, RA and RB of them in parts A and B_k, so the blocks
-// go to coefficients in an orthonormal basis of that space and one more block per
-// part takes the summed coefficients to the nodes: at order 4 175 multiply-adds per
-// field and direction plus 175 per field instead of 304 per field and direction
-// (Maxwell P4, 584,016 tets, whole RHS: 14.3 -> 13.1 ms).
-template <int N, bool RED = false>
+// A derivative lowers the degree by one.  Strong derivatives (RED = 1) therefore map
+// into the polynomials of degree N - 1, RA and RB of them in parts A and B_k: the
+// blocks go to coefficients in an orthonormal basis of that space and one more block
+// per part takes the summed coefficients to the nodes.  Weak derivatives (RED = 2)
+// see of their input only its projection onto that space: one block per part takes
+// the nodes to coefficients, which the volume blocks read.  A field's product along
+// one direction costs 10 / 50 / 175 multiply-adds at orders 2 / 3 / 4 (24 / 100 / 304
+// without), the extra block as much once per field: less where fields share a
+// product's result (Maxwell P4, 584,016 tets, whole RHS: 14.3 -> 13.1 ms) or a field
+// enters several (wave P3, 215,622 tets: 1.24 -> 1.17 ms).  Order 1 has one non-zero
+// block per direction as it is, and Euler's 15 products have 15 different inputs.
+enum { RED_NONE = 0, RED_OUT = 1, RED_IN = 2 };
+
+template <int N, int EQ>
+constexpr int reduction() {
+  return N == 1 || EQ == DG_EULER ? RED_NONE : (EQ == DG_MAXWELL ? RED_OUT : RED_IN);
+}
+
+template <int N, int RED = RED_NONE>
 struct Ops {
   using B = Basis<N>;
-  static constexpr int RA = RED ? Basis<N - RED>::DA : B::DA;
-  static constexpr int RB = RED ? Basis<N - RED>::DB : B::DB;
+  static constexpr int RA = RED ? Basis<N - (RED != 0)>::DA : B::DA;
+  static constexpr int RB = RED ? Basis<N - (RED != 0)>::DB : B::DB;
+  // inputs and outputs of the volume blocks in part A and in the others
+  static constexpr int INA = RED == RED_IN ? RA : B::DA, INB = RED == RED_IN ? RB : B::DB;
+  static constexpr int OUTA = RED == RED_OUT ? RA : B::DA, OUTB = RED == RED_OUT ? RB : B::DB;
   static constexpr int PA = (B::DA + 1) & ~1, PB = (B::DB + 1) & ~1;
   static constexpr int PRA = (RA + 1) & ~1, PRB = (RB + 1) & ~1;
-  static constexpr int VOL0 = 3 * B::DB * PRA;              // entries of part 0
-  static constexpr int VOLB = (B::DA + 2 * B::DB) * PRB;    // of each part B_k
-  static constexpr int EXP = VOL0 + 3 * VOLB;               // RED: coefficients -> nodes
-  static constexpr int EXPB = EXP + (RED ? RA * PA : 0);
-  static constexpr int LIFT = EXPB + (RED ? 3 * RB * PB : 0);
+  static constexpr int POA = (OUTA + 1) & ~1, POB = (OUTB + 1) & ~1;
+  static constexpr int VOL0 = 3 * INB * POA;                // entries of part 0
+  static constexpr int VOLB = (INA + 2 * INB) * POB;        // of each part B_k
+  // coefficients -> nodes (RA rows of pitch PA) or nodes -> coefficients (DA of PRA)
+  static constexpr int EXTRA = VOL0 + 3 * VOLB;
+  static constexpr int EXA = RED == RED_NONE ? 0 : (RED == RED_OUT ? RA * PA : B::DA * PRA);
+  static constexpr int EXB = RED == RED_NONE ? 0 : (RED == RED_OUT ? RB * PB : B::DB * PRB);
+  static constexpr int LIFT = EXTRA + EXA + 3 * EXB;
   static constexpr int LIFTB = LIFT + B::NFP * PA;
   static constexpr int ENTRIES = LIFTB + 3 * B::NFP * PB;
   static constexpr int NODE_SLOT = ENTRIES * 8;             // bytes from here
   static constexpr int SLOT_NODE = NODE_SLOT + pad16(B::NP * 4);
   static constexpr int FACE_POINT = SLOT_NODE + pad16(B::NP * 4);
   static constexpr int SIZE = FACE_POINT + pad16(B::NFPT * 4);
+  static __host__ __device__ constexpr int volume(int rho) {
+    return rho == 0 ? 0 : VOL0 + (rho - 1) * VOLB;
+  }
+  static __host__ __device__ constexpr int extra(int rho) {
+    return EXTRA + (rho == 0 ? 0 : EXA + (rho - 1) * EXB);
+  }
 };
 
-template <int N>
+// RED: RED_OUT for the transposed weak derivatives (wave), RED_NONE
+template <int N, int RED = RED_NONE>
 struct AdjOps {
   using B = Basis<N>;
+  using F = Ops<N, RED>;
   static constexpr int CH = chunk_orbits<N>(), NCH = (B::NFP + CH - 1) / CH;
   static constexpr int PC = (CH + 1) & ~1;
-  static constexpr int LIFT = Ops<N>::LIFT;                 // entries before LIFT^T
+  static constexpr int LIFT = F::LIFT;                      // entries before LIFT^T
   static constexpr int CHUNK = B::NP * PC;                  // entries of a chunk
   static constexpr int NODE_SLOT = (LIFT + NCH * CHUNK) * 8;
   static constexpr int SLOT_NODE = NODE_SLOT + pad16(B::NP * 4);
@@ -124,7 +152,7 @@ struct AdjOps {
 template <int N, int EQ>
 struct Tile {
   using B = Basis<N>;
-  using O = Ops<N, EQ == DG_MAXWELL && N != 1>;
+  using O = Ops<N, reduction<N, EQ>()>;
   static constexpr int NF = EqInfo<EQ>::NF;
   static constexpr int GROUPS = EQ == DG_MAXWELL ? 2 : 1;
   static constexpr int NA = NF / GROUPS;                    // fields of a thread
@@ -169,12 +197,12 @@ __device__ __forceinline__ void load_row(const double* p, double (&r)[P]) {
   }
 }
 
-// Volume term of part rho (D outputs, row pitch P), wave and Maxwell.  x: the
-// thread's element in shared memory; h: metric of the three directions (pitch
+// Volume term of part rho (D outputs, row pitch P; IA and IB inputs of parts A and
+// B_k), wave and Maxwell.  x: the thread's element in shared memory; h: metric of the three directions (pitch
 // PE per entry); f0: first input field (Maxwell); sgn: Maxwell's curl sign,
 // wave's -c.  At order 1 one block per direction is not zero: into part A for
 // strong (and transposed weak) derivatives, from part A for weak ones.
-template <int N, int EQ, int D, int P, bool INTO_A = EQ == DG_MAXWELL>
+template <int N, int EQ, int D, int P, int IA, int IB, bool INTO_A = EQ == DG_MAXWELL>
 __device__ __forceinline__ void volume(const double* __restrict__ x,
                                        const double* __restrict__ h,
                                        const double* __restrict__ row, int rho, int f0,
@@ -184,7 +212,7 @@ __device__ __forceinline__ void volume(const double* __restrict__ x,
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int sig = rho ^ (k + 1);
-    const int din = sig == 0 ? B::DA : B::DB;
+    const int din = sig == 0 ? IA : IB;
     const double* xs = x + (sig == 0 ? 0 : B::DA + (sig - 1) * B::DB) * PE;
     if (N == 1 && (INTO_A ? rho : sig) != 0) {
       row += din * P;
@@ -251,6 +279,21 @@ __device__ __forceinline__ void block_product(const double* __restrict__ x,
     for (int m = 0; m < NA; ++m)
 #pragma unroll
       for (int i = 0; i < D; ++i) acc[m][i] = fma(t[i], v[m], acc[m][i]);
+  }
+}
+
+// acc += expansion of the coefficients c (part's R rows of pitch P).
+template <int NA, int R, int D, int P>
+__device__ __forceinline__ void expand(const double* __restrict__ row,
+                                       const double (&c)[NA][R], double (&acc)[NA][D]) {
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    double t[P];
+    load_row<P>(row + j * P, t);
+#pragma unroll
+    for (int m = 0; m < NA; ++m)
+#pragma unroll
+      for (int i = 0; i < D; ++i) acc[m][i] = fma(t[i], c[m][j], acc[m][i]);
   }
 }
 
@@ -366,6 +409,7 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT, NF = T::NF, NA = T::NA;
   constexpr int E = T::E, PE = T::PE, BLOCK = T::BLOCK;
   constexpr int XS = NP * PE, CH = T::CH, FS = 4 * CH * PE;  // array strides
+  constexpr int RED = reduction<N, EQ>();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t bar;
   __shared__ int ops_ok;
@@ -471,9 +515,11 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
       }
     };
 
-    auto part = [&](auto dtag, auto rtag, int slot0, const double* vops,
-                    [[maybe_unused]] const double* xops, const double* lops) {
+    auto part = [&](auto dtag, auto rtag, int slot0, const double* lops) {
       constexpr int D = decltype(dtag)::value, P = (D + 1) & ~1;
+      constexpr int R = decltype(rtag)::value, PR = (R + 1) & ~1;
+      const double* vops = ops + O::volume(rho);
+      [[maybe_unused]] const double* xops = ops + O::extra(rho);
       double acc[NA][D];
 #pragma unroll
       for (int m = 0; m < NA; ++m)
@@ -491,26 +537,31 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
           vops += din * P;
           cta_sync<BLOCK>();       // the inputs' slots are free
         }
-      } else if constexpr (EQ == DG_MAXWELL && N != 1) {
-        constexpr int R = decltype(rtag)::value, PR = (R + 1) & ~1;
-        double c[NA][R];           // coefficients of degree N - 1, then to the nodes
+      } else if constexpr (RED == RED_OUT) {
+        double c[NA][R];
 #pragma unroll
         for (int m = 0; m < NA; ++m)
 #pragma unroll
           for (int i = 0; i < R; ++i) c[m][i] = 0.0;
-        volume<N, EQ, R, PR>(sX + le, sH + le, vops, rho, f_in, sgn, c);
-#pragma unroll
-        for (int j = 0; j < R; ++j) {
-          double t[P];
-          load_row<P>(xops + j * P, t);
-#pragma unroll
-          for (int m = 0; m < NA; ++m)
-#pragma unroll
-            for (int i = 0; i < D; ++i) acc[m][i] = fma(t[i], c[m][j], acc[m][i]);
-        }
+        volume<N, EQ, R, PR, O::INA, O::INB>(sX + le, sH + le, vops, rho, f_in, sgn, c);
+        expand<NA, R, D, P>(xops, c, acc);
         cta_sync<BLOCK>();         // the state's slots are free
       } else {
-        volume<N, EQ, D, P>(sX + le, sH + le, vops, rho, f_in, sgn, acc);
+        if constexpr (RED == RED_IN) {  // the part's coefficients, in its first slots
+          double c[NF][R];
+#pragma unroll
+          for (int m = 0; m < NF; ++m)
+#pragma unroll
+            for (int i = 0; i < R; ++i) c[m][i] = 0.0;
+          double* x = sX + slot0 * PE + le;
+          block_product<NF, R, PR, PE, XS>(x, xops, D, c);
+#pragma unroll
+          for (int m = 0; m < NF; ++m)
+#pragma unroll
+            for (int i = 0; i < R; ++i) x[m * XS + i * PE] = c[m][i];
+          cta_sync<BLOCK>();
+        }
+        volume<N, EQ, D, P, O::INA, O::INB>(sX + le, sH + le, vops, rho, f_in, sgn, acc);
         cta_sync<BLOCK>();         // the state's slots are free
       }
 #pragma unroll 1
@@ -534,11 +585,9 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
     using RA = std::integral_constant<int, O::RA>;
     using RB = std::integral_constant<int, O::RB>;
     if ((B::DA != B::DB || O::RA != O::RB) && rho == 0)
-      part(IA{}, RA{}, 0, ops, ops + O::EXP, ops + O::LIFT);
+      part(IA{}, RA{}, 0, ops + O::LIFT);
     else
       part(IB{}, RB{}, rho == 0 ? 0 : B::DA + (rho - 1) * B::DB,
-           ops + (rho == 0 ? 0 : O::VOL0 + (rho - 1) * O::VOLB),
-           ops + (rho == 0 ? O::EXP : O::EXPB + (rho - 1) * (O::RB * O::PB)),
            ops + (rho == 0 ? O::LIFT : O::LIFTB + (rho - 1) * (NFP * O::PB)));
     __syncthreads();
     // }}}

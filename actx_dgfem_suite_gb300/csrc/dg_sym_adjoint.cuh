@@ -32,7 +32,7 @@ namespace sym {
 template <int N, int EQ>
 struct AdjTile {
   using B = Basis<N>;
-  using O = AdjOps<N>;
+  using O = AdjOps<N, EQ == DG_WAVE && N != 1 ? RED_OUT : RED_NONE>;
   static constexpr int NF = EqInfo<EQ>::NF;
   static constexpr int E = 32, PE = E + 1, BLOCK = 128;
   static constexpr int X = O::SIZE;
@@ -79,12 +79,11 @@ __device__ __forceinline__ void load_metric(const double* mt, int ecount, double
 }
 
 // The chunk's face adjoints of part rho (DIN inputs) into sF (transformed).
-template <int N, int NF, int DIN, int PE>
+template <int N, class O, int NF, int DIN, int PE>
 __device__ __forceinline__ void lift_transposed(const double* __restrict__ x,
                                                 const double* __restrict__ row, int rho,
                                                 double* __restrict__ f) {
   using B = Basis<N>;
-  using O = AdjOps<N>;
   constexpr int XS = B::NP * PE, FS = 4 * O::CH * PE;
   double acc[NF][O::CH];
 #pragma unroll
@@ -109,29 +108,24 @@ __device__ __forceinline__ void lift_transposed(const double* __restrict__ x,
     for (int o = 0; o < O::CH; ++o) f[m * FS + o * PE] = acc[m][o];
 }
 
-// f(DIN, slot0): the part's size as a compile-time constant
-template <int N, class F>
+// f(DIN, R, slot0): the part's size and its volume blocks' as compile-time constants
+template <int N, class O, class F>
 __device__ __forceinline__ void with_part(int rho, F f) {
   using B = Basis<N>;
-  if (B::DA != B::DB && rho == 0)
-    f(std::integral_constant<int, B::DA>{}, std::integral_constant<int, Ops<N>::PA>{}, 0);
+  if ((B::DA != B::DB || O::F::RA != O::F::RB) && rho == 0)
+    f(std::integral_constant<int, B::DA>{}, std::integral_constant<int, O::F::RA>{}, 0);
   else
-    f(std::integral_constant<int, B::DB>{}, std::integral_constant<int, Ops<N>::PB>{},
+    f(std::integral_constant<int, B::DB>{}, std::integral_constant<int, O::F::RB>{},
       rho == 0 ? 0 : B::DA + (rho - 1) * B::DB);
 }
 
-// offset of part rho's volume blocks
-template <int N>
-__device__ __forceinline__ int volume_offset(int rho) {
-  return rho == 0 ? 0 : Ops<N>::VOL0 + (rho - 1) * Ops<N>::VOLB;
-}
-
-// Wave P3, 16,464 tets, reverse stage: 177 us dense, 127 us here.
+// Wave P3, 16,464 tets, reverse stage: 177 us dense, 127 us here (vjp at 82,944 tets,
+// both launches, with the derivatives reduced as in dg_sym.cuh: 572 -> 557 us).
 template <int N, bool STAGE>
 __global__ void __launch_bounds__(AdjTile<N, DG_WAVE>::BLOCK)
     dg_wave_adjoint_sym_kernel(const AdjArgs a) {
   using T = AdjTile<N, DG_WAVE>;
-  using O = AdjOps<N>;
+  using O = typename T::O;
   using B = Basis<N>;
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT, CH = O::CH;
   constexpr int E = T::E, PE = T::PE, BLOCK = T::BLOCK, XS = NP * PE, FS = 4 * CH * PE;
@@ -199,8 +193,8 @@ __global__ void __launch_bounds__(AdjTile<N, DG_WAVE>::BLOCK)
 #pragma unroll 1
     for (int c = 0; c < O::NCH; ++c) {
       const double* lops = ops + O::LIFT + c * O::CHUNK;
-      with_part<N>(rho, [&](auto dtag, auto, int slot0) {
-        lift_transposed<N, 4, decltype(dtag)::value, PE>(sX + slot0 * PE + le,
+      with_part<N, O>(rho, [&](auto dtag, auto, int slot0) {
+        lift_transposed<N, O, 4, decltype(dtag)::value, PE>(sX + slot0 * PE + le,
                                                          lops + slot0 * O::PC, rho, sF + le);
       });
       __syncthreads();
@@ -230,15 +224,21 @@ __global__ void __launch_bounds__(AdjTile<N, DG_WAVE>::BLOCK)
     // }}}
 
     // {{{ volume transpose: -sum_r W_r^T (G v)_r and -G^T W_r^T u
-    with_part<N>(rho, [&](auto dtag, auto ptag, int slot0) {
-      constexpr int D = decltype(dtag)::value;
-      double acc[4][D];
+    with_part<N, O>(rho, [&](auto dtag, auto rtag, int slot0) {
+      constexpr int D = decltype(dtag)::value, R = decltype(rtag)::value;
+      double acc[4][D], c[4][R];
 #pragma unroll
       for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int i = 0; i < D; ++i) acc[m][i] = 0.0;
-      volume<N, DG_WAVE, D, decltype(ptag)::value, true>(
-          sX + le, sH + le, ops + volume_offset<N>(rho), rho, 0, -1.0, acc);
+        for (int i = 0; i < R; ++i) c[m][i] = 0.0;
+      volume<N, DG_WAVE, R, (R + 1) & ~1, B::DA, B::DB, true>(
+          sX + le, sH + le, ops + O::F::volume(rho), rho, 0, -1.0, c);
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int i = 0; i < D; ++i) acc[m][i] = N == 1 ? c[m][i % R] : 0.0;
+      if constexpr (N != 1)
+        expand<4, R, D, (D + 1) & ~1>(ops + O::F::extra(rho), c, acc);
       cta_sync<BLOCK>();  // every warp has read its inputs
 #pragma unroll
       for (int m = 0; m < 4; ++m)
@@ -264,7 +264,7 @@ template <int N>
 __global__ void __launch_bounds__(AdjTile<N, DG_EULER>::BLOCK)
     dg_euler_vjp_sym_kernel(const VjpArgs a) {
   using T = AdjTile<N, DG_EULER>;
-  using O = AdjOps<N>;
+  using O = typename T::O;
   using B = Basis<N>;
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT, CH = O::CH;
   constexpr int DA = B::DA, DB = B::DB, NO4 = B::NO4;
@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(AdjTile<N, DG_EULER>::BLOCK)
 #pragma unroll 1
     for (int c = 0; c < O::NCH; ++c) {
       const double* lops = ops + O::LIFT + c * O::CHUNK;
-      with_part<N>(rho, [&](auto dtag, auto, int slot0) {
-        lift_transposed<N, 5, decltype(dtag)::value, PE>(sX + slot0 * PE + le,
+      with_part<N, O>(rho, [&](auto dtag, auto, int slot0) {
+        lift_transposed<N, O, 5, decltype(dtag)::value, PE>(sX + slot0 * PE + le,
                                                          lops + slot0 * O::PC, rho, sF + le);
       });
       __syncthreads();
@@ -337,15 +337,15 @@ __global__ void __launch_bounds__(AdjTile<N, DG_EULER>::BLOCK)
     // {{{ volume: per direction, T_k at the nodes, then y += J(h_k)^T T_k
 #pragma unroll 1
     for (int k = 0; k < 3; ++k) {
-      with_part<N>(rho, [&](auto dtag, auto ptag, int slot0) {
-        constexpr int D = decltype(dtag)::value, P = decltype(ptag)::value;
+      with_part<N, O>(rho, [&](auto dtag, auto, int slot0) {
+        constexpr int D = decltype(dtag)::value, P = (D + 1) & ~1;
         double acc[5][D];
 #pragma unroll
         for (int m = 0; m < 5; ++m)
 #pragma unroll
           for (int i = 0; i < D; ++i) acc[m][i] = 0.0;
         const int sig = rho ^ (k + 1);
-        const double* row = ops + volume_offset<N>(rho);
+        const double* row = ops + O::F::volume(rho);
         for (int k2 = 0; k2 < k; ++k2) row += ((rho ^ (k2 + 1)) == 0 ? DA : DB) * P;
         if (N != 1 || rho == 0)  // order 1: transposed weak derivatives reach part A
           block_product<5, D, P, PE, XS>(sX + (sig == 0 ? 0 : DA + (sig - 1) * DB) * PE + le,

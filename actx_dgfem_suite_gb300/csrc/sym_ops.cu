@@ -88,12 +88,12 @@ bool range_basis(std::vector<double> x, int cols, int n, int rank, double* q) {
 // ADJ: the blocks of the transposed operators (sym::AdjOps); RED: derivatives
 // through coefficients of degree N - 1 (sym::Ops); `into_a`: which order-1 blocks
 // may be non-zero (those into part A, else those from it).
-template <int N, bool ADJ, bool RED = false>
+template <int N, bool ADJ, int RED>
 int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool into_a,
          unsigned char* out, int out_bytes) {
   using B = sym::Basis<N>;
   using F = sym::Ops<N, RED>;
-  using O = std::conditional_t<ADJ, sym::AdjOps<N>, F>;
+  using O = std::conditional_t<ADJ, sym::AdjOps<N, RED>, F>;
   constexpr int NP = B::NP, NFP = B::NFP, NFPT = B::NFPT;
   if (!out) return O::SIZE;
   if (out_bytes < O::SIZE) return -1;
@@ -264,24 +264,45 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
         for (int i = 0; i < dim(r); ++i)
           block[r][k - 1].push_back(full[(size_t)(slot0(r) + i) * NP + slot0(r ^ k) + j]);
   }
-  for (int r = 0; r < 4; ++r) {
-    const int d = dim(r), rows = r == 0 ? F::RA : F::RB;  // outputs of a block
-    std::vector<double> q((size_t)rows * d);
-    if constexpr (RED) {
-      std::vector<double> all;
-      for (int k = 0; k < 3; ++k) all.insert(all.end(), block[r][k].begin(), block[r][k].end());
-      if (!range_basis(all, (int)all.size() / d, d, rows, q.data())) return -1;
-      double* dst = ops + (r == 0 ? F::EXP : F::EXPB + (r - 1) * (F::RB * F::PB));
-      for (int j = 0; j < rows; ++j)
-        for (int i = 0; i < d; ++i) dst[j * (r == 0 ? F::PA : F::PB) + i] = q[j * d + i];
+  auto rank = [](int r) { return r == 0 ? F::RA : F::RB; };
+  std::vector<double> q[4];  // basis of the space of degree N - 1, per part
+  for (int r = 0; RED && r < 4; ++r) {
+    const int d = dim(r);
+    q[r].resize((size_t)rank(r) * d);
+    std::vector<double> all;  // columns of the blocks into r, or rows of those from r
+    for (int k = 0; k < 3; ++k) {
+      const int s = r ^ (k + 1), ds = dim(s);
+      if (RED == sym::RED_OUT)
+        all.insert(all.end(), block[r][k].begin(), block[r][k].end());
+      else
+        for (int i = 0; i < ds; ++i)
+          for (int j = 0; j < d; ++j) all.push_back(block[s][k][(size_t)j * ds + i]);
     }
-    const int pitch = r == 0 ? F::PRA : F::PRB;
-    double* dst = ops + (r == 0 ? 0 : F::VOL0 + (r - 1) * F::VOLB);
-    for (int k = 0; k < 3; ++k)
-      for (int j = 0; j < dim(r ^ (k + 1)); ++j, dst += pitch)
-        for (int i = 0; i < rows; ++i)
-          dst[i] = RED ? dot(&q[(size_t)i * d], &block[r][k][(size_t)j * d], d)
-                       : block[r][k][(size_t)j * d + i];
+    if (!range_basis(all, (int)all.size() / d, d, rank(r), q[r].data())) return -1;
+    double* dst = ops + F::extra(r);
+    for (int j = 0; j < rank(r); ++j)
+      for (int i = 0; i < d; ++i)
+        dst[RED == sym::RED_OUT ? j * (r == 0 ? F::PA : F::PB) + i
+                                : i * (r == 0 ? F::PRA : F::PRB) + j] = q[r][(size_t)j * d + i];
+  }
+  for (int r = 0; r < 4; ++r) {
+    double* dst = ops + F::volume(r);
+    for (int k = 0; k < 3; ++k) {
+      const int s = r ^ (k + 1), d = dim(r), ds = dim(s);
+      const std::vector<double>& b = block[r][k];
+      for (int j = 0; j < (s == 0 ? F::INA : F::INB); ++j, dst += r == 0 ? F::POA : F::POB)
+        for (int i = 0; i < (r == 0 ? F::OUTA : F::OUTB); ++i) {
+          if (RED == sym::RED_OUT) {
+            dst[i] = dot(&q[r][(size_t)i * d], &b[(size_t)j * d], d);
+          } else if (RED == sym::RED_IN) {
+            std::vector<double> row(ds);
+            for (int c = 0; c < ds; ++c) row[c] = b[(size_t)c * d + i];
+            dst[i] = dot(&q[s][(size_t)j * ds], row.data(), ds);
+          } else {
+            dst[i] = b[(size_t)j * d + i];
+          }
+        }
+    }
   }
   to_basis(face, NFPT,
            [&](int i, int fj) { return Pair(lift[(size_t)i * NFPT + fj]); });
@@ -307,29 +328,33 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
 
 }  // namespace
 
-int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
-                 bool strong, unsigned char* out, int out_bytes) {
-  switch (strong && order > 1 ? -order : order) {
-    case 1: return pack<1, false>(diff, lift, face_nodes, strong, out, out_bytes);
-    case 2: return pack<2, false>(diff, lift, face_nodes, false, out, out_bytes);
-    case 3: return pack<3, false>(diff, lift, face_nodes, false, out, out_bytes);
-    case 4: return pack<4, false>(diff, lift, face_nodes, false, out, out_bytes);
-    case -2: return pack<2, false, true>(diff, lift, face_nodes, true, out, out_bytes);
-    case -3: return pack<3, false, true>(diff, lift, face_nodes, true, out, out_bytes);
-    case -4: return pack<4, false, true>(diff, lift, face_nodes, true, out, out_bytes);
+// RED_OUT for strong and transposed weak derivatives, RED_IN for weak ones
+template <bool ADJ, bool INTO_A>
+static int pack_order(int order, bool reduce, const double* diff, const double* lift,
+                      const int32_t* face_nodes, unsigned char* out, int out_bytes) {
+  constexpr int RED = INTO_A ? sym::RED_OUT : sym::RED_IN;
+  switch (reduce ? -order : order) {
+    case 1:
+    case -1: return pack<1, ADJ, 0>(diff, lift, face_nodes, INTO_A, out, out_bytes);
+    case 2: return pack<2, ADJ, 0>(diff, lift, face_nodes, INTO_A, out, out_bytes);
+    case 3: return pack<3, ADJ, 0>(diff, lift, face_nodes, INTO_A, out, out_bytes);
+    case 4: return pack<4, ADJ, 0>(diff, lift, face_nodes, INTO_A, out, out_bytes);
+    case -2: return pack<2, ADJ, RED>(diff, lift, face_nodes, INTO_A, out, out_bytes);
+    case -3: return pack<3, ADJ, RED>(diff, lift, face_nodes, INTO_A, out, out_bytes);
+    case -4: return pack<4, ADJ, RED>(diff, lift, face_nodes, INTO_A, out, out_bytes);
     default: return -1;
   }
 }
 
+int pack_sym_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
+                 bool strong, bool reduce, unsigned char* out, int out_bytes) {
+  return (strong ? pack_order<false, true> : pack_order<false, false>)(
+      order, reduce, diff, lift, face_nodes, out, out_bytes);
+}
+
 int pack_sym_adj_ops(int order, const double* weak, const double* lift,
-                     const int32_t* face_nodes, unsigned char* out, int out_bytes) {
-  switch (order) {
-    case 1: return pack<1, true>(weak, lift, face_nodes, true, out, out_bytes);
-    case 2: return pack<2, true>(weak, lift, face_nodes, true, out, out_bytes);
-    case 3: return pack<3, true>(weak, lift, face_nodes, true, out, out_bytes);
-    case 4: return pack<4, true>(weak, lift, face_nodes, true, out, out_bytes);
-    default: return -1;
-  }
+                     const int32_t* face_nodes, bool reduce, unsigned char* out, int out_bytes) {
+  return pack_order<true, true>(order, reduce, weak, lift, face_nodes, out, out_bytes);
 }
 
 }  // namespace dg

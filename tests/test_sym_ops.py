@@ -16,13 +16,15 @@ from actx_dgfem_suite_gb300.refelem import reference_tet
 EPS = np.finfo(np.float64).eps
 
 
-def _pack(order, diff, lift, face_nodes, strong=None):
-    """The block of the forward (``strong`` given) or adjoint operators."""
+def _pack(order, diff, lift, face_nodes, strong=None, reduce=False):
+    """The block of the forward (``strong`` given) or adjoint operators; ``reduce``:
+    products through coefficients of one degree less."""
     lib = ctypes.CDLL(str(_lib.library_path()))
     if strong is None:
-        f, extra = lib._ZN2dg16pack_sym_adj_opsEiPKdS1_PKiPhi, []
+        f, extra = lib._ZN2dg16pack_sym_adj_opsEiPKdS1_PKibPhi, []
     else:
-        f, extra = lib._ZN2dg12pack_sym_opsEiPKdS1_PKibPhi, [ctypes.c_bool(strong)]
+        f, extra = lib._ZN2dg12pack_sym_opsEiPKdS1_PKibbPhi, [ctypes.c_bool(strong)]
+    extra.append(ctypes.c_bool(reduce))
     f.restype = ctypes.c_int
     diff, lift = np.ascontiguousarray(diff), np.ascontiguousarray(lift)
     fn = np.ascontiguousarray(face_nodes, dtype=np.int32)
@@ -36,7 +38,7 @@ def _pack(order, diff, lift, face_nodes, strong=None):
 class _Blocks:
     """The operator block of order N read back in the kernel's layout."""
 
-    def __init__(self, order, buf, adjoint=False, reduced=False):
+    def __init__(self, order, buf, adjoint=False, reduced=None):
         self.np_ = (order + 1) * (order + 2) * (order + 3) // 6
         self.nfp = (order + 1) * (order + 2) // 2
         npr, nsg = int(order % 2 == 0), int(order == 4)
@@ -49,20 +51,24 @@ class _Blocks:
         x = buf.view(np.float64) if buf.size % 8 == 0 else None
         pos = 0
         self.vol, self.lift = {}, {}
-        # derivatives through coefficients of one degree less: their number per part
-        rank = {2: (1, 1), 3: (4, 2), 4: (5, 5)}[order] if reduced else (dim[0], dim[1])
+        # the space of degree N - 1 in every part: the blocks' outputs ("out") or inputs
+        rank = {2: (1, 1), 3: (4, 2), 4: (5, 5)}.get(order, (0, 0))
         rank = [rank[0]] + 3 * [rank[1]]
+        nin, nout = (rank if reduced == "in" else dim), (rank if reduced == "out" else dim)
         for r in range(4):
             for k in range(1, 4):
-                n = dim[r ^ k] * even(rank[r])
-                self.vol[r, k] = x[pos:pos + n].reshape(-1, even(rank[r]))[:, :rank[r]].T
+                n = nin[r ^ k] * even(nout[r])
+                self.vol[r, k] = x[pos:pos + n].reshape(-1, even(nout[r]))[:, :nout[r]].T
                 pos += n
+        more = {}
         for r in range(4 if reduced else 0):
-            n = rank[r] * pitch[r]
-            expand = x[pos:pos + n].reshape(-1, pitch[r])[:, :dim[r]].T
+            rows, cols = (dim[r], rank[r]) if reduced == "in" else (rank[r], dim[r])
+            n = rows * even(cols)
+            more[r] = x[pos:pos + n].reshape(-1, even(cols))[:, :cols].T
             pos += n
-            for k in range(1, 4):
-                self.vol[r, k] = expand @ self.vol[r, k]
+        for r, k in self.vol if reduced else ():
+            self.vol[r, k] = (self.vol[r, k] @ more[r ^ k] if reduced == "in"
+                              else more[r] @ self.vol[r, k])
         if adjoint:                              # chunks of orbits, rows by node slot
             ch = self.nfp if order == 1 else (self.nfp + 1) // 2
             nch = -(-self.nfp // ch)
@@ -101,13 +107,14 @@ class _Blocks:
         return slice(self.slot0[r], self.slot0[r] + self.dim[r])
 
 
+@pytest.mark.parametrize("reduce", [False, True])
 @pytest.mark.parametrize("strong", [False, True])
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
-def test_blocks_reproduce_the_dense_operators(order, strong):
+def test_blocks_reproduce_the_dense_operators(order, strong, reduce):
     ref = reference_tet(order)
     diff = ref.diff if strong else ref.weak_diff
-    b = _Blocks(order, _pack(order, diff, ref.lift, ref.face_nodes, strong),
-                reduced=strong and order > 1)
+    b = _Blocks(order, _pack(order, diff, ref.lift, ref.face_nodes, strong, reduce),
+                reduced=("out" if strong else "in") if reduce and order > 1 else None)
     assert sorted(b.node_slot) == list(range(b.np_))
     assert list(b.slot_node[b.node_slot]) == list(range(b.np_))
     assert sorted(b.face_point) == list(range(4 * b.nfp))
@@ -142,30 +149,36 @@ def test_blocks_reproduce_the_dense_operators(order, strong):
     assert np.all(np.abs(y - f @ lift.T) <= 4 * b.nfp * EPS * scale)
 
 
+@pytest.mark.parametrize("reduce", [False, True])
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
-def test_adjoint_blocks_are_the_transposed_blocks(order):
+def test_adjoint_blocks_are_the_transposed_blocks(order, reduce):
     ref = reference_tet(order)
     args = (order, ref.weak_diff, ref.lift, ref.face_nodes)
     fwd = _Blocks(order, _pack(*args, strong=False))
-    adj = _Blocks(order, _pack(*args), adjoint=True)
+    adj = _Blocks(order, _pack(*args, reduce=reduce), adjoint=True,
+                  reduced="out" if reduce and order > 1 else None)
     assert np.array_equal(fwd.node_slot, adj.node_slot)
     assert np.array_equal(fwd.face_point, adj.face_point)
     for r in range(4):
         assert np.array_equal(adj.lift[r], fwd.lift[r].T)
         for k in (1, 2, 3):
-            # the same sums rounded once to FP64, in another order of summation
-            assert np.allclose(adj.vol[r, k], fwd.vol[r ^ k, k].T, rtol=0,
-                               atol=2 * EPS * np.abs(ref.weak_diff).max())
+            # the same sums rounded once to FP64, in another order of summation; reduced:
+            # products of at most 5 terms, basis rows of unit length times columns of at
+            # most 11 entries, each at most 1.5 times the largest derivative
+            atol = (2 + 48 * reduce) * EPS * np.abs(ref.weak_diff).max()
+            assert np.allclose(adj.vol[r, k], fwd.vol[r ^ k, k].T, rtol=0, atol=atol)
     bad = ref.weak_diff.copy()
     bad[0, 1, 0] += 1e-9
     assert _pack(order, bad, ref.lift, ref.face_nodes) is None
 
 
-@pytest.mark.parametrize("order", [1, 2, 3, 4])
-def test_strong_operators_that_keep_the_degree_are_refused(order):
-    """Weak derivatives have the symmetry, but reach all of degree N."""
+@pytest.mark.parametrize("order", [2, 3, 4])
+def test_operators_that_keep_the_degree_are_refused(order):
+    """Weak derivatives reach all of degree N, strong ones read it."""
     ref = reference_tet(order)
-    assert _pack(order, ref.weak_diff, ref.lift, ref.face_nodes, True) is None
+    for diff, strong in ((ref.weak_diff, True), (ref.diff, False)):
+        assert _pack(order, diff, ref.lift, ref.face_nodes, strong) is not None
+        assert _pack(order, diff, ref.lift, ref.face_nodes, strong, reduce=True) is None
 
 
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
