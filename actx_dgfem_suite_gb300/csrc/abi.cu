@@ -249,6 +249,14 @@ struct dg_plan {
   dg::LaunchShape mix_shape;
   int mix_grid = 0;
   int64_t mix_ntiles = 0;
+  // mixed precision, Maxwell: the tensor-core kernel (dg_mixed_mma.cuh) of variants 1
+  // and 3
+  bool mma = false;
+  void* d_mma_ops = nullptr;
+  uint32_t mma_ops_bytes = 0;
+  dg::LaunchShape mma_shape;
+  int mma_grid = 0;
+  int64_t mma_ntiles = 0;
   float4* d_nodes = nullptr;   // Euler: FP32 node records, filled before each RHS
   int nodes_grid = 0;
   // symmetry-adapted kernel (dg_sym.cuh, dg_sym2d.cuh): the main kernel of the
@@ -401,6 +409,8 @@ constexpr int kShapeModeBits[2] = {dg::MODE_B128, dg::MODE_B512};
 
 // The plan's variant runs dg_rhs_mixed_kernel.
 bool uses_mix(const dg_plan* p) { return p->mix && (p->variant | 2) == 2; }
+// The plan's variant runs dg_maxwell_mma_kernel.
+bool uses_mma(const dg_plan* p) { return p->mma && (p->variant | 2) == 3; }
 
 // Mode bits and grid of the main kernel under the plan's variant.
 int main_mode(const dg_plan* p, int base) {
@@ -419,6 +429,11 @@ int main_grid(const dg_plan* p) {
     if (p->variant & 2)
       return (int)(p->mix_ntiles < 0x7fffffff ? p->mix_ntiles : 0x7fffffff);
     return p->mix_grid;
+  }
+  if (uses_mma(p)) {
+    if (p->variant & 2)
+      return (int)(p->mma_ntiles < 0x7fffffff ? p->mma_ntiles : 0x7fffffff);
+    return p->mma_grid;
   }
   if (p->sym) {
     if (p->variant & 2)
@@ -983,6 +998,43 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     const int64_t nfull = (int64_t)nsm * 8;
     p->nodes_grid = (int)(nblocks < nfull ? nblocks : nfull);
   }
+  // Maxwell, mixed precision, orders 2 and 3: dg_maxwell_mma_kernel (dg_mixed_mma.cuh)
+  // for variants 1 and 3, same bits as dg_rhs_kernel's.  A warp takes 8 elements from
+  // state to result, which needs 16-29 us (RK stage 24-43) however few there are, and 16
+  // warps per SM.  Measured (RHS / RK stage, us, dg_rhs_kernel -> here): P2 at 68 elements
+  // per SM 14 / 18 -> 16 / 24, at 162 29 / 39 -> 29 / 45, at 230 38 / 53 -> 29 / 45, at 546
+  // 101 / 143 -> 69 / 110; P3 at 68 28 / 32 -> 30 / 43, at 162 60 / 69 -> 55 / 84, at 230
+  // 84 / 108 -> 56 / 91, at 546 200 / 237 -> 143 / 206.  Order 1 has too little and order
+  // 4 too large a product for a warp's registers.
+  constexpr int kMmaPerSm = 200;
+  if (kprec == 1 && equation == DG_MAXWELL && (N == 2 || N == 3) &&
+      p->nel >= (int64_t)kMmaPerSm * nsm) {
+    dg::LaunchShape x0, x1;
+    err = dg::mma_shape_maxwell(N, false, &x0);
+    if (err == cudaSuccess) err = dg::mma_shape_maxwell(N, true, &x1);
+    std::vector<unsigned char> xops(
+        dg::pack_mma_ops(N, diff, mesh->lift, mesh->face_nodes, nullptr, 0));
+    const int xbytes = dg::pack_mma_ops(N, diff, mesh->lift, mesh->face_nodes, xops.data(),
+                                        (int)xops.size());
+    if (err == cudaSuccess) err = cudaMalloc(&p->d_mma_ops, xops.size());
+    if (err == cudaSuccess)
+      err = cudaMemcpy(p->d_mma_ops, xops.data(), xops.size(), cudaMemcpyHostToDevice);
+    if (err != cudaSuccess) {
+      dg_plan_destroy(p);
+      return cuda_fail(err, "tensor-core Maxwell kernel configuration");
+    }
+    if (x1.blocks_per_sm < x0.blocks_per_sm) x0.blocks_per_sm = x1.blocks_per_sm;
+    if (xbytes != x0.ops_bytes || x0.blocks_per_sm < 1) {
+      dg_plan_destroy(p);
+      return fail(DG_ERR_CUDA, "tensor-core Maxwell kernel: layout mismatch or does not fit");
+    }
+    p->mma = true;
+    p->mma_ops_bytes = static_cast<uint32_t>(xbytes);
+    p->mma_shape = x0;
+    p->mma_ntiles = (p->nel + x0.elems_per_tile - 1) / x0.elems_per_tile;
+    const int64_t xfull = (int64_t)nsm * x0.blocks_per_sm;
+    p->mma_grid = (int)(p->mma_ntiles < xfull ? p->mma_ntiles : xfull);
+  }
   p->face_partner = mesh->face_partner;
 
   if (kprec == 1 && equation == DG_EULER) {
@@ -1451,6 +1503,11 @@ cudaError_t launch_main(const dg_plan* p, dg::RhsArgs a, bool stage, cudaStream_
                ? dg::mixed_launch_wave(p->order, stage, a, main_grid(p), s)
                : dg::mixed_launch_euler(p->order, stage, a, main_grid(p), s);
   }
+  if (uses_mma(p)) {
+    a.ops = p->d_mma_ops;
+    a.ops_bytes = p->mma_ops_bytes;
+    return dg::mma_launch_maxwell(p->order, stage, a, main_grid(p), s);
+  }
   if (p->sym) {
     a.ops = p->d_sym_ops;
     a.ops_bytes = p->sym_ops_bytes;
@@ -1860,7 +1917,7 @@ int dg_plan_destroy(dg_plan* p) {
                   (void*)p->d_tc_ops, p->d_tcm_ops[0], p->d_tcm_ops[1],
                   p->d_tcm_ops[2] != p->d_tcm_ops[1] ? p->d_tcm_ops[2] : nullptr,
                   (void*)p->d_pres, p->d_sym_ops, p->d_adj_sym_ops,
-                  p->d_mix_ops, (void*)p->d_nodes})
+                  p->d_mix_ops, (void*)p->d_nodes, p->d_mma_ops})
     if (b && cudaFree(b) != cudaSuccess) code = DG_ERR_CUDA;
   delete p;
   if (code != DG_OK) return fail(code, "cudaFree failed");
@@ -1964,12 +2021,14 @@ int dg_plan_info(const dg_plan* p, int64_t* nelements, int32_t* order,
                    : (m4 ? p->tcm_shape[k].threads
                          : (mb ? p->tcb_shape[kb].threads
                                : (uses_mix(p) ? p->mix_shape.threads
+                                : uses_mma(p) ? p->mma_shape.threads
                                               : (p->sym ? p->sym_shape.threads : dg::kBlock))));
   if (smem_bytes)
     *smem_bytes = p->tc ? p->tc_shape.smem_bytes
                         : (m4 ? p->tcm_shape[k].smem_bytes
                               : (mb ? p->tcb_shape[kb].smem_bytes
                                     : (uses_mix(p) ? p->mix_shape.smem_bytes
+                                     : uses_mma(p) ? p->mma_shape.smem_bytes
                                                    : (p->sym ? p->sym_shape.smem_bytes
                                                              : p->shape.smem_bytes))));
   return DG_OK;

@@ -129,6 +129,14 @@ cudaError_t mixed_nodes_euler(const double* q, float4* rec, int64_t nelnp, doubl
 int pack_mixed_ops(int order, const double* diff, const double* lift,
                    const int32_t* face_nodes, unsigned char* out, int out_bytes);
 
+// Mixed precision on the tensor cores, Maxwell at orders 2 and 3
+// (dg_mixed_mma.cuh), and its operator block (mma::Ops; conventions as above).
+cudaError_t mma_shape_maxwell(int order, bool stage, LaunchShape* out);
+cudaError_t mma_launch_maxwell(int order, bool stage, const RhsArgs& a, int grid,
+                               cudaStream_t s);
+int pack_mma_ops(int order, const double* diff, const double* lift, const int32_t* face_nodes,
+                 unsigned char* out, int out_bytes);
+
 // Triangle meshes (rhs_2d.cu): shape query and launch of dg_rhs2d_kernel
 // for mode MODE_RHS or MODE_STAGE (FP64), and the operator block
 // [Wt (2 Np Np) | Lt (3 Nfp Np) | int32 edge nodes (3 Nfp)] packed from the

@@ -1,6 +1,6 @@
-"""The CUDA-core mixed-precision kernels of wave and Euler at element counts
-around their 32-element tile: within the mixed path's bound of the FP64 result,
-and the same on both grids."""
+"""The mixed-precision kernels of wave and Euler (CUDA cores) and Maxwell (tensor
+cores) at element counts around their tiles: within the mixed path's bound of the
+FP64 result, and the same on both grids (Maxwell: as the general kernel's too)."""
 
 from __future__ import annotations
 
@@ -49,4 +49,40 @@ def test_mixed_tile_edges(equation, order, extra):
         got[prec, variant] = (r, res, qo, un)
     for ref, a, b in zip(*got.values()):
         assert torch.equal(a, b)
+        assert float(torch.linalg.norm(a - ref)) <= MIXED_RTOL * float(torch.linalg.norm(ref))
+
+
+@pytest.mark.parametrize("order", [2, 3])
+@pytest.mark.parametrize("extra", [0, 1, 9])
+def test_maxwell_warp_tile_edges(order, extra):
+    """Warps of 8 elements: variants 1 and 3 from 200 elements per SM on."""
+    from actx_dgfem_suite_gb300.mesh import TetMesh
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    nel = 200 * nsm + extra
+    n = 2
+    while 6 * n**3 < nel:
+        n += 1
+    mesh = jittered_box_mesh(n)
+    mesh = TetMesh(vertices=mesh.vertices, elements=mesh.elements[:nel])
+    prob = make_problem("maxwell", mesh, order, seed=extra)
+    dm = DeviceMesh(prob.disc, "cuda:0")
+    q = torch.from_numpy(prob.fields).cuda()
+    scale = torch.linspace(0.8, 1.2, nel, dtype=torch.float64, device="cuda")
+    got = {}
+    for prec, variant in (("fp64", 0), ("fp32-mixed", 7), ("fp32-mixed", 1), ("fp32-mixed", 3)):
+        plan = DevicePlan(dm, "maxwell", (0.8, 1.3, 0.7), prec)
+        plan.set_variant(variant)
+        if variant in (1, 3):
+            assert plan.info()["block"] == 512
+        r = plan.rhs(q)
+        plan.set_element_scale(scale)
+        res, qo, un = 0.5 * q, torch.empty_like(q), torch.empty_like(q)
+        plan.rk_stage(q, qo, res, 0.3, 0.7, 1e-2, rhs_unscaled=un)
+        first = torch.full_like(q, float("nan"))   # a = 0 does not read it
+        plan.rk_stage(q, qo, first, 0.0, 0.7, 1e-2)
+        plan.finish()
+        got[prec, variant] = (r, res, qo, un, first)
+    for ref, a, b, c in zip(*got.values()):
+        assert torch.equal(a, b) and torch.equal(a, c)
         assert float(torch.linalg.norm(a - ref)) <= MIXED_RTOL * float(torch.linalg.norm(ref))
