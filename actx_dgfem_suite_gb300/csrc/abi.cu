@@ -1003,12 +1003,14 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
   // state to result, which needs 16-29 us (RK stage 24-43) however few there are, and 16
   // warps per SM.  Measured (RHS / RK stage, us, dg_rhs_kernel -> here): P2 at 68 elements
   // per SM 14 / 18 -> 16 / 24, at 162 29 / 39 -> 29 / 45, at 230 38 / 53 -> 29 / 45, at 546
-  // 101 / 143 -> 69 / 110; P3 at 68 28 / 32 -> 30 / 43, at 162 60 / 69 -> 55 / 84, at 230
-  // 84 / 108 -> 56 / 91, at 546 200 / 237 -> 143 / 206.  Order 1 has too little and order
-  // 4 too large a product for a warp's registers.
-  constexpr int kMmaPerSm = 200;
+  // 101 / 143 -> 69 / 110; P3 at 68 28 / 32 -> 30 / 43, at 162 60 / 69 -> 55 / 84, at 316
+  // 119 / 141 -> 89 / 130, at 546 200 / 237 -> 143 / 206.  The lines lie where dg_rhs_kernel's
+  // tensor-core variants are faster than its FP32 ones (P2 at 316 48 / 46, at 546 88 / 99;
+  // P3 at 230 84 / 72, at 316 119 / 124), so that autotuning keeps to the arithmetic it
+  // chose.  Order 1 has too little and order 4 too large a product for a warp's registers.
+  const int mma_per_sm = N == 2 ? 450 : 300;
   if (kprec == 1 && equation == DG_MAXWELL && (N == 2 || N == 3) &&
-      p->nel >= (int64_t)kMmaPerSm * nsm) {
+      p->nel >= (int64_t)mma_per_sm * nsm) {
     dg::LaunchShape x0, x1;
     err = dg::mma_shape_maxwell(N, false, &x0);
     if (err == cudaSuccess) err = dg::mma_shape_maxwell(N, true, &x1);

@@ -266,10 +266,10 @@ __device__ __forceinline__ float dot4(const float4 w, const float4 x, float acc)
 }
 
 // double -> arithmetic type; the mixed path converts on the integer ALU
-template <typename Real>
+template <typename Real, int N, int EQ>
 __device__ __forceinline__ Real to_real(double v) {
   if constexpr (std::is_same<Real, double>::value) return v;
-  else return d2f_alu(v);
+  else return state_to_float<N, EQ>(v);
 }
 
 template <int N, int EQ, typename Real, int MODE>
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
           sQ[k * (E * NP) + rem] = v;
           if constexpr (T::MIXED) {
             const int le = rem / NP;
-            sQr[(k * E + le) * ROW + (rem - le * NP)] = to_real<Real>(v);
+            sQr[(k * E + le) * ROW + (rem - le * NP)] = to_real<Real, N, EQ>(v);
           }
         }
       }
@@ -357,11 +357,11 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
     {
       const double* mt = a.metric + e0 * 9;
       for (int idx = t; idx < 9 * E; idx += BLOCK)
-        sG[idx] = idx < 9 * ecount ? to_real<Real>(__ldg(mt + idx)) : zero;
+        sG[idx] = idx < 9 * ecount ? to_real<Real, N, EQ>(__ldg(mt + idx)) : zero;
       if constexpr (!SPLIT) {  // face geometry: the fused path's fluxes only
         const double* ft = a.face_geom + e0 * 16;
         for (int idx = t; idx < 16 * E; idx += BLOCK)
-          sFG[idx] = idx < 16 * ecount ? to_real<Real>(__ldg(ft + idx)) : zero;
+          sFG[idx] = idx < 16 * ecount ? to_real<Real, N, EQ>(__ldg(ft + idx)) : zero;
       }
     }
     // face values of the tile, contiguous per field (split Euler: after the
@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
 #pragma unroll
         for (int k = 0; k < NF; ++k, qk += nelnp) {
           qed[k] = __ldg(qk);
-          qe[k] = to_real<Real>(qed[k]);
+          qe[k] = to_real<Real, N, EQ>(qed[k]);
         }
       }
       Real* out = sFlux + elp * FROW + fj;
@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
         }
         if constexpr (EQ == DG_MAXWELL) acc = acc * (k < 3 ? inv_eps : inv_mu);
         double val;
-        if constexpr (T::MIXED) val = f2d_alu(acc);
+        if constexpr (T::MIXED) val = float_to_result<N, EQ>(acc);
         else val = acc;
         if constexpr (STAGE)
           if (a.rhs_unscaled) a.rhs_unscaled[gidx] = val;

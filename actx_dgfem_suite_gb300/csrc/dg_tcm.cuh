@@ -332,7 +332,7 @@ __device__ __forceinline__ float levels4(const uint32_t* l, int jj) {
 // Numerical flux of one face point in FP32 (FP64 exterior state; Euler:
 // interior and exterior pressures from the per-node table); out[c] = the
 // lifted face value of field c.
-template <int EQ, int NF>
+template <int N, int EQ, int NF>
 __device__ __forceinline__ void face_point_flux(const FluxConsts& fc, const float* qi,
                                                 const double* qed, bool bdry, float nx,
                                                 float ny, float nz, float scale,
@@ -340,7 +340,7 @@ __device__ __forceinline__ void face_point_flux(const FluxConsts& fc, const floa
   float qe[NF];
   if (!bdry) {
 #pragma unroll
-    for (int k = 0; k < NF; ++k) qe[k] = d2f_alu(qed[k]);
+    for (int k = 0; k < NF; ++k) qe[k] = state_to_float<N, EQ>(qed[k]);
   }
   if constexpr (EQ == DG_WAVE) {
     if (bdry) {  // Dirichlet mirror: exterior (-u, v)
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(tcm::MPlan<N, EQ, TF, ALT>::THREADS,
                             : (valid ? __ldg(a.q + k * nelnp + gnode) : (k == 0 ? 1.0 : 0.0));
           else
             qd = valid ? __ldg(a.q + k * nelnp + gnode) : (k == 0 ? 1.0 : 0.0);
-          qf[k] = d2f_alu(qd);
+          qf[k] = state_to_float<N, EQ>(qd);
           if (item) sq[(k * E + e) * QP + j] = qf[k];
         }
         if constexpr (EQ == DG_EULER) {  // pressure table: FP64 recovery once per node
@@ -802,7 +802,7 @@ __global__ void __launch_bounds__(tcm::MPlan<N, EQ, TF, ALT>::THREADS,
             pi = sP[e * NP + node];
             pe = bdry ? pi : __ldg(a.pres + gi);
           }
-          tcm::face_point_flux<EQ, NF>(fc, qi, qed, bdry, nx, ny, nz, scale, pi, pe,
+          tcm::face_point_flux<N, EQ, NF>(fc, qi, qed, bdry, nx, ny, nz, scale, pi, pe,
                                        fv[rd][h]);
         }
         fm[rd] = e | (fj0 << 8);
@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(tcm::MPlan<N, EQ, TF, ALT>::THREADS,
       const double es = a.elem_scale ? __ldg(a.elem_scale + e0 + e) : 1.0;
 #pragma unroll
       for (int k = 0; k < NF; ++k, gidx += nelnp) {
-        double val = f2d_alu(sOut[(k * E + e) * OP + i]);
+        double val = float_to_result<N, EQ>(sOut[(k * E + e) * OP + i]);
         if constexpr (STAGE)
           if (a.rhs_unscaled) a.rhs_unscaled[gidx] = val;
         if (a.elem_scale) val *= es;

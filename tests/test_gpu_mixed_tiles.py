@@ -55,11 +55,11 @@ def test_mixed_tile_edges(equation, order, extra):
 @pytest.mark.parametrize("order", [2, 3])
 @pytest.mark.parametrize("extra", [0, 1, 9])
 def test_maxwell_warp_tile_edges(order, extra):
-    """Warps of 8 elements: variants 1 and 3 from 200 elements per SM on."""
+    """Warps of 8 elements: variants 1 and 3 from 450 or 300 elements per SM on."""
     from actx_dgfem_suite_gb300.mesh import TetMesh
     from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
     nsm = torch.cuda.get_device_properties(0).multi_processor_count
-    nel = 200 * nsm + extra
+    nel = {2: 450, 3: 300}[order] * nsm + extra
     n = 2
     while 6 * n**3 < nel:
         n += 1
