@@ -1001,7 +1001,7 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
   // Maxwell, mixed precision, orders 2 and 3: dg_maxwell_mma_kernel (dg_mixed_mma.cuh)
   // for variants 1 and 3, same bits as dg_rhs_kernel's.  A warp takes 8 elements from
   // state to result, which needs 16-29 us (RK stage 24-43) however few there are, and 16
-  // warps per SM.  Measured (RHS / RK stage, us, dg_rhs_kernel -> here): P2 at 68 elements
+  // or 12 run per SM.  Measured (RHS / RK stage, us, dg_rhs_kernel -> here): P2 at 68 elements
   // per SM 14 / 18 -> 16 / 24, at 162 29 / 39 -> 29 / 45, at 230 38 / 53 -> 29 / 45, at 546
   // 101 / 143 -> 69 / 110; P3 at 68 28 / 32 -> 30 / 43, at 162 60 / 69 -> 55 / 84, at 316
   // 119 / 141 -> 89 / 130, at 546 200 / 237 -> 143 / 206.  The lines lie where dg_rhs_kernel's

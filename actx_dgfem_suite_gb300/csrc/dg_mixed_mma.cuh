@@ -15,12 +15,11 @@
 //   - a thread's gathered traces are loaded for two face points at a time, the
 //     indices of the next two meanwhile.
 // Measured (GB300, whole RHS, the fastest variant of dg_rhs_kernel -> here): P2 at
-// 511,104 tets 557 -> 371 us, P3 at 279,936 tets 651 -> 419 us; RK stage P3 at 82,944
-// tets 237 -> 206 us (the stage's FP64 operations, 180 FP64-pipe cycles per element,
-// come on top).  ncu (P3, 82,944 tets): issue slots 49 % busy while the SMs are, tensor
-// pipe 26 %, 7.9 cycles per issued instruction of a warp (waits for fixed latencies 1.9,
-// loads 1.4, shared memory 1.0) with four warps per scheduler, all that registers and
-// shared memory allow.
+// 511,104 tets 557 -> 371 us, P3 at 279,936 tets 651 -> 407 us; RK stage P3 at 82,944
+// tets 237 -> 188 us (the stage's FP64 operations, 180 FP64-pipe cycles per element,
+// come on top).  ncu (P3, 82,944 tets, 16 warps): issue slots 49 % busy while the SMs
+// are, tensor pipe 26 %, 7.9 cycles per issued instruction of a warp (waits for fixed
+// latencies 1.9, loads 1.4, shared memory 1.0, math pipes 0.8).
 // The m16n8k8 products run over the same columns k in the same order as there, and
 // the flux in the same operations, so results are bit for bit the same.
 #pragma once
@@ -46,11 +45,13 @@ struct Ops {
 };
 
 // Shared memory: operators, then per warp the state and the face values in FP32
-// ([field][node][8 elements]), metric and face geometry.  One CTA of 16 warps per SM.
+// ([field][node][8 elements]), metric and face geometry.  One CTA per SM: 16 warps of
+// 128 registers at order 2; at order 3, whose products need more, 12 of 168 (279,936
+// tets: RHS 419 -> 407 us, RK stage 609 -> 558; at order 2 12 warps took 462 us, 16 371).
 template <int N>
 struct Tile {
   static constexpr int NP = Shape<N>::NP, NFPT = Shape<N>::NFPT;
-  static constexpr int E = 8, WARPS = 16, BLOCK = 32 * WARPS;
+  static constexpr int E = 8, WARPS = N == 3 ? 12 : 16, BLOCK = 32 * WARPS;
   static constexpr int X = 0, F = X + 6 * NP * E, G = F + 6 * NFPT * E, FG = G + 9 * E;
   static constexpr int WORDS = FG + 16 * E;                 // of a warp
   static constexpr int SMEM = Ops<N>::SIZE + WARPS * WORDS * 4;

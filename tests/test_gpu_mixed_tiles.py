@@ -74,7 +74,7 @@ def test_maxwell_warp_tile_edges(order, extra):
         plan = DevicePlan(dm, "maxwell", (0.8, 1.3, 0.7), prec)
         plan.set_variant(variant)
         if variant in (1, 3):
-            assert plan.info()["block"] == 512
+            assert plan.info()["block"] == {2: 512, 3: 384}[order]
         r = plan.rhs(q)
         plan.set_element_scale(scale)
         res, qo, un = 0.5 * q, torch.empty_like(q), torch.empty_like(q)
