@@ -294,6 +294,8 @@ dg::RhsArgs base_args(const dg_plan* p) {
   a.p1 = p->params[1];
   a.p2 = p->params[2];
   for (int k = 0; k < 6; ++k) a.k[k] = p->k[k];
+  a.c32[0] = (float)a.p0;
+  for (int k = 0; k < 6; ++k) a.c32[k + 1] = (float)a.k[k];
   a.elem_scale = p->elem_scale;
   a.flux_in = p->split ? p->d_flux : nullptr;
   a.aux = p->split ? p->d_aux : nullptr;

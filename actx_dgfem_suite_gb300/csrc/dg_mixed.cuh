@@ -121,7 +121,7 @@ __device__ __forceinline__ void face_flux(const RhsArgs& a, const float* qi, flo
       qe[2] = qi[2];
       qe[3] = qi[3];
     }
-    const float c = (float)a.p0;
+    const float c = a.c32[0];
     const float vavg_n = dot3(0.5f * (qi[1] + qe[1]), 0.5f * (qi[2] + qe[2]),
                               0.5f * (qi[3] + qe[3]), nx, ny, nz);
     const float uavg = 0.5f * (qi[0] + qe[0]);
@@ -140,7 +140,7 @@ __device__ __forceinline__ void face_flux(const RhsArgs& a, const float* qi, flo
       qe[2] = fmaf(-2.0f * nx, mn, qi[2]);
       qe[3] = fmaf(-2.0f * ny, mn, qi[3]);
       qe[4] = fmaf(-2.0f * nz, mn, qi[4]);
-      se = euler_trace(qe, si.p, (float)a.p0);
+      se = euler_trace(qe, si.p, a.c32[0]);
     }
     const float uni = dot3(qi[2] * si.rinv, qi[3] * si.rinv, qi[4] * si.rinv, nx, ny, nz);
     const float une = dot3(qe[2] * se.rinv, qe[3] * se.rinv, qe[4] * se.rinv, nx, ny, nz);
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(Tile<N, EQ>::BLOCK, Tile<N, EQ>::MIN_CTAS)
 
   const int64_t nel = a.nel, nelnp = nel * NP;
   const int64_t ntiles = (nel + E - 1) / E;
-  const float p0 = (float)a.p0;
+  const float p0 = a.c32[0];
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t e0 = tile * E;
     const int ecount = (nel - e0) < (int64_t)E ? (int)(nel - e0) : E;

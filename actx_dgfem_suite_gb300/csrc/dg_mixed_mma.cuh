@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(Tile<N>::BLOCK) dg_maxwell_mma_kernel(const Rh
 
     // {{{ face gather + numerical flux: 8 NFPT points, consecutive ones of an element
     // on consecutive lanes (a face's traces share memory sectors)
-    const float alpha = (float)a.p0, z = (float)a.k[0], y = (float)a.k[1];
-    const float ce = (float)a.k[2], ch = (float)a.k[3];
+    const float alpha = a.c32[0], z = a.c32[1], y = a.c32[2];
+    const float ce = a.c32[3], ch = a.c32[4];
     constexpr int PPT = 2;  // points whose loads are in flight together
     static_assert(E * NFPT % (32 * PPT) == 0, "whole rounds of face points");
     const uint32_t* gt = a.gather + e0 * NFPT + lane;
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(Tile<N>::BLOCK) dg_maxwell_mma_kernel(const Rh
 
     // {{{ LIFT; the sums go over the state's arrays, so that the loads and stores of
     // the epilogue are coalesced and independent
-    const float inv_eps = (float)a.k[4], inv_mu = (float)a.k[5];
+    const float inv_eps = a.c32[5], inv_mu = a.c32[6];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       float acc[O::LM][3][4];

@@ -81,6 +81,8 @@ struct RhsArgs {
   const double* aux;       // MODE_SPLIT euler: (3, Nel, Np) p, 1/rho, |u| + c
   const float* pres;       // mixed-precision euler: (Nel, Np) pressure, recovered
                            // from total energy in FP64 once per node, as FP32
+  float c32[7];            // p0, k[0..5] in FP32 (converted in the kernel they took 11 %
+                           // of the FP64 pipe: Maxwell P3, 279,936 tets 678 -> 654 us)
   const float4* nodes;     // dg_rhs_mixed_kernel: FP32 node records (dg_mixed.cuh)
 };
 
@@ -272,8 +274,30 @@ __device__ __forceinline__ Real to_real(double v) {
   else return state_to_float<N, EQ>(v);
 }
 
+// Constant n of RhsArgs (p0, k[0..5]) in the arithmetic type; order-4 Maxwell: see
+// d2f_alu_fields.
+template <int N, int EQ, typename Real>
+__device__ __forceinline__ Real constant(const RhsArgs& a, int n) {
+  if constexpr (std::is_same<Real, double>::value || (N == 4 && EQ == DG_MAXWELL))
+    return (Real)(n == 0 ? a.p0 : a.k[n == 0 ? 0 : n - 1]);
+  else
+    return a.c32[n];
+}
+
+// Order-3 Maxwell on the CUDA cores waits for its gathers (long scoreboard 4.0 of 10
+// cycles per issued instruction, 38 % of the issue slots used) with the two CTAs per SM
+// that 107 registers allow; three at 80 registers (48 bytes spilled): 279,936 tets
+// 654 -> 544 us, RK stage 895 -> 692 us.  Other orders and equations: not limited by it, or
+// faster variants exist.
 template <int N, int EQ, typename Real, int MODE>
-__global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a) {
+constexpr int min_ctas() {
+  return N == 3 && EQ == DG_MAXWELL && !std::is_same<Real, double>::value && !(MODE & MODE_TC)
+             ? 3 : 0;
+}
+
+template <int N, int EQ, typename Real, int MODE>
+__global__ void __launch_bounds__(block_of(MODE), (min_ctas<N, EQ, Real, MODE>()))
+    dg_rhs_kernel(const RhsArgs a) {
   constexpr int BLOCK = block_of(MODE);
   using T = Tile<N, EQ, Real, (MODE & MODE_SPLIT) != 0, BLOCK>;
   using Ops = OpsLayout<N, Real>;
@@ -330,9 +354,9 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
   const int64_t nel = a.nel;
   const int64_t nelnp = nel * NP;
   const int64_t ntiles = (nel + E - 1) / E;
-  const Real p0 = (Real)a.p0;
+  const Real p0 = constant<N, EQ, Real>(a, 0);
   const Real half = (Real)0.5, two = (Real)2, zero = (Real)0;
-  const Real inv_eps = (Real)a.k[4], inv_mu = (Real)a.k[5];
+  const Real inv_eps = constant<N, EQ, Real>(a, 5), inv_mu = constant<N, EQ, Real>(a, 6);
 
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int64_t e0 = tile * E;
@@ -758,7 +782,7 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
           qe[5] = qi[5];
         }
         const Real alpha = p0;
-        const Real z = (Real)a.k[0], y = (Real)a.k[1];
+        const Real z = constant<N, EQ, Real>(a, 1), y = constant<N, EQ, Real>(a, 2);
         const Real je[3] = {qe[0] - qi[0], qe[1] - qi[1], qe[2] - qi[2]};
         const Real jh[3] = {qe[3] - qi[3], qe[4] - qi[4], qe[5] - qi[5]};
         const Real n[3] = {nx, ny, nz};
@@ -777,7 +801,7 @@ __global__ void __launch_bounds__(block_of(MODE)) dg_rhs_kernel(const RhsArgs a)
         }
         cross(n, te, fe);
         cross(n, th, fh);
-        const Real ce = (Real)a.k[2], ch = (Real)a.k[3];
+        const Real ce = constant<N, EQ, Real>(a, 3), ch = constant<N, EQ, Real>(a, 4);
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
           out[x * FS] = -scale * (ce * fe[x]);
