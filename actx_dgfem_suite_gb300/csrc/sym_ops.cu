@@ -51,7 +51,12 @@ double dot(const double* a, const double* b, int n) {  // rounded once
 // Gram-Schmidt with the largest remaining column next, each orthogonalised twice.
 // False unless the columns have that rank to rounding.
 bool range_basis(std::vector<double> x, int cols, int n, int rank, double* q) {
-  auto norm = [&](int c) { return std::sqrt(dot(&x[c * n], &x[c * n], n)); };
+  auto inner = [n](const double* a, const double* b) {
+    double s = 0.0;
+    for (int k = 0; k < n; ++k) s = std::fma(a[k], b[k], s);
+    return s;
+  };
+  auto norm = [&](int c) { return std::sqrt(inner(&x[c * n], &x[c * n])); };
   double big = 0.0;
   for (int c = 0; c < cols; ++c) big = std::fmax(big, norm(c));
   for (int r = 0; r <= rank; ++r) {
@@ -70,15 +75,15 @@ bool range_basis(std::vector<double> x, int cols, int n, int rank, double* q) {
     std::memcpy(v, &x[best * n], n * sizeof(double));
     for (int pass = 0; pass < 2; ++pass) {
       for (int p = 0; p < r; ++p) {
-        const double h = dot(q + p * n, v, n);
+        const double h = inner(q + p * n, v);
         for (int k = 0; k < n; ++k) v[k] = std::fma(-h, q[p * n + k], v[k]);
       }
-      const double l = std::sqrt(dot(v, v, n));
+      const double l = std::sqrt(inner(v, v));
       for (int k = 0; k < n; ++k) v[k] /= l;
     }
     for (int c = 0; c < cols; ++c)
       for (int pass = 0; pass < 2; ++pass) {
-        const double h = dot(v, &x[c * n], n);
+        const double h = inner(v, &x[c * n]);
         for (int k = 0; k < n; ++k) x[c * n + k] = std::fma(-h, v[k], x[c * n + k]);
       }
   }
@@ -295,9 +300,9 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
           if (RED == sym::RED_OUT) {
             dst[i] = dot(&q[r][(size_t)i * d], &b[(size_t)j * d], d);
           } else if (RED == sym::RED_IN) {
-            std::vector<double> row(ds);
+            double row[B::DA];
             for (int c = 0; c < ds; ++c) row[c] = b[(size_t)c * d + i];
-            dst[i] = dot(&q[s][(size_t)j * ds], row.data(), ds);
+            dst[i] = dot(&q[s][(size_t)j * ds], row, ds);
           } else {
             dst[i] = b[(size_t)j * d + i];
           }
