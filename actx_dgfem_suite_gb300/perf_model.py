@@ -130,18 +130,23 @@ def bytes_per_element(equation: str, order: int, dim: int = 3) -> int:
             + 4 * 4 * nfp_of(order))
 
 
+#: FP64 multiply-adds per field of the symmetry-adapted blocks (``csrc/dg_sym.cuh``):
+#: one derivative, one through degree N - 1 (order 1: its one non-zero block), LIFT
+_SYM_FMA = {1: (1, 1, 12), 2: (24, 10, 60), 3: (100, 50, 200), 4: (304, 175, 525)}
+
+
 def fp64_fma_per_element(equation: str, order: int) -> int:
-    """FP64 fused multiply-adds the CUDA kernel issues per element in its
-    contractions (the reference derivatives of a field are shared by its
-    gradient components; see ``csrc/dg_rhs_fp64.cuh``)."""
-    n, nf = np_of(order), 4 * nfp_of(order)
-    lift = NFIELDS[equation] * n * nf
+    """FP64 fused multiply-adds that the face-shared path's volume/LIFT kernel issues
+    per element in its contractions (``csrc/dg_sym.cuh``); plans on other kernels
+    issue more (the dense products: up to 4 times as many)."""
+    diff, low, lift = _SYM_FMA[order]
+    extra = low if order > 1 else 0      # nodes <-> coefficients of degree N - 1
     if equation == "wave":
-        return 6 * n * n + lift          # 3 D_r u + sum_r D_r (G v)_r
+        return 6 * low + 4 * extra + 4 * lift    # 3 for u, 3 for G v
     if equation == "euler":
-        return 15 * n * n + lift         # 5 fields x sum_r D_r (G F)_r
+        return 15 * diff + 5 * lift              # 5 fluxes along 3 directions
     if equation == "maxwell":
-        return 18 * n * n + lift         # 6 fields x 3 D_r
+        return 18 * low + 6 * extra + 6 * lift   # 6 curl components x 3 directions
     raise ValueError(equation)
 
 

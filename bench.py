@@ -700,8 +700,9 @@ def our_arm(args) -> None:
         kname = f"dg_rhs_tc_kernel<{rd['order']}, {rd['eq']}, SPLIT>"
     else:
         kname = (f"dg_rhs_kernel<{rd['order']}, {rd['eq']}, "
-                 f"{'float' if args.precision == 'fp32-mixed' else 'double'}, "
-                 f"{'SPLIT' if info['face_shared'] else 'RHS'}>")
+                 f"{'float' if args.precision == 'fp32-mixed' else 'double'}, RHS>")
+    if info["face_shared"] and not info["tensor_cores"]:
+        kname = f"dg_rhs_sym_kernel<{rd['order']}, {rd['eq']}>"
     if info["face_shared"]:
         kname = (f"dg_face_flux_kernel<{rd['order']}, {rd['eq']}>"
                  + (" + dg_euler_aux_kernel" if rd["eq"] == "euler" else "")

@@ -88,8 +88,15 @@ typedef struct dg_mesh_desc {
  * pair whole faces consistently with gather, which plan creation checks
  * (DG_ERR_ARGUMENT otherwise).  Such a plan keeps face values in its own
  * device buffers, so its dg_rhs / dg_rk_stage calls must not run
- * concurrently with each other (issue them on one stream).  All other plans
- * evaluate the RHS in one fused launch and have no such restriction.
+ * concurrently with each other (issue them on one stream).  DG_FP32_MIXED
+ * Euler plans fill a per-node FP32 table (pressure, or whole node records of
+ * 32 bytes) before each call and have the same restriction.  All other plans
+ * evaluate the RHS in one fused launch and have none.
+ *
+ * Which kernels a plan takes depends on its operators and size only: where
+ * diff and lift have the reference tetrahedron's four-group symmetry to
+ * rounding, FP64 volume, LIFT and adjoint products run in the symmetry-adapted
+ * basis (a quarter of the multiply-adds) on all but small meshes.
  *
  * Replaces the compile step of the reference's array contexts:
  * actx.compile(rhs) (actx_dgfem_suite/run/__main__.py:74) and the DAG/loopy
@@ -121,7 +128,7 @@ typedef struct dg_mesh2d_desc {
 } dg_mesh2d_desc;
 
 /* Build a plan for a triangle mesh: FP64 arithmetic, one fused persistent
- * launch per RHS (dg_rhs2d_kernel).  params as for dg_plan_create.  The plan
+ * launch per RHS.  params as for dg_plan_create.  The plan
  * works with dg_rhs, dg_rk_stage, dg_plan_set_element_scale, dg_finish,
  * dg_plan_info, dg_plan_path and dg_plan_destroy; dg_plan_set_variant
  * accepts variant 0 only, and the adjoint entry points and autotuners return
@@ -313,7 +320,9 @@ int dg_box_mesh_build(const dg_box_desc* desc, void* stream);
  * mma.sync products at the two other tile shapes of that kernel, one
  * thread per (element, node) of the tile: 7 (persistent) and 8 (one CTA
  * per tile) with 128 threads and 128 / Np elements per tile, 9 and 10 with
- * 512 threads and 512 / Np elements (variants 1 and 3: 256 / Np).  A
+ * 512 threads and 512 / Np elements (variants 1 and 3: 256 / Np).  On large
+ * meshes variants 0 and 2 of wave and Euler, and 1 and 3 of Maxwell at orders
+ * 2 and 3, run on kernels of their own with the same results bit for bit.  A
  * variant the plan does not support (a precision it does not apply to, or
  * a tile that does not fit on an SM) is refused with DG_ERR_UNSUPPORTED.
  * Default 0.  No counterpart in the reference. */
