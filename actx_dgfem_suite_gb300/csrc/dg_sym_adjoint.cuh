@@ -11,7 +11,7 @@
 //   dg_euler_vjp_sym_kernel      replaces dg_euler_vjp_volume: per direction k
 //     T_k = D'_k^T x back at the nodes, then y += J(h_k)^T T_k with the flux
 //     Jacobian in direction h_k (linear in the direction, so the metric needs no
-//     combinations of its own: 3 Jacobian products of ~35 operations per node,
+//     combinations of its own: 3 Jacobian products of 36 operations per node,
 //     where the dense kernel formed 45 combinations and 3 products of ~60);
 //     and the lifted adjoints of the five fields.
 //
@@ -259,7 +259,8 @@ __global__ void __launch_bounds__(AdjTile<N, DG_WAVE>::BLOCK)
   }
 }
 
-// Euler P3, 82,944 tets: 1.93 ms dense, 1.07 ms here.
+// Euler P3, 82,944 tets: 1.93 ms dense, 1.07 ms here before the shorter flux adjoint
+// (euler_flux_vjp).
 template <int N>
 __global__ void __launch_bounds__(AdjTile<N, DG_EULER>::BLOCK)
     dg_euler_vjp_sym_kernel(const VjpArgs a) {
@@ -386,14 +387,12 @@ __global__ void __launch_bounds__(AdjTile<N, DG_EULER>::BLOCK)
           for (int m = 0; m < 5; ++m) {
             q[m] = __ldg(a.q + m * nelnp + g);
             w[m] = z[m][n];
+            y[m] = k == 0 ? 0.0 : a.y[m * nelnp + g];
           }
           euler_flux_vjp(q, __ldg(a.aux + nelnp + g), __ldg(a.aux + g), h0, h1, h2, w, a.gamma,
                          y);
 #pragma unroll
-          for (int m = 0; m < 5; ++m) {
-            double* ym = a.y + m * nelnp + g;
-            *ym = k == 0 ? y[m] : *ym + y[m];
-          }
+          for (int m = 0; m < 5; ++m) a.y[m * nelnp + g] = y[m];
         }
       };
       for (int idx = t; idx < E * NO4; idx += BLOCK) {
