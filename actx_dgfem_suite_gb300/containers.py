@@ -21,7 +21,6 @@ from dataclasses import dataclass
 from typing import Any, Callable
 
 import numpy as np
-import torch
 
 
 class _Arith:
@@ -184,9 +183,9 @@ def map_leaves(state, f: Callable[[DOFArray], DOFArray]):
 
 def from_stacked(actx, template, stacked) -> Any:
     """Container of DOFArray views into ``stacked`` (nfields, Nel, Np)."""
-    views = stacked.unbind(0) if isinstance(stacked, torch.Tensor) else stacked
-    return rebuild(template, [DOFArray(actx, [v], stack=(stacked, k))
-                              for k, v in enumerate(views)])
+    # one index per field: autograd refuses in-place changes of unbind's views
+    return rebuild(template, [DOFArray(actx, [stacked[k]], stack=(stacked, k))
+                              for k in range(stacked.shape[0])])
 
 
 # }}}

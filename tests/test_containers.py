@@ -2,10 +2,11 @@
 
 import numpy as np
 import pytest
+import torch
 
 from actx_dgfem_suite_gb300.containers import (ConservedEulerField, DOFArray,
-                                               WaveState, _obj_array, leaves,
-                                               rebuild)
+                                               WaveState, _obj_array,
+                                               from_stacked, leaves, rebuild)
 from actx_dgfem_suite_gb300.rhs_builder import get_problem, split_equation_name
 
 
@@ -65,3 +66,23 @@ def test_unsupported_dims_and_equations():
         get_problem("tiny_wave", 1, 1)
     with pytest.raises(NotImplementedError):
         get_problem("tiny_burgers", 3, 1)
+
+
+@pytest.mark.parametrize("tracked", ["operand", "stack"])
+def test_stacked_views_can_be_changed_in_place_under_autograd(tracked):
+    """The arrays of a result are views of one stack; a program may add to one of
+    them in place and differentiate through it."""
+    template = _obj_array([_d([0.0])] * 6)
+    base = torch.arange(12.0, dtype=torch.float64).reshape(6, 2)
+    p = torch.tensor([0.5, -1.0], dtype=torch.float64, requires_grad=True)
+    stack = base.clone() if tracked == "operand" else base * p
+    leaf = leaves(from_stacked(None, template, stack))[3][0]
+    if tracked == "operand":
+        leaf.add_(p)
+        grad = [1.0, 1.0]
+    else:
+        leaf.mul_(2.0)
+        grad = (2.0 * base[3]).tolist()
+    assert stack[3].data_ptr() == leaf.data_ptr()
+    stack[3].sum().backward()
+    assert p.grad.tolist() == grad
