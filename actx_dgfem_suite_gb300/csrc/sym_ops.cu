@@ -146,6 +146,15 @@ int pack(const double* diff, const double* lift, const int32_t* face_nodes, bool
         fperm[g][f * NFP + j] = target * NFP + hit;
       }
     }
+  // a face that lists a node twice has no such permutation: its points would be left
+  // without a slot
+  for (int g = 0; g < 4; ++g) {
+    bool seen[NFPT] = {};
+    for (int k = 0; k < NFPT; ++k) {
+      if (seen[fperm[g][k]]) return -1;
+      seen[fperm[g][k]] = true;
+    }
+  }
   // }}}
 
   // {{{ orbits, slots and the symmetric combinations

@@ -206,6 +206,27 @@ def test_operators_without_the_symmetry_are_refused(order):
         assert order == 1
 
 
+@pytest.mark.parametrize("table", ["one vertex", "first node twice"])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_faces_that_list_a_node_twice_are_refused(order, table):
+    """With LIFT zero such a table commutes with the group, but its points are not
+    four to an orbit; the general kernel evaluates it as given."""
+    ref = reference_tet(order)
+    full = np.asarray(ref.face_nodes).reshape(4, -1)
+    fn = full.copy()
+    for f in range(4):
+        others = [set(full[g].tolist()) for g in range(4) if g != f]
+        vertex = set.intersection(*others).pop()      # the one opposite face f
+        if table == "one vertex":
+            nodes = [vertex] * fn.shape[1]
+        else:
+            nodes = [fn[f, 0], *fn[f, :-1]]
+        fn[f] = nodes
+    zero = np.zeros_like(ref.lift)
+    assert _pack(order, ref.weak_diff, zero, fn, False) is None
+    assert _pack(order, ref.weak_diff, zero, fn) is None
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("equation,order", [("wave", 1), ("wave", 4), ("euler", 2),
                                             ("euler", 3), ("maxwell", 3), ("maxwell", 4)])
