@@ -124,14 +124,14 @@ __device__ __forceinline__ void mirror(double* x, int narrays, int stride, int n
   }
 }
 
-// Euler: p, 1/rho and |u| + c of a state.
+// Euler: p, 1/rho and |u| + c = sqrt(|m|^2) / |rho| + sqrt(gamma p / rho) of a state.
 __device__ __forceinline__ void euler_node(const double* q, double gamma, double* s) {
   const double mm = fma(q[2], q[2], q[3] * q[3]);
   const double rinv = 1.0 / q[0];
   const double p = (gamma - 1.0) * fma(-0.5 * mm, rinv, q[1]);
   s[0] = p;
   s[1] = rinv;
-  s[2] = fma(sqrt(mm), rinv, sqrt(gamma * (p * rinv)));
+  s[2] = fma(sqrt(mm), fabs(rinv), sqrt(gamma * (p * rinv)));
 }
 
 // Flux of one edge point with interior and exterior trace (and Euler's per-node
