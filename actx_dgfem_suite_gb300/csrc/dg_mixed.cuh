@@ -66,10 +66,14 @@ struct Tile {
   static constexpr int G = A + pad16(AREA * PE * 4);
   static constexpr int FG = G + pad16(9 * PE * 4);
   static constexpr int SMEM = FG + pad16(16 * PE * 4);
-  // 16 warps per SM at least (128 registers per thread); 32 at order 1, whose
-  // short tiles need more of them in flight (wave P1, 663,552 tets: 180 us with 16,
-  // 148 with 32)
-  static constexpr int MIN_CTAS = (N == 1 ? 1024 : 512) / BLOCK;
+  // 16 warps per SM at least (128 registers per thread); at order 1, whose short
+  // tiles need more of them in flight, 32 for wave (663,552 tets: 180 us with 16, 148
+  // with 32) and 20 for Euler, whose stage spills at 32 (RK stage at 162,000 / 235,824 /
+  // 663,552 tets with 32, 28, 24, 20: 94 / 127 / 290, 87 / 118 / 280, 82 / 123 / 289, 80
+  // / 105 / 267 us, dg_rhs_kernel 90 / 122 / 324; RHS 66 / 91 / 211 with 32, 59 / 79 /
+  // 205 with 20)
+  static constexpr int WARPS = N == 1 ? (EQ == DG_EULER ? 20 : 32) : 16;
+  static constexpr int MIN_CTAS = WARPS / Ops<N>::NW;
 };
 
 struct Trace {
