@@ -86,3 +86,54 @@ def test_maxwell_warp_tile_edges(order, extra):
     for ref, a, b, c in zip(*got.values()):
         assert torch.equal(a, b) and torch.equal(a, c)
         assert float(torch.linalg.norm(a - ref)) <= MIXED_RTOL * float(torch.linalg.norm(ref))
+
+
+@pytest.mark.parametrize("equation,order,variants", [
+    *[(eq, o, (0, 2)) for eq in ("wave", "euler") for o in (1, 2, 3, 4)],
+    ("maxwell", 2, (1, 3)), ("maxwell", 3, (1, 3))])
+def test_members_of_a_large_mesh_have_their_own_meshs_bits(equation, order, variants):
+    """The kernels that plans take from some size on give the bits of the general
+    kernel, which serves each member's own mesh: copies of one mesh of 750 elements
+    (no multiple of any tile) side by side, each with a state of its own, RHS and RK
+    stage."""
+    from actx_dgfem_suite_gb300.discretization import union_discretization
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    per_sm = {2: 450, 3: 300}[order] if equation == "maxwell" else PER_SM[equation][order - 1]
+    params = {"wave": (0.9,), "euler": (1.4,), "maxwell": (0.8, 1.3, 0.7)}[equation]
+    prob = make_problem(equation, jittered_box_mesh(5), order, seed=order)
+    other = make_problem(equation, jittered_box_mesh(5), order, seed=order + 7)
+    nel = prob.disc.nelements
+    count = per_sm * nsm // nel + 1
+    union, offsets = union_discretization([prob.disc] * count)
+    # convex combinations of two admissible states
+    t = torch.linspace(0.0, 1.0, count, dtype=torch.float64, device="cuda")[:, None, None, None]
+    both = [torch.from_numpy(p.fields).cuda() for p in (prob, other)]
+    states = (1.0 - t) * both[0] + t * both[1]
+    scale = torch.linspace(0.8, 1.2, nel * count, dtype=torch.float64, device="cuda")
+
+    def evaluate(plan, q, scale):
+        plan.set_element_scale(None)
+        r = plan.rhs(q)
+        plan.set_element_scale(scale)
+        res, qo, un = 0.5 * q, torch.empty_like(q), torch.empty_like(q)
+        plan.rk_stage(q, qo, res, 0.3, 0.7, 1e-2, rhs_unscaled=un)
+        first, qf = torch.full_like(q, float("nan")), torch.empty_like(q)
+        plan.rk_stage(q, qf, first, 0.0, 0.7, 1e-2)
+        plan.finish()
+        return r, res, qo, un, first, qf
+
+    small = DevicePlan(DeviceMesh(prob.disc, "cuda:0"), equation, params, "fp32-mixed")
+    small.set_variant(variants[0])
+    assert small.info()["block"] == 256
+    want = [torch.cat(x, dim=1) for x in zip(*[
+        evaluate(small, states[k].contiguous(), scale[k * nel:(k + 1) * nel].contiguous())
+        for k in range(count)])]
+    large = DevicePlan(DeviceMesh(union, "cuda:0"), equation, params, "fp32-mixed")
+    q = torch.cat(list(states), dim=1).contiguous()
+    assert list(offsets) == [nel * k for k in range(count + 1)]
+    for variant in variants:
+        large.set_variant(variant)
+        assert large.info()["block"] != 256
+        for a, b in zip(evaluate(large, q, scale), want):
+            assert torch.equal(a, b)
