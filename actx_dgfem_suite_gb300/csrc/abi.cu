@@ -258,6 +258,7 @@ struct dg_plan {
   int mma_grid = 0;
   int64_t mma_ntiles = 0;
   float4* d_nodes = nullptr;   // Euler: FP32 node records, filled before each RHS
+                               // (d_pres is then this memory too)
   int nodes_grid = 0;
   // symmetry-adapted kernel (dg_sym.cuh, dg_sym2d.cuh): the main kernel of the
   // face-shared path and of triangle meshes for operators that have the element's
@@ -962,9 +963,33 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
   // 24 / 24, at 162 45 / 34; Euler P3 at 39 24 / 27, at 68 34 / 34, at 162 78 / 68.
   // Both kernels give the same bits.
   constexpr int kMixedPerSm[2][4] = {{540, 350, 120, 120}, {800, 100, 72, 72}};
-  const bool mix =
+  bool mix =
       kprec == 1 && equation != DG_MAXWELL &&
       p->nel >= (int64_t)kMixedPerSm[equation == DG_EULER ? 1 : 0][N - 1] * nsm;
+  // Euler's per-node table: node records for that kernel, FP32 pressures for the other
+  // variants, whichever the variant of a call needs in the same memory.  Where the
+  // records (32 bytes per node) do not fit, the general kernel serves variants 0 and 2
+  // too, with its 4 bytes.
+  if (kprec == 1 && equation == DG_EULER) {
+    const size_t nodes = (size_t)p->nel * np;
+    err = mix ? cudaMalloc(&p->d_nodes, nodes * 32) : cudaSuccess;
+    if (err == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      p->d_nodes = nullptr;
+      mix = false;
+    }
+    if (p->d_nodes)
+      p->d_pres = reinterpret_cast<float*>(p->d_nodes);
+    else if (!mix)
+      err = cudaMalloc(&p->d_pres, nodes * sizeof(float));
+    if (err != cudaSuccess) {
+      dg_plan_destroy(p);
+      return cuda_fail(err, "per-node table");
+    }
+    const int64_t pblocks = (p->nel * np + dg::kFaceBlock - 1) / dg::kFaceBlock;
+    const int64_t pfull = (int64_t)nsm * 8;
+    p->pres_grid = (int)(pblocks < pfull ? pblocks : pfull);
+  }
   if (mix) {
     dg::LaunchShape x0, x1;
     err = equation == DG_WAVE ? dg::mixed_shape_wave(N, false, &x0)
@@ -976,8 +1001,6 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
         dg::pack_mixed_ops(N, diff, mesh->lift, mesh->face_nodes, nullptr, 0));
     const int xbytes = dg::pack_mixed_ops(N, diff, mesh->lift, mesh->face_nodes, xops.data(),
                                           (int)xops.size());
-    if (err == cudaSuccess && equation == DG_EULER)
-      err = cudaMalloc(&p->d_nodes, (size_t)p->nel * np * 32);
     if (err == cudaSuccess) err = cudaMalloc(&p->d_mix_ops, xops.size());
     if (err == cudaSuccess)
       err = cudaMemcpy(p->d_mix_ops, xops.data(), xops.size(), cudaMemcpyHostToDevice);
@@ -1040,17 +1063,6 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     p->mma_grid = (int)(p->mma_ntiles < xfull ? p->mma_ntiles : xfull);
   }
   p->face_partner = mesh->face_partner;
-
-  if (kprec == 1 && equation == DG_EULER) {
-    err = cudaMalloc(&p->d_pres, (size_t)p->nel * np * sizeof(float));
-    if (err != cudaSuccess) {
-      dg_plan_destroy(p);
-      return cuda_fail(err, "pressure table");
-    }
-    const int64_t pblocks = (p->nel * np + dg::kFaceBlock - 1) / dg::kFaceBlock;
-    const int64_t pfull = (int64_t)nsm * 8;
-    p->pres_grid = (int)(pblocks < pfull ? pblocks : pfull);
-  }
 
   if (split) {
     p->d_face_nodes = reinterpret_cast<const int32_t*>(
@@ -1920,7 +1932,7 @@ int dg_plan_destroy(dg_plan* p) {
   for (void* b : {(void*)p->d_owned, (void*)p->d_flux, (void*)p->d_aux,
                   (void*)p->d_tc_ops, p->d_tcm_ops[0], p->d_tcm_ops[1],
                   p->d_tcm_ops[2] != p->d_tcm_ops[1] ? p->d_tcm_ops[2] : nullptr,
-                  (void*)p->d_pres, p->d_sym_ops, p->d_adj_sym_ops,
+                  p->d_nodes ? nullptr : (void*)p->d_pres, p->d_sym_ops, p->d_adj_sym_ops,
                   p->d_mix_ops, (void*)p->d_nodes, p->d_mma_ops})
     if (b && cudaFree(b) != cudaSuccess) code = DG_ERR_CUDA;
   delete p;

@@ -137,3 +137,22 @@ def test_members_of_a_large_mesh_have_their_own_meshs_bits(equation, order, vari
         assert large.info()["block"] != 256
         for a, b in zip(evaluate(large, q, scale), want):
             assert torch.equal(a, b)
+
+
+def test_euler_plan_holds_one_table_per_node():
+    """Node records (32 bytes) and pressures (4 bytes) of a mixed Euler plan serve
+    different variants, so the plan holds room for one of them."""
+    from actx_dgfem_suite_gb300.device_setup import DeviceBoxDiscretization
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    disc = DeviceBoxDiscretization(4, 28, -0.5, 0.5, with_nodes=False)
+    mesh = DeviceMesh(disc, "cuda:0")
+    used = []
+    for _ in range(2):                           # the first loads the kernels
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        plan = DevicePlan(mesh, "euler", (1.4,), "fp32-mixed")
+        used.append(before - torch.cuda.mem_get_info()[0])
+        plan.close()
+    nodes = mesh.nelements * mesh.np_            # 4.6 million: 147.5 and 18.4 MB
+    # operator blocks and allocation granularity: 8 MB
+    assert used[1] <= 32 * nodes + 8 * 2**20
