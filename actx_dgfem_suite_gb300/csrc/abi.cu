@@ -1079,8 +1079,9 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     // tiles of 256 / Np elements finish sooner than tiles of 32 (one tile per SM and
     // less).  Measured (RHS, us, general / symmetric): at 1,296 elements, 8.5 per SM,
     // wave P3 29 / 36, Euler P3 51 / 68, wave P4 72 / 72, Euler P4 132 / 135; at 3,072
-    // wave P3 51 / 38, Euler P3 91 / 75, Euler P4 250 / 142.  Order 1 and Maxwell (tiles
-    // of 16): no slower at any size (Maxwell P3 at 162 elements 55 / 36).
+    // wave P3 51 / 38, Euler P3 91 / 75, Euler P4 250 / 142; order 2 at 14 elements per SM
+    // wave 23 / 22, Euler 38 / 40, at 26 wave 36 / 24, Euler 62 / 44.  Order 1 and Maxwell
+    // (tiles of 16): no slower at any size (Maxwell P3 at 162 elements 55 / 36).
     const int per_sm = equation == DG_MAXWELL || N == 1 ? 0 : (N == 4 ? 9 : 13);
     const bool strong = equation == DG_MAXWELL, reduce = equation != DG_EULER;
     std::vector<unsigned char> sops(
@@ -1186,10 +1187,14 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
     const int64_t afull = (int64_t)nsm * ashape.blocks_per_sm;
     p->adj_grid = (int)(atiles < afull ? atiles : afull);
 
-    // as for the RHS, with two phases per tile: measured (vjp, us, dense / symmetric)
-    // Euler P2 at 6,000 elements 103 / 109, at 10,368 162 / 151; Euler P3 at 3,072
-    // 129 / 142, at 6,000 245 / 209; Euler P4 at 1,296 174 / 222, at 3,072 256 / 241
-    const int per_sm = N <= 2 ? 48 : (N == 3 ? 32 : 16);
+    // as for the RHS, with two phases per tile.  Measured by elements per SM (vjp, us,
+    // dense / symmetric): wave P1 at 32 16 / 14, at 43-64 16 / 17 (one round of dense
+    // tiles), at 68 25 / 23; P2 at 48 32 / 34, at 53 46 / 37; P3 at 36 61 / 64, at 39 79 / 67;
+    // P4 at 14 61 / 77, at 18 89 / 80.  Euler P1 at 39 48 / 49, at 48 64 / 61; P2 at 18 58 /
+    // 62, at 48 118 / 98; P3 at 12 71 / 103, at 32 187 / 129; P4 at 14 175 / 181, at 18 257 /
+    // 193.  The reverse RK stage: the same ratios within 3 %.
+    constexpr int kPerSm[2][4] = {{64, 50, 36, 16}, {48, 48, 32, 16}};
+    const int per_sm = kPerSm[equation == DG_EULER ? 1 : 0][N - 1];
     std::vector<unsigned char> sops(
         dg::pack_sym_adj_ops(N, diff, mesh->lift, mesh->face_nodes, equation == DG_WAVE, nullptr,
                              0));

@@ -498,3 +498,36 @@ def test_triangles_glued_with_a_turn_are_not_shared():
         blocks.append(plan.info()["block"])
     assert blocks[0] != blocks[1]
     assert float(torch.linalg.norm(got[0] - got[1])) <= 1e-10 * float(torch.linalg.norm(got[1]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order,per_sm", [(1, 64), (2, 50), (3, 36)])
+@pytest.mark.parametrize("extra", [0, 1, 31, 33])
+def test_wave_adjoint_size_rule(order, per_sm, extra):
+    """The wave adjoint from the smallest mesh that takes the symmetric kernel,
+    against the dense one (operators moved by 1e-11)."""
+    import torch
+
+    from actx_dgfem_suite_gb300.mesh import TetMesh
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import jittered_box_mesh, make_problem
+    nel = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    mesh = jittered_box_mesh(12)
+    mesh = TetMesh(vertices=mesh.vertices, elements=mesh.elements[:nel])
+    prob = make_problem("wave", mesh, order, seed=nel)
+    x = torch.from_numpy(prob.fields).cuda()
+    lq = x.roll(1, dims=0).contiguous()
+    got = []
+    for off in (0.0, 1e-11):
+        dm = DeviceMesh(prob.disc, "cuda:0")
+        dm._weak = dm._weak.copy()
+        dm._weak.reshape(-1)[1] += off * abs(dm._weak).max()
+        plan = DevicePlan(dm, "wave", prob.params, "fp64")
+        y = plan.vjp(x, x)
+        lam, rbar, scr = 0.3 * x, torch.empty_like(x), torch.empty_like(x)
+        cbar = torch.ones(nel, dtype=torch.float64, device="cuda")
+        plan.adjoint_stage(x, 0.7, lam, rbar, lq, cbar, 0.4, 0.9, 1e-2, scr)
+        plan.finish()
+        got.append((y, lam, rbar, cbar))
+    for a, b in zip(*got):
+        assert float(torch.linalg.norm(a - b)) <= 1e-10 * float(torch.linalg.norm(b))
