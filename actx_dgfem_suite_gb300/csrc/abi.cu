@@ -264,6 +264,7 @@ struct dg_plan {
   // face-shared path and of triangle meshes for operators that have the element's
   // symmetry
   bool sym = false;
+  bool sym_stage = true;       // its RK stage too (tetrahedra)
   void* d_sym_ops = nullptr;
   uint32_t sym_ops_bytes = 0;
   dg::LaunchShape sym_shape;
@@ -414,6 +415,8 @@ constexpr int kShapeModeBits[2] = {dg::MODE_B128, dg::MODE_B512};
 bool uses_mix(const dg_plan* p) { return p->mix && (p->variant | 2) == 2; }
 // The plan's variant runs dg_maxwell_mma_kernel.
 bool uses_mma(const dg_plan* p) { return p->mma && (p->variant | 2) == 3; }
+// The RHS or RK stage of the plan runs dg_rhs_sym_kernel.
+bool uses_sym(const dg_plan* p, bool stage) { return p->sym && (!stage || p->sym_stage); }
 
 // Mode bits and grid of the main kernel under the plan's variant.
 int main_mode(const dg_plan* p, int base) {
@@ -421,7 +424,7 @@ int main_mode(const dg_plan* p, int base) {
     return base | dg::MODE_TC | kShapeModeBits[shape_index(p->variant)];
   return base | ((p->variant & 1) && p->precision == DG_FP32_MIXED ? dg::MODE_TC : 0);
 }
-int main_grid(const dg_plan* p) {
+int main_grid(const dg_plan* p, bool stage = false) {
   if (is_shape_variant(p->variant)) {
     const int k = shape_index(p->variant);
     if ((p->variant - kFirstShapeVariant) & 1)
@@ -438,7 +441,7 @@ int main_grid(const dg_plan* p) {
       return (int)(p->mma_ntiles < 0x7fffffff ? p->mma_ntiles : 0x7fffffff);
     return p->mma_grid;
   }
-  if (p->sym) {
+  if (uses_sym(p, stage)) {
     if (p->variant & 2)
       return (int)(p->sym_ntiles < 0x7fffffff ? p->sym_ntiles : 0x7fffffff);
     return p->sym_grid;
@@ -1112,6 +1115,15 @@ int dg_plan_create(dg_plan** plan_out, int32_t equation, int32_t precision,
       p->sym_ntiles = (p->nel + s0.elems_per_tile - 1) / s0.elems_per_tile;
       const int64_t sfull = (int64_t)nsm * s0.blocks_per_sm;
       p->sym_grid = (int)(p->sym_ntiles < sfull ? p->sym_ntiles : sfull);
+      // The RK stage, whose loads and stores the dense kernel's smaller tiles overlap
+      // better, crosses a little later: order 4 after two rounds of dense tiles (at 14 per
+      // SM wave 75 / 80, Euler 135 / 145; at 15 106 / 79, 198 / 146), Euler order 2 after
+      // one (at 14 40 / 42, at 23 45 / 46, at 26 64 / 47).
+      const int stage_per_sm = equation == DG_MAXWELL       ? 0
+                               : N == 4                     ? 14
+                               : N == 2 && equation == DG_EULER ? 25
+                                                            : 0;
+      p->sym_stage = p->nel > (int64_t)stage_per_sm * nsm;
     }
   }
 
@@ -1529,13 +1541,13 @@ cudaError_t launch_main(const dg_plan* p, dg::RhsArgs a, bool stage, cudaStream_
     a.ops_bytes = p->mma_ops_bytes;
     return dg::mma_launch_maxwell(p->order, stage, a, main_grid(p), s);
   }
-  if (p->sym) {
+  if (uses_sym(p, stage)) {
     a.ops = p->d_sym_ops;
     a.ops_bytes = p->sym_ops_bytes;
-    return sym_launch_of(p->equation, p->order, stage, a, main_grid(p), s);
+    return sym_launch_of(p->equation, p->order, stage, a, main_grid(p, stage), s);
   }
   const int base = (stage ? dg::MODE_STAGE : dg::MODE_RHS) | (p->split ? dg::MODE_SPLIT : 0);
-  return launch_of(p->equation, p->order, prec, main_mode(p, base), a, main_grid(p), s);
+  return launch_of(p->equation, p->order, prec, main_mode(p, base), a, main_grid(p, stage), s);
 }
 
 // Triangle meshes: the one launch of an RHS or RK stage.

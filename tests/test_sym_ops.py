@@ -501,6 +501,38 @@ def test_triangles_glued_with_a_turn_are_not_shared():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("equation,order,per_sm", [("wave", 4, 14), ("euler", 4, 14),
+                                                   ("euler", 2, 25)])
+@pytest.mark.parametrize("extra", [0, 1, 33])
+def test_stage_size_rule(equation, order, per_sm, extra):
+    """RK stages around the size from which they take the symmetric kernel: as the
+    fused general kernel, and the bits of the RHS only above the line."""
+    import torch
+
+    from actx_dgfem_suite_gb300.mesh import TetMesh
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import jittered_box_mesh, make_problem
+    nel = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    mesh = jittered_box_mesh(9)
+    mesh = TetMesh(vertices=mesh.vertices, elements=mesh.elements[:nel])
+    prob = make_problem(equation, mesh, order, seed=nel)
+    q = torch.from_numpy(prob.fields).cuda()
+    got = []
+    for partner in (True, False):
+        plan = DevicePlan(DeviceMesh(prob.disc, "cuda:0", with_partner=partner), equation,
+                          prob.params, "fp64")
+        r = plan.rhs(q)
+        res, qo, un = 0.5 * q, torch.empty_like(q), torch.empty_like(q)
+        plan.rk_stage(q, qo, res, 0.3, 0.7, 1e-2, rhs_unscaled=un)
+        plan.finish()
+        if partner:
+            assert torch.equal(un, r) == (extra > 0)
+        got.append((res, qo, un))
+    for a, b in zip(*got):
+        assert float(torch.linalg.norm(a - b)) <= 1e-12 * float(torch.linalg.norm(b))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("order,per_sm", [(1, 64), (2, 50), (3, 36)])
 @pytest.mark.parametrize("extra", [0, 1, 31, 33])
 def test_wave_adjoint_size_rule(order, per_sm, extra):
