@@ -1341,12 +1341,24 @@ int dg_plan_create_2d(dg_plan** plan_out, int32_t equation,
   const int sbytes = dg::pack_sym_ops_2d(N, diff, mesh->lift, mesh->face_nodes, sops.data(),
                                          (int)sops.size());
   // The symmetry-adapted kernel's tile of 32 elements takes longer from start to end
-  // than the dense kernel's smaller ones, which pays once SMs hold more than one.
-  // Measured (dense / symmetric, us): at 32 elements per SM wave P4 21 / 31, Euler P4
+  // than the dense kernel's of 256 / Np, which pays once SMs hold more than one.
+  // Measured (RHS, dense / symmetric, us): at 32 elements per SM wave P4 21 / 31, Euler P4
   // 47 / 59, wave P2 10 / 14; at 48 wave P4 31 / 31, Euler P4 69 / 60, wave P3 19 / 21,
-  // wave P2 16 / 14; at 84 wave P4 50 / 41, Euler P3 86 / 56; order 1 at any size
-  // (wave 10 / 9, Euler 24 / 15 at 800 elements).
-  const bool fills = N == 1 || p->nel >= (int64_t)48 * nsm;
+  // wave P2 16 / 14; at 84 wave P4 50 / 41, Euler P3 86 / 56.  Order 1 from two tiles
+  // (Euler: more than one) on: wave 6.2 / 8.0 at 32 elements, 8.3 / 8.5 at 64, 10 / 8.3 at
+  // 128; Euler 12.4 / 12.2 at 32, 18 / 13 at 50.  Where the fullest SM holds three tiles
+  // against one dense tile at order 1, or three against two at order 2, the dense kernel
+  // finishes first for wave and Maxwell: P1 at 65-84 per SM wave 10.4 / 11.9, Maxwell 11.0 /
+  // 12.5 (Euler 24.5 / 22.5), six against two at 161-170 wave 24 / 27; P2 at 65-83 wave 16.7 /
+  // 18.2, Maxwell 18.7 / 19.4.
+  const auto rounds = [&](int64_t elems) { return (p->nel + elems * nsm - 1) / (elems * nsm); };
+  const int64_t dense_rounds = rounds(shape.elems_per_tile), sym_rounds = rounds(32);
+  const bool light = equation != DG_EULER;
+  bool fills = p->nel >= (int64_t)48 * nsm;
+  if (N == 1)
+    fills = light ? p->nel >= 64 && sym_rounds < 3 * dense_rounds : p->nel > 32;
+  else if (N == 2 && light && sym_rounds == 3 && dense_rounds == 2)
+    fills = false;
   if (sbytes > 0 && fills) {  // the operators have the symmetry
     dg::LaunchShape s0, s1;
     err = dg::sym_shape_2d(equation, N, dg::MODE_RHS, &s0);

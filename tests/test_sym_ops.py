@@ -501,6 +501,50 @@ def test_triangles_glued_with_a_turn_are_not_shared():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("equation", ["wave", "euler", "maxwell"])
+@pytest.mark.parametrize("order,tiles,extra", [(1, 0, 2), (1, 0, 32), (1, 0, 34), (1, 0, 62),
+                                               (1, 0, 64), (1, 2, 0), (1, 2, 2), (1, 6, 0),
+                                               (2, 2, 0), (2, 2, 2), (2, 3, 0)])
+def test_triangle_size_rule(equation, order, tiles, extra):
+    """Element counts on both sides of the lines between the dense and the symmetric
+    kernel, in rounds of 32 elements per SM: the kernel that the rule names, and the
+    dense kernel's result (as above on operators moved by 1e-11)."""
+    import torch
+
+    from actx_dgfem_suite_gb300.mesh import TriMesh, generate_box_tri_mesh
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    from tests._helpers import make_problem_2d
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    nel = 32 * tiles * nsm + extra
+    full = generate_box_tri_mesh(0.0, 1.0, (8, nel // 16 + 1))
+    prob = make_problem_2d(equation, TriMesh(vertices=full.vertices, elements=full.elements[:nel]),
+                           order, seed=nel)
+    dense = 256 // prob.disc.np_                 # elements per tile
+    rounds, dense_rounds = -(-nel // (32 * nsm)), -(-nel // (dense * nsm))
+    if order == 1:
+        symmetric = nel > 32 if equation == "euler" else nel >= 64 and rounds < 3 * dense_rounds
+    else:
+        symmetric = equation == "euler" or (rounds, dense_rounds) != (3, 2)
+    q = torch.from_numpy(prob.fields).cuda()
+    got = []
+    for off in (0.0, 1e-11):
+        dm = DeviceMesh(prob.disc, "cuda:0")
+        for name in ("_weak", "_strong"):
+            ops = getattr(dm, name).copy()
+            ops.reshape(-1)[1] += off * abs(ops).max()
+            setattr(dm, name, ops)
+        plan = DevicePlan(dm, equation, prob.params, "fp64")
+        r = plan.rhs(q)
+        res, qo = 0.5 * q, torch.empty_like(q)
+        plan.rk_stage(q, qo, res, 0.3, 0.7, 1e-2)
+        plan.finish()
+        assert (plan.info()["block"] == 128) == (symmetric and off == 0.0)
+        got.append((r, res, qo))
+    for a, b in zip(*got):
+        assert float(torch.linalg.norm(a - b)) <= 1e-10 * float(torch.linalg.norm(b))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("equation,order,per_sm", [("wave", 4, 14), ("euler", 4, 14),
                                                    ("euler", 2, 25)])
 @pytest.mark.parametrize("extra", [0, 1, 33])
