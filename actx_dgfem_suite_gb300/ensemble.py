@@ -7,6 +7,11 @@ loop balances uneven members automatically and no member-level control flow
 exists on the device.  The launch can be captured in a CUDA graph and
 replayed once per RHS.
 
+In FP32-mixed precision a member's result has the bits of the member
+evaluated alone with the same launch variant.  FP64 plans sum in another
+order on small meshes than on large ones, so there a small wave or Euler
+member of a large union agrees with the member alone to rounding.
+
 The reference has no ensemble path; this is the batched form asked of the
 GB300 build (64 Maxwell P3 members on boxes with n ~ U[12, 40]).
 """

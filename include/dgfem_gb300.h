@@ -96,7 +96,9 @@ typedef struct dg_mesh_desc {
  * Which kernels a plan takes depends on its operators and size only: where
  * diff and lift have the reference tetrahedron's four-group symmetry to
  * rounding, FP64 volume, LIFT and adjoint products run in the symmetry-adapted
- * basis (a quarter of the multiply-adds) on all but small meshes.
+ * basis (a quarter of the multiply-adds) on all but small meshes.  The two sum in
+ * different orders, so FP64 results of one mesh alone and as part of a larger one agree
+ * to rounding, not bit for bit (DG_FP32_MIXED results of one variant do, bit for bit).
  *
  * Replaces the compile step of the reference's array contexts:
  * actx.compile(rhs) (actx_dgfem_suite/run/__main__.py:74) and the DAG/loopy
