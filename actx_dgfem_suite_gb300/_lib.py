@@ -38,7 +38,8 @@ EXPORTED_SYMBOLS = ("dg_plan_create", "dg_plan_create_2d", "dg_rhs", "dg_rk_stag
                     "dg_rhs_adjoint", "dg_rhs_adjoint_noalloc",
                     "dg_rhs_adjoint_stage", "dg_rhs_vjp", "dg_rhs_vjp_stage",
                     "dg_box_mesh_build",
-                    "dg_plan_path", "dg_plan_info", "dg_plan_set_variant",
+                    "dg_plan_path", "dg_plan_info", "dg_plan_kernel",
+                    "dg_plan_set_variant",
                     "dg_plan_autotune", "dg_plan_autotune_bounded",
                     "dg_fp64_fma_probe", "dg_wait_probe", "dg_stream_copy",
                     "dg_last_error",
@@ -170,6 +171,8 @@ def lib() -> ctypes.CDLL:
     L.dg_plan_info.argtypes = [vp, ctypes.POINTER(ctypes.c_int64), i32p, i32p,
                                i32p, i32p, i32p]
     L.dg_plan_info.restype = ctypes.c_int
+    L.dg_plan_kernel.argtypes = [vp]
+    L.dg_plan_kernel.restype = ctypes.c_char_p
     L.dg_plan_path.argtypes = [vp, i32p, i32p, i32p, ctypes.POINTER(ctypes.c_int64)]
     L.dg_plan_set_variant.argtypes = [vp, ctypes.c_int32]
     L.dg_plan_set_variant.restype = ctypes.c_int

@@ -2049,6 +2049,16 @@ int dg_plan_path(const dg_plan* p, int32_t* face_shared, int32_t* tensor_cores,
   return DG_OK;
 }
 
+const char* dg_plan_kernel(const dg_plan* p) {
+  if (!p) return "";
+  if (p->dim == 2) return p->sym ? "dg_rhs2d_sym_kernel" : "dg_rhs2d_kernel";
+  if (p->tc) return "dg_rhs_tc_kernel";
+  if (is_tcm_variant(p->variant)) return "dg_rhs_tcm_kernel";
+  if (uses_mix(p)) return "dg_rhs_mixed_kernel";
+  if (uses_mma(p)) return "dg_maxwell_mma_kernel";
+  return uses_sym(p, false) ? "dg_rhs_sym_kernel" : "dg_rhs_kernel";
+}
+
 int dg_plan_info(const dg_plan* p, int64_t* nelements, int32_t* order,
                  int32_t* nfields, int32_t* grid, int32_t* block,
                  int32_t* smem_bytes) {

@@ -135,10 +135,20 @@ def bytes_per_element(equation: str, order: int, dim: int = 3) -> int:
 _SYM_FMA = {1: (1, 1, 12), 2: (24, 10, 60), 3: (100, 50, 200), 4: (304, 175, 525)}
 
 
-def fp64_fma_per_element(equation: str, order: int) -> int:
-    """FP64 fused multiply-adds that the face-shared path's volume/LIFT kernel issues
-    per element in its contractions (``csrc/dg_sym.cuh``); plans on other kernels
-    issue more (the dense products: up to 4 times as many)."""
+def fp64_fma_per_element(equation: str, order: int,
+                         kernel: str = "dg_rhs_sym_kernel") -> int:
+    """FP64 fused multiply-adds that the volume/LIFT kernel ``kernel`` (the plan's
+    ``info()["kernel"]``) issues per element in its contractions: the
+    symmetry-adapted blocks (``csrc/dg_sym.cuh``) or the dense products of
+    ``dg_rhs_kernel``, up to 4 times as many.  Both share the reference derivatives of
+    a field between its gradient components."""
+    if kernel == "dg_rhs_kernel":
+        n, points = np_of(order), 4 * nfp_of(order)
+        # wave 3 D_r u + sum_r D_r (G v)_r, Euler 5 fluxes, Maxwell 6 fields x 3 D_r
+        products = {"wave": 6, "euler": 15, "maxwell": 18}[equation]
+        return products * n * n + NFIELDS[equation] * n * points
+    if kernel != "dg_rhs_sym_kernel":
+        raise ValueError(f"no FP64 multiply-add count for {kernel}")
     diff, low, lift = _SYM_FMA[order]
     extra = low if order > 1 else 0      # nodes <-> coefficients of degree N - 1
     if equation == "wave":
@@ -159,6 +169,8 @@ class RhsCost:
     #: faces on the boundary (box of n^3 hexahedra: 12 n^2), for the wave
     #: boundary pair's extra operation; 0 leaves it out
     boundary_faces: int = 0
+    #: volume/LIFT kernel whose multiply-adds :attr:`fma` counts
+    kernel: str = "dg_rhs_sym_kernel"
 
     @property
     def dofs(self) -> int:
@@ -179,7 +191,7 @@ class RhsCost:
 
     @property
     def fma(self) -> int:
-        return self.nelements * fp64_fma_per_element(self.equation, self.order)
+        return self.nelements * fp64_fma_per_element(self.equation, self.order, self.kernel)
 
     def roofline_seconds(self, peak_flops: float, peak_bytes: float) -> float:
         """``max(F / peak_F, B / peak_BW)`` (``perf_analysis.py:643-651``)."""

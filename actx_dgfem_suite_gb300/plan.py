@@ -179,7 +179,8 @@ class DevicePlan:
         return dict(nelements=nel.value, order=order, nfields=nf, grid=grid,
                     block=block, smem_bytes=smem, face_shared=bool(shared.value),
                     tensor_cores=bool(tcores.value),
-                    launches_per_rhs=launches.value, owned_faces=owned.value)
+                    launches_per_rhs=launches.value, owned_faces=owned.value,
+                    kernel=self._lib.dg_plan_kernel(self._handle).decode())
 
     @property
     def launches_per_rhs(self) -> int:

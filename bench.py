@@ -547,7 +547,8 @@ def our_arm(args) -> None:
         runs.append(dict(eq=eq, order=order, n=n_eff, compiled=compiled,
                          call_args=call_args, q=q, out=out,
                          cost=pm.RhsCost(eq, order, nel,
-                                         boundary_faces=12 * n_eff * n_eff)))
+                                         boundary_faces=12 * n_eff * n_eff,
+                                         kernel=compiled.plan.info()["kernel"])))
         if hasattr(rhs.dg_operator.disc, "_cache"):
             rhs.dg_operator.disc._cache.clear()
     clear_box_cache()
@@ -696,18 +697,15 @@ def our_arm(args) -> None:
     traffic = _ncu_traffic(path).get(f"{rd['eq']}{rd['order']}")
     if traffic is not None and (args.scale != 1 or args.precision == "fp32-mixed"):
         traffic = None
-    if info["tensor_cores"]:
-        kname = f"dg_rhs_tc_kernel<{rd['order']}, {rd['eq']}, SPLIT>"
-    else:
-        kname = (f"dg_rhs_kernel<{rd['order']}, {rd['eq']}, "
-                 f"{'float' if args.precision == 'fp32-mixed' else 'double'}, RHS>")
-    if info["face_shared"] and not info["tensor_cores"]:
-        kname = f"dg_rhs_sym_kernel<{rd['order']}, {rd['eq']}>"
+    kname = f"{info['kernel']}<{rd['order']}, {rd['eq']}>"
     if info["face_shared"]:
         kname = (f"dg_face_flux_kernel<{rd['order']}, {rd['eq']}>"
                  + (" + dg_euler_aux_kernel" if rd["eq"] == "euler" else "")
                  + " + " + kname + " (one RHS)")
-    fp64_achieved = 2.0 * c.fma / t_dom / 1e12
+    # multiply-adds of the FP64 kernels' products; no count for the other precisions
+    fp64_rate = ((lambda cost, sec: 2.0 * cost.fma / sec / 1e12) if args.precision == "fp64"
+                 else (lambda cost, sec: None))
+    fp64_achieved = fp64_rate(c, t_dom)
     roofline = {
         "bound": "hbm", "achieved": achieved_gbs, "peak": peaks["hbm_gbs"],
         "unit": "GB/s", "frac": achieved_gbs / peaks["hbm_gbs"],
@@ -716,7 +714,7 @@ def our_arm(args) -> None:
         "peak_source": peaks["source"],
         "fp64_pipe": {"achieved_tflops": fp64_achieved,
                       "peak_tflops": fp64_peak,
-                      "frac": fp64_achieved / fp64_peak,
+                      "frac": fp64_achieved and fp64_achieved / fp64_peak,
                       "peak_source": "measured live (dg_fp64_fma_probe)"},
         "limiter": "fp64 pipe",
         "suite_model_frac": c.roofline_seconds(fp64_peak * 1e12,
@@ -743,7 +741,7 @@ def our_arm(args) -> None:
                  "nel": r["cost"].nelements, "ms": case_ms[k],
                  "gdof_s": r["cost"].dofs / case_ms[k] / 1e6,
                  "gflops_suite": r["cost"].flops / case_ms[k] / 1e6,
-                 "fp64_frac": 2 * r["cost"].fma / (case_ms[k] * 1e-3) / 1e12 / fp64_peak,
+                 "fp64_frac": fp64_rate(r["cost"], case_ms[k] * 1e-3 * fp64_peak),
                  "hbm_frac": r["cost"].bytes / (case_ms[k] * 1e-3) / 1e9 / peaks["hbm_gbs"]}
                 for k, r in enumerate(runs)]
     if rank == 0:

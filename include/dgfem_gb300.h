@@ -377,6 +377,12 @@ int dg_plan_info(const dg_plan* plan, int64_t* nelements, int32_t* order,
                  int32_t* nfields, int32_t* grid, int32_t* block,
                  int32_t* smem_bytes);
 
+/* Name of the kernel that evaluates volume term and LIFT in dg_rhs under the plan's
+ * variant (a static string; "" for NULL): dg_rhs_sym_kernel, dg_rhs_tc_kernel,
+ * dg_rhs_mixed_kernel, dg_maxwell_mma_kernel, dg_rhs_tcm_kernel, dg_rhs_kernel, and on
+ * triangles dg_rhs2d_sym_kernel or dg_rhs2d_kernel. */
+const char* dg_plan_kernel(const dg_plan* plan);
+
 /* Measurement helper (no counterpart in the reference, which hard-codes
  * datasheet peaks in actx_dgfem_suite/consts.py:1-12): runs `grid` x `block`
  * threads, each issuing 8 independent FP64 FMA chains of `iters` steps, and

@@ -238,3 +238,29 @@ def test_bounded_autotune_at_mid_size_wave_p3():
     out = mixed.rhs(q)
     mixed.finish()
     assert float(torch.linalg.norm(out - r64) / torch.linalg.norm(r64)) <= MIXED_RTOL
+
+
+@pytest.mark.parametrize("equation,order,precision,small,large", [
+    ("wave", 3, "fp64", "dg_rhs_kernel", "dg_rhs_sym_kernel"),
+    ("euler", 2, "fp64", "dg_rhs_kernel", "dg_rhs_sym_kernel"),
+    ("maxwell", 4, "fp64", "dg_rhs_sym_kernel", "dg_rhs_sym_kernel"),
+    ("euler", 3, "fp64-tc", "dg_rhs_tc_kernel", "dg_rhs_tc_kernel"),
+    ("euler", 4, "fp32-mixed", "dg_rhs_kernel", "dg_rhs_mixed_kernel")])
+def test_info_names_the_kernel(equation, order, precision, small, large):
+    """Small meshes and large ones; and operators without the symmetry."""
+    from actx_dgfem_suite_gb300.discretization import make_box_discretization
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    params = {"wave": (1.0,), "euler": (1.4,), "maxwell": (1.0, 1.0, 1.0)}[equation]
+    for n, name in ((2, small), (13, large)):
+        mesh = DeviceMesh(make_box_discretization(order, n), "cuda:0")
+        plan = DevicePlan(mesh, equation, params, precision)
+        assert plan.info()["kernel"] == name
+        if precision == "fp32-mixed":
+            for variant, other in ((1, "dg_rhs_kernel"), (5, "dg_rhs_tcm_kernel"),
+                                   (7, "dg_rhs_kernel")):
+                plan.set_variant(variant)
+                assert plan.info()["kernel"] == other
+        if precision == "fp64":
+            mesh._weak, mesh._strong = 1.01 * mesh._weak, 1.01 * mesh._strong
+            mesh._weak.reshape(-1)[0] = mesh._strong.reshape(-1)[0] = 0.0
+            assert DevicePlan(mesh, equation, params).info()["kernel"] == "dg_rhs_kernel"

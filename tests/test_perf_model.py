@@ -95,3 +95,19 @@ def test_print_roofline_dims_2_and_3(capsys):
         (dim, eq, d) for dim in (2, 3) for eq in ("tiny_wave", "euler") for d in (1, 4)}
     assert all(r[4] > 0 and r[5] > 0 and r[6] > 0 for r in rows)
     assert " 2 euler" in capsys.readouterr().out
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_fma_count_is_the_kernels(order):
+    """The symmetry-adapted blocks issue fewer multiply-adds than the dense products,
+    which have 3 Np x Np derivatives and an Np x 4 Nfp LIFT per field at least."""
+    n, points = pm.np_of(order), 4 * pm.nfp_of(order)
+    for eq, nf, products in (("wave", 4, 6), ("euler", 5, 15), ("maxwell", 6, 18)):
+        dense = pm.fp64_fma_per_element(eq, order, "dg_rhs_kernel")
+        assert dense == products * n * n + nf * n * points
+        sym = pm.fp64_fma_per_element(eq, order)
+        assert sym == pm.fp64_fma_per_element(eq, order, "dg_rhs_sym_kernel")
+        assert 3 * sym < dense
+        assert pm.RhsCost(eq, order, 7, kernel="dg_rhs_kernel").fma == 7 * dense
+    with pytest.raises(ValueError):
+        pm.fp64_fma_per_element("wave", order, "dg_rhs_tcm_kernel")
