@@ -26,6 +26,9 @@ RHS), whole job.
   time of the device-resident step.
 * ``parity``: every case at the CPU sample's size (n // cpu-scale) through
   the public API against the CPU oracle's RHS of the same run.
+* Output: one JSON line of a few kilobytes on standard output (times per case, plain
+  numbers of the extras); the full record, with every variant's times and errors, on
+  standard error after ``details:``.
 * ``--impl reference``: the CPU FP64 oracle (a restatement of the
   reference's operators; the reference itself cannot run here) on a bounded
   sample of every case, one process per case over the host's cores.
@@ -86,6 +89,32 @@ def replica_rate(units_per_rank: float, seconds: float, world: int) -> float:
     """Whole-job rate of ``world`` independent replicas that each process
     ``units_per_rank`` in at most ``seconds`` (the max over ranks)."""
     return world * units_per_rank / seconds
+
+
+def _short(x):
+    """A number to five digits; other scalars as they are."""
+    return float(f"{x:.5g}") if isinstance(x, float) else x
+
+
+def result_line(record: dict) -> dict:
+    """What is printed on standard output: the record with its long parts cut down to
+    one number per case and the plain numbers of every extra, a few kilobytes that
+    line-oriented readers take whole (the full record goes to standard error)."""
+    line = dict(record)
+    line["e2e"] = {k: v for k, v in record["e2e"].items()
+                   if k not in ("logged_steps", "overlap")}
+    line["case_ms"] = {c["case"].split(" n=")[0]: _short(c["ms"]) for c in line.pop("cases")}
+    if record.get("parity"):
+        line["parity"] = {k: v for k, v in record["parity"].items() if k != "cases"}
+    extras = {}
+    for name, entry in (line.pop("extras") or {}).items():
+        if isinstance(entry, dict):
+            extras[name] = {k: _short(v) for k, v in entry.items()
+                            if isinstance(v, (bool, int, float))}
+            if "error" in entry:
+                extras[name]["error"] = str(entry["error"])[:100]
+    line["extras"] = extras
+    return line
 
 
 # {{{ clocks sampling
@@ -745,7 +774,7 @@ def our_arm(args) -> None:
                  "hbm_frac": r["cost"].bytes / (case_ms[k] * 1e-3) / 1e9 / peaks["hbm_gbs"]}
                 for k, r in enumerate(runs)]
     if rank == 0:
-        line = {
+        record = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
             "steps": K, "warmup": args.warmup, "ms_per_step": ms_step,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -778,7 +807,8 @@ def our_arm(args) -> None:
             "cases": per_case,
             "extras": extras,
         }
-        print(json.dumps(line), flush=True)
+        print("details:", json.dumps(record), file=sys.stderr, flush=True)
+        print(json.dumps(result_line(record)), flush=True)
     if world > 1:
         dist.destroy_process_group()
 
