@@ -18,7 +18,10 @@ __global__ void __launch_bounds__(256)
     // this launch)
     const float f[5] = {d2f_alu(rho), d2f_alu(en), d2f_alu(m0), d2f_alu(m1), d2f_alu(m2)};
     const double r0 = f2d_alu(__frcp_rn(f[0]));
-    const double rinv = fma(r0, fma(-rho, r0, 1.0), r0);
+    double rinv = fma(r0, fma(-rho, r0, 1.0), r0);
+    // these conversions know normal floats only: 2^-126 <= |rho| < 2^126
+    if (((uint32_t)__double2hiint(rho) & 0x7fffffffu) - (897u << 20) >= (252u << 20))
+      rinv = rcp64_fast(rho);
     const float p = d2f_alu((gamma - 1.0) * (en - 0.5 * (m0 * m0 + m1 * m1 + m2 * m2) * rinv));
     const mix::Trace s = mix::euler_trace(f, p, (float)gamma);
     rec[2 * n] = make_float4(f[0], f[1], f[2], f[3]);

@@ -156,3 +156,44 @@ def test_euler_plan_holds_one_table_per_node():
     nodes = mesh.nelements * mesh.np_            # 4.6 million: 147.5 and 18.4 MB
     # operator blocks and allocation granularity: 8 MB
     assert used[1] <= 32 * nodes + 8 * 2**20
+
+
+@pytest.mark.parametrize("equation,order,variant", [
+    *[(eq, o, 0) for eq in ("wave", "euler") for o in (1, 2, 3, 4)],
+    ("maxwell", 2, 1), ("maxwell", 3, 1)])
+def test_extreme_states_have_the_general_kernels_bits(equation, order, variant):
+    """Values outside the normal floats (and NaN, infinities, zeros) in whole elements
+    and in single nodes of a member: the same values, signs and NaNs on both kernels."""
+    from actx_dgfem_suite_gb300.discretization import union_discretization
+    from actx_dgfem_suite_gb300.plan import DeviceMesh, DevicePlan
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    per_sm = {2: 450, 3: 300}[order] if equation == "maxwell" else PER_SM[equation][order - 1]
+    prob = make_problem(equation, jittered_box_mesh(5), order, seed=order)
+    nel = prob.disc.nelements
+    count = per_sm * nsm // nel + 1
+    q = torch.from_numpy(prob.fields).cuda()
+    values = [float("nan"), float("inf"), -float("inf"), 0.0, -0.0, 1e300, -1e300, 1e-300,
+              1e38, 3.5e38, 1.1e-38, 1e-39, 1e-44, -1.1e-38, 1.7e38, -2.5]
+    item = 0
+    for value in values:
+        for k in range(q.shape[0]):
+            for node in (slice(None), item % q.shape[2]):
+                q[k, (37 * item + 5) % nel, node] = value
+                item += 1
+    big = torch.cat([q] * count, dim=1).contiguous()
+    union, _ = union_discretization([prob.disc] * count)
+    got = []
+    for disc, x in ((prob.disc, q), (union, big)):
+        plan = DevicePlan(DeviceMesh(disc, "cuda:0"), equation, prob.params, "fp32-mixed")
+        plan.set_variant(variant)
+        r = plan.rhs(x)
+        res, qo = torch.zeros_like(x), torch.empty_like(x)
+        plan.rk_stage(x, qo, res, 0.3, 0.7, 1e-2)
+        plan.finish()
+        got.append([y[:, -nel:] for y in (r, res, qo)] + [plan.info()["kernel"]])
+    assert got[0][3] != got[1][3]
+    for a, b in zip(got[0][:3], got[1][:3]):
+        nan = torch.isnan(a)
+        assert torch.equal(nan, torch.isnan(b))
+        assert torch.equal(a[~nan].view(torch.int64), b[~nan].view(torch.int64))
+        assert bool(torch.isfinite(a).any())
