@@ -14,8 +14,8 @@
 //     and only exterior traces from outside the tile recompute pressure, 1/rho and
 //     wave speed (Euler); a row of squares puts two thirds of a tile's edge sides
 //     inside it.  Which sides glue is read off the gather index, point by point
-//     and in both directions, and off the normals, for every tile; sides that do
-//     not match exactly are evaluated on their own.  Sides with outside traces
+//     and in both directions, and off the normals (opposite to 1e-12), for every tile;
+//     sides that do not match are evaluated on their own.  Sides with outside traces
 //     come first in the work list, because an FP64 instruction takes the pipe for
 //     a whole warp however few lanes need it.
 //
