@@ -284,23 +284,30 @@ __device__ __forceinline__ Real constant(const RhsArgs& a, int n) {
     return a.c32[n];
 }
 
-// CTAs per SM that the registers must allow, FP32 products on the CUDA cores (0: left to
-// the compiler).
+// CTAs per SM that the registers must allow, mixed precision (0: left to the compiler).
 //   Maxwell, order 3: waits for its gathers (long scoreboard 4.0 of 10 cycles per issued
 // instruction, 38 % of the issue slots used) with the two CTAs per SM that 107 registers
 // allow; three at 80 registers (48 bytes spilled): 279,936 tets 654 -> 544 us, RK stage
-// 895 -> 692 us.  Order 1 at five CTAs and order 4 at three: within 8 % either way (663,552
-// tets 192 -> 176 us, 82,944 tets 22 -> 23; P4 45 -> 52 and 420 -> 410).  Order 2 would gain
-// (384,000 tets: 469 us, at three 353, at four 342) and is left as the autotuner's choices
-// were measured with it.
+// 895 -> 692 us.  Five CTAs at order 1 and three at order 4 gain on large
+// meshes and lose on small ones (order 1: 663,552 tets 192 -> 176 us, 82,944 tets 22 -> 23;
+// order 4: 82,944 tets 420 -> 410, 10,368 tets 45 -> 52).  Order 2 would gain (384,000 tets:
+// 469 us, at three 353, at four 342) and is left as the autotuner's choices were measured
+// with it.
 //   Wave order 1, wave order 2 (RK stage), Euler order 3 (RK stage): left alone the compiler
 // holds them to 40 / 66 / 80 registers since the FP64 to FP32 conversion got shorter, and
 // keeps fewer loads in flight or spills.  Limits of 5 / 3 / 2 CTAs give 46 / 80 / 122:
 // wave P1 48,000 tets 12.3 -> 10.7 us, wave P2 stage 34,992 tets 30.4 -> 28.4, Euler P3
 // stage 7,986 tets 31.8 -> 29.8.
+//   Maxwell order 1 on mma.sync, for the same reason (RK stages of 256 and 128 threads held
+// to 48 registers, RHS of 512 to 56; here 64 / 56 / 64): 162,000 tets, variant 1 stage 118 ->
+// 110 us, 7 stage 102 -> 97, 9 RHS 153 -> 126.
 template <int N, int EQ, typename Real, int MODE>
 constexpr int min_ctas() {
-  if (std::is_same<Real, double>::value || (MODE & MODE_TC)) return 0;
+  if (std::is_same<Real, double>::value) return 0;
+  if (N == 1 && EQ == DG_MAXWELL && MODE == (MODE_TC | MODE_STAGE)) return 4;
+  if (N == 1 && EQ == DG_MAXWELL && MODE == (MODE_TC | MODE_B512)) return 2;
+  if (N == 1 && EQ == DG_MAXWELL && MODE == (MODE_TC | MODE_B128 | MODE_STAGE)) return 9;
+  if (MODE & MODE_TC) return 0;
   if (N == 3 && EQ == DG_MAXWELL) return 3;
   if (N == 1 && EQ == DG_WAVE && MODE == MODE_RHS) return 5;
   if (N == 2 && EQ == DG_WAVE && MODE == MODE_STAGE) return 3;
